@@ -315,6 +315,12 @@ size_t b200_lm_head_argmax_workspace_bytes(void);
 int b200_lm_head_argmax(const void* x, const void* w, int64_t* next_tokens, void* workspace,
                         size_t workspace_bytes, void* status_word, int num_rows, int vocab_size,
                         int hidden, void* stream);
+/* The same, and the logits [num_rows, vocab_size] of logits_dtype (B200_DTYPE_*), 4-byte aligned: the values of
+ * b200_dense_gemm_bf16 / _f32 on the same operands, without a second pass over w. */
+int b200_lm_head_argmax_logits(const void* x, const void* w, int64_t* next_tokens, void* logits,
+                               int logits_dtype, void* workspace, size_t workspace_bytes,
+                               void* status_word, int num_rows, int vocab_size, int hidden,
+                               void* stream);
 
 /* ----------------------------------------------------- fused step glue -- */
 

@@ -50,8 +50,10 @@
 // up rows of the same 128 features); or (lm_head) a running arg-max: every epilogue thread owns one feature of
 // the current weight tile and keeps, for each of its 128 rows of X, the largest logit it has seen over
 // all the tiles of the CTA as one integer key in a register; the warp-wide maximum is taken once, after
-// the last tile.  The [M, vocab] logits are never written; a small second kernel folds the per-warp
-// candidates (largest value, ties to the lower token id).
+// the last tile, the four lane quarters of a CTA are folded through shared memory, and a small second kernel
+// folds the CTAs' candidates (largest value, ties to the lower token id).  The [M, vocab] logits are written
+// only when the caller asks for them, from the same registers: a second product over the output matrix reads
+// its 622 MB (vocabulary 151936, width 2048) once more, 107 us at one row and 140 us at 256.
 
 #include <mutex>
 
@@ -91,8 +93,8 @@ struct DenseCfg {
 };
 
 struct DenseParams {
-  __nv_bfloat16* y;   // kEpiStore, kEpiGlu: [M, ldy]
-  float* y_f32;       // kEpiStore: instead of y
+  __nv_bfloat16* y;   // kEpiStore, kEpiGlu: [M, ldy]; kEpiArgmax: the logits, or NULL
+  float* y_f32;       // kEpiStore, kEpiArgmax: instead of y
   int ldy;            // row pitch of y
   int groups, x_step, w_step, y_step;
   // kEpiSplit (positions, block_table, page, num_blocks, max_pages below serve its page segments; positions NULL =
@@ -106,7 +108,7 @@ struct DenseParams {
   const MoeTile* tiles;
   const int* num_tiles;
   int num_experts, max_tiles;
-  float* part_val;    // kEpiArgmax: [grid * 4, 256] candidates per TMEM lane quarter
+  float* part_val;    // kEpiArgmax: [256, grid] candidates of the CTAs
   int* part_idx;
   float* exchange;    // kEpiStore, split K: [tile][finishing CTA][source CTA][rows_per][128] fp32
   // kEpiQkvRope: the q/k/v projection of heads of 128 with per-head RMSNorm, RoPE and the page write in its
@@ -540,6 +542,26 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
                 const uint32_t key = n < p.N ? ((float_key(__uint_as_float(v[i])) & ~31u) | tag) : 0u;
                 best[EPI == kEpiArgmax ? c * 32 + i : 0] = max(best[EPI == kEpiArgmax ? c * 32 + i : 0], key);
               }
+              const int row0 = (half * 4 + c) * 32, left = p.M - row0;
+              if (p.y != nullptr) {
+                if ((p.N & 1) == 0) {
+                  __nv_bfloat16* dst = p.y + static_cast<size_t>(row0 + (lane & 1)) * p.N + (n & ~1);
+#pragma unroll
+                  for (int i = 0; i < 32; i += 2) {
+                    if (i >= left) break;  // uniform across the warp
+                    const uint32_t two = pack_row_pair(__uint_as_float(v[i]), __uint_as_float(v[i + 1]), lane);
+                    if (n < p.N && i + (lane & 1) < left) *reinterpret_cast<uint32_t*>(dst + static_cast<size_t>(i) * p.N) = two;
+                  }
+                } else if (n < p.N) {
+#pragma unroll
+                  for (int i = 0; i < 32; ++i)
+                    if (i < left) p.y[static_cast<size_t>(row0 + i) * p.N + n] = __float2bfloat16(__uint_as_float(v[i]));
+                }
+              } else if (p.y_f32 != nullptr && n < p.N) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (i < left) p.y_f32[static_cast<size_t>(row0 + i) * p.N + n] = __uint_as_float(v[i]);
+              }
             }
           }
         }
@@ -640,7 +662,10 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
           win_lane[j >> 5] = __ffs(who) - 1;  // equal logits of one tile: the lower feature
         }
       }
-      const size_t prow = static_cast<size_t>(blockIdx.x) * 4 + quarter;
+      // The four lane quarters meet in the ring (every copy and every MMA of this CTA has completed), so that the fold
+      // has one candidate per CTA to read, in rows: with four per CTA in columns it took 50-60 us at 256 rows.
+      float* quarter_val = reinterpret_cast<float*>(ring_ptr);
+      int* quarter_idx = reinterpret_cast<int*>(ring_ptr) + 4 * kDenseMaxRows;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int col = half * 128 + c * 32 + lane;
@@ -653,8 +678,25 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
           idx = (tile * A_TILES + a_of) * 128 + quarter * 32 + win_lane[c];
           val = key_float(win_key[c] & ~31u);
         }
-        p.part_val[prow * kDenseMaxRows + col] = val;
-        p.part_idx[prow * kDenseMaxRows + col] = idx;
+        quarter_val[quarter * kDenseMaxRows + col] = val;
+        quarter_idx[quarter * kDenseMaxRows + col] = idx;
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      const int col = (warp - 2) * 32 + lane;
+      float val = quarter_val[col];
+      int idx = quarter_idx[col];
+#pragma unroll
+      for (int q = 1; q < 4; ++q) {
+        const float v = quarter_val[q * kDenseMaxRows + col];
+        const int i = quarter_idx[q * kDenseMaxRows + col];
+        if (v > val || (v == val && i < idx)) {
+          val = v;
+          idx = i;
+        }
+      }
+      if (col < p.M) {
+        p.part_val[static_cast<size_t>(col) * gridDim.x + blockIdx.x] = val;
+        p.part_idx[static_cast<size_t>(col) * gridDim.x + blockIdx.x] = idx;
       }
     }
   }
@@ -755,7 +797,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
 #endif
 }
 
-// Folds the per-warp arg-max candidates: one warp per row of X.
+// Folds the CTAs' arg-max candidates: one warp per row of X.
 __global__ void __launch_bounds__(128)
 argmax_fold_kernel(const float* __restrict__ part_val, const int* __restrict__ part_idx, int parts, int M,
                    long long* __restrict__ out) {
@@ -767,8 +809,8 @@ argmax_fold_kernel(const float* __restrict__ part_val, const int* __restrict__ p
   float bv = -INFINITY;
   int bi = 0x7fffffff;
   for (int r = lane; r < parts; r += 32) {
-    const float v = part_val[static_cast<size_t>(r) * kDenseMaxRows + m];
-    const int i = part_idx[static_cast<size_t>(r) * kDenseMaxRows + m];
+    const float v = part_val[static_cast<size_t>(m) * parts + r];
+    const int i = part_idx[static_cast<size_t>(m) * parts + r];
     if (v > bv || (v == bv && i < bi)) {
       bv = v;
       bi = i;
@@ -1294,13 +1336,13 @@ extern "C" int b200_qkv_rope_append_gemm(const void* x, const void* wqkv, const 
 }
 
 extern "C" size_t b200_lm_head_argmax_workspace_bytes(void) {
-  // candidates of 4 epilogue warps of up to 256 CTAs for 256 rows: value + index
+  // candidates of up to 256 CTAs for 256 rows, value + index (a multiple of what is used: the size is part of the interface)
   return static_cast<size_t>(256) * 4 * kDenseMaxRows * 8;
 }
 
-extern "C" int b200_lm_head_argmax(const void* x, const void* w, int64_t* next_tokens, void* workspace,
-                                   size_t workspace_bytes, void* status_word, int num_rows, int vocab_size,
-                                   int hidden, void* stream) {
+static int lm_head_any(const void* x, const void* w, int64_t* next_tokens, __nv_bfloat16* logits, float* logits_f32,
+                       void* workspace, size_t workspace_bytes, void* status_word, int num_rows, int vocab_size, int hidden,
+                       void* stream) {
   int rc = dense_args_ok(x, w, num_rows, vocab_size, hidden, "lm_head_argmax");
   if (rc) return rc;
   B200_REQUIRE(next_tokens && workspace, "lm_head_argmax: null pointer");
@@ -1316,6 +1358,8 @@ extern "C" int b200_lm_head_argmax(const void* x, const void* w, int64_t* next_t
   rc = device_sm_count(&sms);
   if (rc) return rc;
   DenseParams p{};
+  p.y = logits;
+  p.y_f32 = logits_f32;
   p.err = static_cast<int*>(status_word);
   p.M = num_rows;
   p.groups = 1;
@@ -1338,6 +1382,25 @@ extern "C" int b200_lm_head_argmax(const void* x, const void* w, int64_t* next_t
   rc = launch_dense<2, kEpiArgmax>(w_map, x_map, p, grid, as_stream(stream));
   if (rc) return rc;
   B200_CUDA(launch_overlapped(argmax_fold_kernel, dim3((num_rows + 3) / 4), dim3(128), 0, as_stream(stream), p.part_val,
-                              p.part_idx, grid * 4, num_rows, reinterpret_cast<long long*>(next_tokens)));
+                              p.part_idx, grid, num_rows, reinterpret_cast<long long*>(next_tokens)));
   return 0;
+}
+
+extern "C" int b200_lm_head_argmax(const void* x, const void* w, int64_t* next_tokens, void* workspace,
+                                   size_t workspace_bytes, void* status_word, int num_rows, int vocab_size,
+                                   int hidden, void* stream) {
+  return lm_head_any(x, w, next_tokens, nullptr, nullptr, workspace, workspace_bytes, status_word, num_rows, vocab_size, hidden,
+                     stream);
+}
+
+extern "C" int b200_lm_head_argmax_logits(const void* x, const void* w, int64_t* next_tokens, void* logits, int logits_dtype,
+                                          void* workspace, size_t workspace_bytes, void* status_word, int num_rows,
+                                          int vocab_size, int hidden, void* stream) {
+  B200_REQUIRE(logits && (reinterpret_cast<uintptr_t>(logits) & 3) == 0, "lm_head_argmax_logits: logits null or unaligned");
+  B200_REQUIRE(logits_dtype == B200_DTYPE_BF16 || logits_dtype == B200_DTYPE_F32, "lm_head_argmax_logits: logits_dtype %d",
+               logits_dtype);
+  const bool f32 = logits_dtype == B200_DTYPE_F32;
+  return lm_head_any(x, w, next_tokens, f32 ? nullptr : static_cast<__nv_bfloat16*>(logits),
+                     f32 ? static_cast<float*>(logits) : nullptr, workspace, workspace_bytes, status_word, num_rows, vocab_size,
+                     hidden, stream);
 }

@@ -146,6 +146,7 @@ class PagedEngine:
                                                `row` (and state slot `slot`)
       _mixed_hidden(tokens, pos, table, first_pos, n, B, slot)   rows of a chunk (first n) and of a decode step (the rest)
       _pick(h, out) / _logits(h)               next tokens (arg-max) / logits of hidden rows
+      _pick_with_logits(h, out)                both, from one pass over lm_head where the model has a kernel for it
 
     A model with recurrent layers also keeps a state per sequence, in slots: `num_slots` of them for sequences and one more
     for padding rows.  `state_slots[i]` names the slot of row i (row i itself unless the caller says otherwise), a prompt
@@ -167,8 +168,8 @@ class PagedEngine:
             raise RuntimeError(f"{type(self).__name__} needs a CUDA device; this path has no CPU implementation")
         self.device = torch.device(device)
         # The step picks its next tokens inside the lm_head kernel and never writes the [batch, vocab] logits.
-        # With keep_logits they are computed as well, by a second pass over lm_head, into `last_logits` (for
-        # tests and inspection; set before the first step, the graphs are captured with or without it).
+        # With keep_logits that kernel writes them as well, into `last_logits` (for tests, sampling and inspection;
+        # set before the first step, the graphs are captured with or without it).
         self.keep_logits = keep_logits
         self.last_logits = None
         self.max_batch = max_batch
@@ -192,8 +193,9 @@ class PagedEngine:
         """One decode step over rows [0, B) of the static buffers; advances ctx_lens by one."""
         h = self._decode_hidden(B)
         if self.keep_logits:
-            self.last_logits = self._logits(h)
-        self._pick(h, self.next_tokens[:B])
+            _, self.last_logits = self._pick_with_logits(h, self.next_tokens[:B])
+        else:
+            self._pick(h, self.next_tokens[:B])
         self.ctx_lens[:B] += 1
 
     GRAPH_BUCKETS = (1, 2, 4, 8, 16, 24, 32, 48, 64, 96, 128, 192, 256, 384, 512, 768, 1024)
@@ -280,6 +282,9 @@ class PagedEngine:
             self.last_logits = self._graph_logits[B]  # the buffer this graph writes
         return self.next_tokens[:real]
 
+    def _pick_with_logits(self, h, out=None) -> tuple[torch.Tensor, torch.Tensor]:
+        return self._pick(h, out), self._logits(h)
+
     def _check_slot(self, slot: int) -> None:
         if self.num_slots and not 0 <= slot < self.num_slots:
             raise ValueError(f"state slot {slot} outside [0, {self.num_slots})")
@@ -333,11 +338,10 @@ class PagedEngine:
                 logits = self._logits(h[torch.tensor([want[i] - lo for i in here], device=self.device)])
                 wanted[torch.tensor(here, device=self.device)] = logits
             h_last = h[hi - lo - 1:hi - lo].contiguous()
-        first = self._pick(h_last)
-        if want is not None:
-            return int(first[0]), wanted
-        # the logits cost a second pass over lm_head: only for engines built to keep them (tests, debugging)
-        return int(first[0]), self._logits(h_last)[0] if self.keep_logits else None
+        if want is not None or not self.keep_logits:
+            return int(self._pick(h_last)[0]), wanted
+        first, logits = self._pick_with_logits(h_last)
+        return int(first[0]), logits[0]
 
     @torch.no_grad()
     def mixed_step(self, B: int, chunk_token_ids: list[int], block_ids: list[int], first_pos: int,
@@ -610,6 +614,10 @@ class DecodeEngine(PagedEngine):
 
     def _pick(self, h, out=None) -> torch.Tensor:
         return ops.lm_head_argmax(h, self.lm_head, self.argmax_ws, out=out, status=self.gemm_status)
+
+    def _pick_with_logits(self, h, out=None) -> tuple[torch.Tensor, torch.Tensor]:
+        logits = torch.empty(h.shape[0], self.vocab_size, dtype=self.logits_dtype, device=self.device)
+        return ops.lm_head_argmax(h, self.lm_head, self.argmax_ws, out=out, status=self.gemm_status, logits=logits), logits
 
     def _logits(self, h) -> torch.Tensor:
         return ops.dense_gemm(h, self.lm_head, status=self.gemm_status)

@@ -589,6 +589,12 @@ class LayeredEngine(gated.GatedMechanisms, PagedEngine):
             return ops.lm_head_argmax(h, self.lm_head, self.argmax_ws, out=out, status=self.status)
         return ops.argmax_rows(ops.gemm_f32(h, self.lm_head), out)
 
+    def _pick_with_logits(self, h, out=None) -> tuple[torch.Tensor, torch.Tensor]:
+        if self.dtype != torch.bfloat16:
+            return super()._pick_with_logits(h, out)
+        logits = torch.empty(h.shape[0], self.lm_head.shape[0], dtype=torch.float32, device=self.device)
+        return ops.lm_head_argmax(h, self.lm_head, self.argmax_ws, out=out, status=self.status, logits=logits), logits
+
     def _logits(self, h) -> torch.Tensor:
         if self.dtype == torch.bfloat16:
             return ops.dense_gemm_f32_out(h, self.lm_head, self.status)

@@ -250,8 +250,10 @@ def lm_head_argmax_workspace(device) -> torch.Tensor:
 
 
 def lm_head_argmax(x: torch.Tensor, w: torch.Tensor, workspace: torch.Tensor | None = None,
-                   out: torch.Tensor | None = None, status: torch.Tensor | None = None) -> torch.Tensor:
-    """argmax_n (x w^T)[m, n] per row without writing the logits; ties go to the lower index.  int64 [M]."""
+                   out: torch.Tensor | None = None, status: torch.Tensor | None = None,
+                   logits: torch.Tensor | None = None) -> torch.Tensor:
+    """argmax_n (x w^T)[m, n] per row; ties go to the lower index.  int64 [M].  The logits are written only to a `logits`
+    tensor [M, N] (bfloat16 or float32) given for them."""
     _need(x, "x", torch.bfloat16)
     _need(w, "w", torch.bfloat16)
     M, K = x.shape
@@ -262,8 +264,18 @@ def lm_head_argmax(x: torch.Tensor, w: torch.Tensor, workspace: torch.Tensor | N
     if out is None:
         out = torch.empty(M, dtype=torch.int64, device=x.device)
     _need(out, "out", torch.int64)
+    if logits is not None:
+        _need(logits, "logits")
+        if logits.dtype not in DTYPE_CODE or logits.shape != (M, w.shape[0]):
+            raise ValueError(f"logits must be [{M}, {w.shape[0]}] float32 or bfloat16, got {list(logits.shape)} {logits.dtype}")
     for lo in range(0, M, 256):  # the kernel keeps one running candidate per row in registers: 256 rows a call
         hi = min(M, lo + 256)
+        if logits is not None:
+            rc = _lib.load().b200_lm_head_argmax_logits(_ptr(x[lo:hi]), _ptr(w), out[lo:hi].data_ptr(), _ptr(logits[lo:hi]),
+                                                        DTYPE_CODE[logits.dtype], _ptr(workspace), workspace.numel(), _ptr(status),
+                                                        hi - lo, w.shape[0], K, _stream())
+            check(rc, "b200_lm_head_argmax_logits")
+            continue
         rc = _lib.load().b200_lm_head_argmax(_ptr(x[lo:hi]), _ptr(w), out[lo:hi].data_ptr(), _ptr(workspace),
                                              workspace.numel(), _ptr(status), hi - lo, w.shape[0], K, _stream())
         check(rc, "b200_lm_head_argmax")

@@ -104,6 +104,19 @@ def test_lm_head_argmax_agrees_with_argmax_of_the_written_logits(ops):
     assert bool((picked == logits.max(dim=1).values).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,V,K", [(1, 8192, 1024), (33, 1001, 512), (256, 3000, 128), (300, 129, 64)])
+def test_lm_head_argmax_writes_the_logits_of_the_plain_product(ops, M, V, K, dtype):
+    """Same operands, same order of sums: the same bits, odd vocabularies and more rows than one launch takes included."""
+    x, w, _ = make(M, V, K, seed=V + M)
+    xd, wd = x.to(DEV), w.to(DEV)
+    want = ops.dense_gemm(xd, wd, k_split=1) if dtype == torch.bfloat16 else ops.dense_gemm_f32_out(xd, wd)
+    logits = torch.full((M, V), float("nan"), dtype=dtype, device=DEV)
+    tok = ops.lm_head_argmax(xd, wd, logits=logits)
+    assert torch.equal(logits, want)
+    assert torch.equal(tok, ops.lm_head_argmax(xd, wd))
+
+
 @pytest.mark.parametrize("R,hq,hkv,K", [(256, 32, 4, 2048), (1, 32, 4, 2048), (37, 64, 4, 4096), (300, 8, 2, 512)])
 def test_qkv_projection_with_norm_rope_and_page_write_equals_the_two_kernels(ops, R, hq, hkv, K):
     """b200_qkv_rope_append_gemm against b200_dense_gemm_bf16 (no K split) + b200_qk_norm_rope_append: the query
