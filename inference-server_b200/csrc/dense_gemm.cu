@@ -80,17 +80,23 @@ struct DenseSeg {
   int heads, dim;  // kSegPages: pool [num_blocks, heads, page, dim]
   void* ptr;       // kSegBf16 / kSegF32: [M, end - begin]
 };
-constexpr int kQkvStageBytes = kDenseMaxRows * 128 * 2;  // kEpiQkvRope: one head of up to 256 rows, bf16
 
+// Shared memory: a ring of as many stages as fit (a stage holds A_TILES W tiles and one X box of the launch's width, so a
+// narrow X box leaves room for a deeper ring: 4 stages at 256 rows, 9 at 32), and for kEpiQkvRope a bf16 copy of one head's
+// tile behind it.  The total leaves room on the SM for the blocks of the small kernel in front.
+constexpr int kDenseMaxStages = 12;
 template <int A_TILES, int EPI = kEpiStore>
 struct DenseCfg {
-  // the q/k/v epilogue keeps a bf16 copy of one head's tile beside the ring and gives a stage for it
-  static constexpr int kStages = (A_TILES == 1 && EPI != kEpiQkvRope) ? 4 : 3;
-  static constexpr int kStageBytes = A_TILES * kDenseWBytes + kDenseXBytesMax;
-  static constexpr int kRingBytes = kStages * kStageBytes;  // 192 KiB, or 144 KiB + 64 KiB of head tile
-  static constexpr int kExtraBytes = EPI == kEpiQkvRope ? kQkvStageBytes : 0;
-  static constexpr int kSmemBytes = kRingBytes + kExtraBytes + 1024 /* alignment */ + 256 /* barriers, tmem base */;
+  static constexpr int kAreaBytes = EPI == kEpiQkvRope ? 208 * 1024 : 192 * 1024;
+  static constexpr int kBarBytes = 16 * kDenseMaxStages + 64;
+  static constexpr int kSmemBytes = kAreaBytes + 1024 /* alignment */ + kBarBytes /* and tmem base */;
+  __host__ __device__ static constexpr int stage_bytes(int xbox) { return A_TILES * kDenseWBytes + xbox * 128; }
+  static constexpr int stages(int xbox) {
+    const int n = (kAreaBytes - (EPI == kEpiQkvRope ? xbox * 256 : 0)) / stage_bytes(xbox);
+    return n < kDenseMaxStages ? n : kDenseMaxStages;
+  }
 };
+static_assert(DenseCfg<1, kEpiQkvRope>::stages(256) >= 3 && DenseCfg<2>::stages(256) >= 3, "a ring of at least three stages");
 
 struct DenseParams {
   __nv_bfloat16* y;   // kEpiStore, kEpiGlu: [M, ldy]; kEpiArgmax: the logits, or NULL
@@ -124,9 +130,12 @@ struct DenseParams {
   __nv_bfloat16* v_pool;
   float eps;
   int hq, hkv, page, num_blocks, max_pages, max_pos;
+  bool wide;          // norm weights, tables, q_out and pools are 8-byte aligned: four features per access
   int page_shift;     // kEpiSplit: page is a power of two
   int* err;
   int M, N, K;
+  int stages;         // of the ring
+  int prefetch;       // K blocks of W per CTA that are asked into L2 ahead of the kernel before
   int m_tiles;        // ceil(M / xbox)
   int n_tiles;        // ceil(N / (128 * A_TILES))
   int ksplit;         // CTAs of a cluster that share one tile (1 = no cluster)
@@ -182,6 +191,35 @@ __device__ __forceinline__ uint32_t pack_row_pair(float row_i, float row_i1, int
   return odd ? pack_bf16x2(other, row_i1) : pack_bf16x2(row_i, other);
 }
 
+// Byte of (row, feature) in the bf16 copy of a head's tile.
+__device__ __forceinline__ uint32_t head_at(int row, int d) {
+  return static_cast<uint32_t>(row) * 256u + (static_cast<uint32_t>((d >> 3) ^ ((row & 1) << 2)) << 4) + (d & 7) * 2u;
+}
+__device__ __forceinline__ void unpack_bf16x4(uint2 raw, float (&v)[4]) {
+  v[0] = __uint_as_float(raw.x << 16);
+  v[1] = __uint_as_float(raw.x & 0xffff0000u);
+  v[2] = __uint_as_float(raw.y << 16);
+  v[3] = __uint_as_float(raw.y & 0xffff0000u);
+}
+
+// Four consecutive bf16; `wide`: the address is a multiple of 8 bytes.
+__device__ __forceinline__ uint2 load_bf16x4(const __nv_bfloat16* p, bool wide) {
+  if (wide) return __ldg(reinterpret_cast<const uint2*>(p));
+  const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
+  return make_uint2(__ldg(h) | static_cast<uint32_t>(__ldg(h + 1)) << 16, __ldg(h + 2) | static_cast<uint32_t>(__ldg(h + 3)) << 16);
+}
+__device__ __forceinline__ void store_bf16x4(__nv_bfloat16* p, uint2 v, bool wide) {
+  if (wide) {
+    *reinterpret_cast<uint2*>(p) = v;
+    return;
+  }
+  unsigned short* h = reinterpret_cast<unsigned short*>(p);
+  h[0] = static_cast<unsigned short>(v.x);
+  h[1] = static_cast<unsigned short>(v.x >> 16);
+  h[2] = static_cast<unsigned short>(v.y);
+  h[3] = static_cast<unsigned short>(v.y >> 16);
+}
+
 // Which weight rows and which rows of X an item multiplies: W tile nt of group (or expert) g, rows [m0, m_end).
 struct DenseItem {
   int g, nt, m0, m_end;
@@ -215,14 +253,14 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
                   const DenseParams p) {
 #ifdef B200_DEVICE_OK
   using Cfg = DenseCfg<A_TILES, EPI>;
-  constexpr int kStages = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* ring_ptr = smem_raw + (ring - smem_u32(smem_raw));
-  const uint32_t bars = ring + Cfg::kRingBytes + Cfg::kExtraBytes;
-  const uint32_t bar_full = bars, bar_empty = bars + 8 * kStages;
-  const uint32_t bar_tfull = bars + 16 * kStages, bar_tempty = bar_tfull + 16;
-  uint32_t* tmem_base_sm = reinterpret_cast<uint32_t*>(ring_ptr + Cfg::kRingBytes + Cfg::kExtraBytes + 16 * kStages + 32);
+  const uint32_t stages = p.stages, stage_bytes = Cfg::stage_bytes(p.xbox);
+  const uint32_t bars = ring + Cfg::kAreaBytes;
+  const uint32_t bar_full = bars, bar_empty = bars + 8 * kDenseMaxStages;
+  const uint32_t bar_tfull = bars + 16 * kDenseMaxStages, bar_tempty = bar_tfull + 16;
+  uint32_t* tmem_base_sm = reinterpret_cast<uint32_t*>(ring_ptr + Cfg::kAreaBytes + 16 * kDenseMaxStages + 32);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // accumulator buffers: one W tile -> two buffers of 256 columns that alternate between work items;
@@ -234,7 +272,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
     tma_prefetch_desc(&x_map);
   }
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (uint32_t s = 0; s < stages; ++s) {
       mbar_init(bar_full + 8 * s, 1);
       mbar_init(bar_empty + 8 * s, 1);
     }
@@ -250,13 +288,23 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_sm;
+  const int ks = p.ksplit;
+  const int kb_per = (p.K + kDenseBlockK - 1) / kDenseBlockK / ks;  // K blocks of one work item
   // Everything above is this CTA's own set-up; X (and the buffers the epilogues write) belong to the kernels
-  // before this one.
+  // before this one.  W's first blocks are asked into L2 while those kernels finish: a hint, so it does not matter who wrote
+  // W and when, and with a few rows it keeps the whole of a CTA's W in flight instead of the ring's share of it.
+  if (p.prefetch > 0 && threadIdx.x == 64 && p.tiles == nullptr) {
+    const int tile = static_cast<int>(blockIdx.x) / ks, kidx = static_cast<int>(blockIdx.x) - tile * ks;
+    const DenseItem item = dense_item(p, tile);
+    const int w_tiles = (EPI == kEpiGlu ? 2 : 1) * ((p.N + 127) / 128);
+    for (int kb = 0; kb < p.prefetch; ++kb)
+#pragma unroll
+      for (int a = 0; a < A_TILES; ++a)
+        if (item.nt * A_TILES + a < w_tiles) tma_prefetch_2d(&w_map, (kidx * kb_per + kb) * kDenseBlockK, item.g * p.w_step + (item.nt * A_TILES + a) * 128);
+  }
   grid_dep_wait();
   grid_dep_launch();
 
-  const int ks = p.ksplit;
-  const int kb_per = (p.K + kDenseBlockK - 1) / kDenseBlockK / ks;  // K blocks of one work item
   int listed = p.groups * p.m_tiles;
   if (p.tiles != nullptr) {
     listed = *p.num_tiles;
@@ -271,17 +319,16 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
   if (warp == 0) {
     // ------------------------------------------------------------ TMA ------
     if (lane == 0) {
-      uint32_t it = 0;
+      uint32_t slot = 0, phase = 0;
       bool alive = true;
       for (int w = blockIdx.x; w < total && alive; w += gridDim.x) {
         const int tile = w / ks, kidx = w - tile * ks;
         const DenseItem item = dense_item(p, tile);
         const int g = item.g, nt = item.nt;
-        for (int kb = 0; kb < kb_per; ++kb, ++it) {
-          const uint32_t slot = it % kStages, phase = (it / kStages) & 1;
+        for (int kb = 0; kb < kb_per; ++kb) {
           alive = mbar_wait(bar_empty + 8 * slot, phase ^ 1, p.err);
           if (!alive) break;
-          const uint32_t sw = ring + slot * Cfg::kStageBytes, sx = sw + A_TILES * kDenseWBytes;
+          const uint32_t sw = ring + slot * stage_bytes, sx = sw + A_TILES * kDenseWBytes;
           const int kx = (kidx * kb_per + kb) * kDenseBlockK;
           mbar_arrive_expect_tx(bar_full + 8 * slot, stage_tx);
 #pragma unroll
@@ -289,6 +336,10 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
             tma_load_2d(sw + a * kDenseWBytes, &w_map, bar_full + 8 * slot, kx,
                         g * p.w_step + (nt * A_TILES + a) * 128);
           tma_load_2d(sx, &x_map, bar_full + 8 * slot, g * p.x_step + kx, item.m0);
+          if (++slot == stages) {
+            slot = 0;
+            phase ^= 1;
+          }
         }
       }
     }
@@ -296,19 +347,18 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
     // ------------------------------------------------------------ MMA ------
     if (lane == 0) {
       const uint32_t idesc = umma_idesc_bf16(128, static_cast<uint32_t>(p.xbox));
-      uint32_t it = 0, item = 0;
+      uint32_t slot = 0, phase = 0, item = 0;
       bool alive = true;
       for (int w = blockIdx.x; w < total && alive; w += gridDim.x, ++item) {
         const uint32_t buf = item % kBufs, aphase = (item / kBufs) & 1;
         alive = mbar_wait(bar_tempty + 8 * buf, aphase ^ 1, p.err);
         if (!alive) break;
         tc_fence_after();
-        for (int kb = 0; kb < kb_per; ++kb, ++it) {
-          const uint32_t slot = it % kStages, phase = (it / kStages) & 1;
+        for (int kb = 0; kb < kb_per; ++kb) {
           alive = mbar_wait(bar_full + 8 * slot, phase, p.err);
           if (!alive) break;
           tc_fence_after();
-          const uint32_t sw = ring + slot * Cfg::kStageBytes, sx = sw + A_TILES * kDenseWBytes;
+          const uint32_t sw = ring + slot * stage_bytes, sx = sw + A_TILES * kDenseWBytes;
           const uint64_t b_desc = umma_desc_k128(sx);
 #pragma unroll
           for (int a = 0; a < A_TILES; ++a) {
@@ -319,6 +369,10 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
               tc_mma_bf16(d, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
           tc_commit(bar_empty + 8 * slot);
+          if (++slot == stages) {
+            slot = 0;
+            phase ^= 1;
+          }
         }
         if (alive) tc_commit(bar_tfull + 8 * buf);
       }
@@ -349,11 +403,11 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
       const int g = di.g, nt = di.nt;
       const uint32_t buf = item % kBufs, aphase = (item / kBufs) & 1;
       const int m0 = di.m0, m_end = di.m_end;
-      // kEpiQkvRope: position and page of the rows this warp will finish (lane i: row (warp - 2) + 8 i of the
-      // tile), fetched while the MMAs of the item are still running; -1 = not a row, or reported as bad
+      // kEpiQkvRope: position and page of the rows this warp will finish (four of every 32; lane i: row i % 4 of the
+      // four in rows 32 (i / 4) ...), fetched while the MMAs of the item are still running; -1 = not a row, or reported as bad
       int row_pos = -1, row_page = -1;
       if (EPI == kEpiQkvRope) {
-        const int r = (warp - 2) + 8 * lane, m = m0 + r;
+        const int r = 32 * (lane >> 2) + 4 * (warp - 2) + (lane & 3), m = m0 + r;
         if (r < p.xbox && m < p.M) {
           const int ps = p.positions[m];
           if (ps < 0 || ps >= p.max_pos || ps >= p.max_pages * p.page) {
@@ -495,14 +549,19 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
         const uint32_t t0 = lane_addr + (A_TILES == 1 ? buf : static_cast<uint32_t>(a)) * kDenseMaxRows;
         if (EPI == kEpiQkvRope) {
           // the tile is one head (128 features) of up to 256 rows: a bf16 copy goes to shared memory as
-          // [row][feature] - the projection's output is bf16 in the model, so this rounding is the model's
-          __nv_bfloat16* head = reinterpret_cast<__nv_bfloat16*>(ring_ptr + Cfg::kRingBytes);
+          // [row][feature] - the projection's output is bf16 in the model, so this rounding is the model's.
+          // Odd rows have their 64-byte halves swapped in pairs, so that the two rows a warp touches at a time
+          // lie in different banks.
+          uint8_t* head = ring_ptr + stages * stage_bytes;
           for (int c = half; c < chunks; c += 2) {
             uint32_t v[32];
             tmem_ld32(t0 + c * 32, v);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) head[(c * 32 + i) * 128 + t] = __float2bfloat16(__uint_as_float(v[i]));
+            for (int i = 0; i < 32; i += 2) {
+              const uint32_t two = pack_row_pair(__uint_as_float(v[i]), __uint_as_float(v[i + 1]), lane);
+              *reinterpret_cast<uint32_t*>(head + head_at(c * 32 + i + (lane & 1), t & ~1)) = two;
+            }
           }
         } else if (EPI == kEpiStore) {
           for (int c = half; c < chunks; c += 2) {
@@ -572,77 +631,92 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
       if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
       if (EPI == kEpiQkvRope) {
         // ---- per row of X: RMSNorm over the head (q and k), RoPE (rotate-half), then q to its output row
-        // and k / v into their page slot; warp e takes rows e, e + 8, ...; lane l holds d = l + 32 j.  Position
-        // and page of every row were fetched before the accumulator was awaited (lane i: the warp's i-th row), and
-        // the rows go four at a time so that their cos/sin loads are in flight together: done one row after the
-        // other, the dependent loads of 16-32 rows per warp cost more than the separate kernel they replace.
+        // and k / v into their page slot.  Eight lanes share a row, so a warp finishes four rows at a time, and two such
+        // passes go together so that their cos/sin loads overlap; lane m of the eight holds d = 4 m + b + 32 j, which
+        // leaves the partner element d +- 64 in the same lane and adds the squares in the order of a warp with
+        // d = lane + 32 j (b200_qk_norm_rope_append: the two must agree to the bit).  One row per warp with 2-byte
+        // accesses, as it was, took as long as the tile's MMAs: 1024 rows of 5120 features, width 2048, 40 us.
         asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight epilogue warps: the head tile is complete
-        const __nv_bfloat16* head = reinterpret_cast<const __nv_bfloat16*>(ring_ptr + Cfg::kRingBytes);
+        const uint8_t* head = ring_ptr + stages * stage_bytes;
         const int h = nt;  // weight tile = head: q heads, then k heads, then v heads
         const bool is_q = h < p.hq, is_k = !is_q && h < p.hq + p.hkv;
-        const __nv_bfloat16* nw = is_q ? p.q_norm_w : p.k_norm_w;
-        float nwf[4];
+        const int d0 = (lane & 7) * 4, sub = lane >> 3;
+        float nwf[4][4];
+        if (is_q || is_k) {
+          const __nv_bfloat16* nw = is_q ? p.q_norm_w : p.k_norm_w;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) nwf[j] = (is_q || is_k) ? __bfloat162float(nw[lane + 32 * j]) : 1.f;
-        const int my_rows = p.xbox / 8;  // rows this warp handles: 4..32
-        for (int i0 = 0; i0 < my_rows; i0 += 4) {
-          int pos[4], dstoff_ok[4];
-          __nv_bfloat16* dst[4];
-          float v[4][4], cs[4][4], sn[4][4];
+          for (int j = 0; j < 4; ++j) unpack_bf16x4(load_bf16x4(nw + d0 + 32 * j, p.wide), nwf[j]);
+        }
+        constexpr int kAtOnce = 2;
+        for (int i0 = 0; i0 < chunks; i0 += kAtOnce) {
+          uint2 raw[kAtOnce][4], cs[kAtOnce][4], sn[kAtOnce][4];
+          __nv_bfloat16* dst[kAtOnce];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
+          for (int u = 0; u < kAtOnce; ++u) {
+            dst[u] = nullptr;
             const int i = i0 + u;
-            pos[u] = __shfl_sync(0xffffffffu, row_pos, i & 31);
-            const int id = __shfl_sync(0xffffffffu, row_page, i & 31);
-            const int r = (warp - 2) + 8 * i, m = m0 + r;
-            dstoff_ok[u] = i < my_rows && pos[u] >= 0 && (is_q || id >= 0);
-            if (dstoff_ok[u]) {
+            const int pos = __shfl_sync(0xffffffffu, row_pos, (i * 4 + sub) & 31);
+            const int id = __shfl_sync(0xffffffffu, row_page, (i * 4 + sub) & 31);
+            if (i >= chunks || pos < 0 || !(is_q || id >= 0)) continue;
+            const int r = 32 * i + 4 * (warp - 2) + sub;
 #pragma unroll
-              for (int j = 0; j < 4; ++j) v[u][j] = __bfloat162float(head[r * 128 + lane + 32 * j]);
-              if (is_q || is_k) {
-                const __nv_bfloat16* c = p.cos_t + static_cast<size_t>(pos[u]) * 128;
-                const __nv_bfloat16* sp = p.sin_t + static_cast<size_t>(pos[u]) * 128;
+            for (int j = 0; j < 4; ++j) raw[u][j] = *reinterpret_cast<const uint2*>(head + head_at(r, d0 + 32 * j));
+            if (is_q || is_k) {
+              const __nv_bfloat16* c = p.cos_t + static_cast<size_t>(pos) * 128 + d0;
+              const __nv_bfloat16* sp = p.sin_t + static_cast<size_t>(pos) * 128 + d0;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  cs[u][j] = __bfloat162float(c[lane + 32 * j]);
-                  sn[u][j] = __bfloat162float(sp[lane + 32 * j]);
-                }
+              for (int j = 0; j < 4; ++j) {
+                cs[u][j] = load_bf16x4(c + 32 * j, p.wide);
+                sn[u][j] = load_bf16x4(sp + 32 * j, p.wide);
               }
-              if (is_q) {
-                dst[u] = p.q_out + (static_cast<size_t>(m) * p.hq + h) * 128;
-              } else {
-                const int kvh = is_k ? h - p.hq : h - p.hq - p.hkv;
-                __nv_bfloat16* pool = is_k ? p.k_pool : p.v_pool;
-                dst[u] = pool + ((static_cast<size_t>(id) * p.hkv + kvh) * p.page + pos[u] % p.page) * 128;
-              }
+            }
+            if (is_q) {
+              dst[u] = p.q_out + (static_cast<size_t>(m0 + r) * p.hq + h) * 128 + d0;
+            } else {
+              const int kvh = is_k ? h - p.hq : h - p.hq - p.hkv;
+              __nv_bfloat16* pool = is_k ? p.k_pool : p.v_pool;
+              dst[u] = pool + ((static_cast<size_t>(id) * p.hkv + kvh) * p.page + pos % p.page) * 128 + d0;
             }
           }
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (!dstoff_ok[u]) continue;  // uniform across the warp
-            if (is_q || is_k) {
-              float ss = 0.f;
-#pragma unroll
-              for (int j = 0; j < 4; ++j) ss += v[u][j] * v[u][j];
-              ss = warp_sum(ss);
-              const float inv = rsqrtf(ss / 128.f + p.eps);
+          for (int u = 0; u < kAtOnce; ++u) {
+            if (is_q || is_k) {  // uniform; all lanes take part in the sums
+              float v[4][4], ss[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                const float nrm = __bfloat162float(__float2bfloat16(v[u][j] * inv));
-                v[u][j] = __bfloat162float(__float2bfloat16(nwf[j] * nrm));
+                unpack_bf16x4(raw[u][j], v[j]);
+#pragma unroll
+                for (int b = 0; b < 4; ++b) ss[b] += v[j][b] * v[j][b];
               }
-              float rot[4];
+#pragma unroll
+              for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) ss[b] += __shfl_xor_sync(0xffffffffu, ss[b], o);
+              const float inv = rsqrtf(((ss[0] + ss[2]) + (ss[1] + ss[3])) / 128.f + p.eps);
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                  const float nrm = __bfloat162float(__float2bfloat16(v[j][b] * inv));
+                  v[j][b] = __bfloat162float(__float2bfloat16(nwf[j][b] * nrm));
+                }
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                const int jp = (j + 2) & 3;  // partner element d +- 64 lives in the same lane
-                const float other = j < 2 ? -v[u][jp] : v[u][jp];
-                rot[j] = v[u][j] * cs[u][j] + other * sn[u][j];
-              }
+                float c4[4], s4[4], rot[4];
+                unpack_bf16x4(cs[u][j], c4);
+                unpack_bf16x4(sn[u][j], s4);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) v[u][j] = rot[j];
+                for (int b = 0; b < 4; ++b) {
+                  const float other = j < 2 ? -v[(j + 2) & 3][b] : v[(j + 2) & 3][b];
+                  rot[b] = v[j][b] * c4[b] + other * s4[b];
+                }
+                raw[u][j] = make_uint2(pack_bf16x2(rot[0], rot[1]), pack_bf16x2(rot[2], rot[3]));
+              }
             }
+            if (dst[u] != nullptr) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dst[u][lane + 32 * j] = __float2bfloat16(v[u][j]);
+              for (int j = 0; j < 4; ++j) store_bf16x4(dst[u] + 32 * j, raw[u][j], p.wide);
+            }
           }
         }
         asm volatile("bar.sync 1, 256;" ::: "memory");  // the head tile may be overwritten by the next item
@@ -922,9 +996,13 @@ static int plan_dense(int M, int n_tiles, int k_blocks, int sms, size_t workspac
 }
 
 template <int A_TILES, int EPI>
-static int launch_dense(const CUtensorMap& w_map, const CUtensorMap& x_map, const DenseParams& p, int grid,
-                        cudaStream_t st) {
+static int launch_dense(const CUtensorMap& w_map, const CUtensorMap& x_map, DenseParams p, int grid, cudaStream_t st) {
   using Cfg = DenseCfg<A_TILES, EPI>;
+  p.stages = Cfg::stages(p.xbox);
+  // W's share of L2 while the kernel before runs: at most half of it, and where row tiles share a W tile it comes once anyway
+  const int k_blocks = (p.K + kDenseBlockK - 1) / kDenseBlockK / p.ksplit;
+  const int fits = (64 << 20) / (grid * A_TILES * kDenseWBytes);
+  p.prefetch = p.m_tiles == 1 && p.tiles == nullptr ? (k_blocks < fits ? k_blocks : fits) : 0;
   const void* fn = reinterpret_cast<const void*>(&dense_gemm_kernel<A_TILES, EPI>);
   int rc = ensure_dynamic_smem(fn, Cfg::kSmemBytes);
   if (rc) return rc;
@@ -1326,6 +1404,9 @@ extern "C" int b200_qkv_rope_append_gemm(const void* x, const void* wqkv, const 
   p.num_blocks = num_blocks;
   p.max_pages = max_pages_per_seq;
   p.max_pos = max_positions;
+  p.wide = ((reinterpret_cast<uintptr_t>(q_norm_weight) | reinterpret_cast<uintptr_t>(k_norm_weight) |
+             reinterpret_cast<uintptr_t>(cos_table) | reinterpret_cast<uintptr_t>(sin_table) |
+             reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool)) & 7) == 0;
   CUtensorMap w_map, x_map;
   rc = get_tensor_map_2d(wqkv, p.N, in_features, 2, 128, 64, &w_map);
   if (rc) return rc;

@@ -147,6 +147,25 @@ def test_qkv_projection_with_norm_rope_and_page_write_equals_the_two_kernels(ops
     assert not torch.equal(k1, pools[0])  # something was written
 
 
+@pytest.mark.parametrize("R", [1, 33, 200])
+def test_qkv_projection_takes_tables_and_norms_at_any_element(ops, R):
+    """Norm weights and tables that begin at an odd element (2-byte aligned) give the bits of aligned ones."""
+    hq, hkv, K, D, pages = 8, 2, 256, 128, 16
+    g = torch.Generator().manual_seed(R)
+    x = torch.randn(R, K, generator=g).bfloat16().to(DEV)
+    w = (torch.randn((hq + 2 * hkv) * D, K, generator=g) * 0.05).bfloat16().to(DEV)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV)[None].expand(R, -1).contiguous()
+    pos = torch.arange(R, dtype=torch.int32, device=DEV)
+    loose = [torch.randn(n * D + 1, generator=g).bfloat16().to(DEV)[1:].view(n, D) for n in (1, 1, 16 * pages, 16 * pages)]
+    outs = []
+    for qn, kn, cos, sin in (loose, [t.clone() for t in loose]):
+        kp, vp = (torch.zeros(pages, hkv, 16, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        q = ops.qkv_rope_append_gemm(x, w, qn.view(-1), kn.view(-1), cos, sin, pos, table, kp, vp, hq, 1e-6)
+        outs.append((q, kp, vp))
+    assert loose[0].data_ptr() % 8 == 2
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
 def test_qkv_projection_epilogue_reports_bad_positions_and_pages(ops):
     R, hq, hkv, K, D = 4, 32, 4, 2048, 128
     g = torch.Generator().manual_seed(0)
