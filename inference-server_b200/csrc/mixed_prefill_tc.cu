@@ -63,16 +63,6 @@ struct MixedPrefillParams {
 __host__ __device__ constexpr uint32_t mp_idesc(uint32_t n, uint32_t b_mn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn << 16) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
-// Issued by a converged warp: one elected lane sends the instruction, and the descriptors, the same in all lanes, can stay in
-// uniform registers (a branch on the lane number around the loop costs more than the instructions themselves).
-__device__ __forceinline__ void mp_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p, e;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc)
-      : "memory");
-}
 // A from TMEM: lane = row, a 32-bit column = two neighbouring K elements.
 __device__ __forceinline__ void mp_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile(
@@ -81,17 +71,6 @@ __device__ __forceinline__ void mp_mma_ts(uint32_t d, uint32_t a, uint64_t b, ui
       "setp.ne.b32 p, %4, 0;\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc)
       : "memory");
-}
-__device__ __forceinline__ void mp_commit(uint32_t bar) {
-  asm volatile(
-      "{\n\t.reg .pred e;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar)
-      : "memory");
-}
-// A wait of a whole warp, true if it has not run out for any lane.
-__device__ __forceinline__ bool mp_wait_all(uint32_t bar, uint32_t parity, int* err) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err));
 }
 // Operand descriptors, 128-byte swizzle.  MN-major (16 K rows of it): the next 8 K rows are 1024 bytes, the next 64 columns 2048
 // bytes further.  K-major: groups of 8 rows are `sbo` bytes apart.
@@ -225,7 +204,7 @@ mixed_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
     if (QTMEM && warp == 0) {  // the raw queries of all heads, a box per 64-wide piece: rows position x head
 #pragma unroll 1
       for (int s0 = 0; s0 < p.k_chunks && alive; s0 += p.nc) {
-        alive = mp_wait_all(bar_kempty + 8 * slot, kphase, p.err);
+        alive = mbar_wait_warp(bar_kempty + 8 * slot, kphase, p.err);
         if (!alive) break;
         if (lane == 0) mbar_arrive_expect_tx(bar_kfull + 8 * slot, static_cast<uint32_t>(p.nc * QT * per) * 128u);
         __syncwarp();
@@ -255,7 +234,7 @@ mixed_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
         const int my_page = __shfl_sync(0xffffffffu, page, (lane >> 1) & 7);  // lanes 0-15: half a page each
 #pragma unroll 1
         for (int s0 = 0; s0 < p.k_chunks; s0 += p.nc) {
-          alive = mp_wait_all(bar_kempty + 8 * slot, kphase, p.err);
+          alive = mbar_wait_warp(bar_kempty + 8 * slot, kphase, p.err);
           if (!alive) break;
           if (lane == 0) mbar_arrive_expect_tx(bar_kfull + 8 * slot, stage_bytes);
           __syncwarp();
@@ -268,7 +247,7 @@ mixed_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
           }
         }
       } else {
-        alive = mp_wait_all(bar_vempty, (j & 1) ^ 1, p.err);
+        alive = mbar_wait_warp(bar_vempty, (j & 1) ^ 1, p.err);
         if (!alive) break;
         if (lane == 0) mbar_arrive_expect_tx(bar_vfull, kVChunks * kMpChunk);
         __syncwarp();
@@ -288,44 +267,44 @@ mixed_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
       int round = 0, c = 0, cc = 0;
 #pragma unroll 1
       for (int s0 = 0; s0 < p.k_chunks && alive; s0 += p.nc) {
-        alive = mp_wait_all(bar_kfull + 8 * slot, kphase, p.err);
+        alive = mbar_wait_warp(bar_kfull + 8 * slot, kphase, p.err);
 #pragma unroll 1
         for (int i = 0; i < p.nc && alive; ++i) {
-          if (cc == 0) alive = mp_wait_all(bar_a, c & 1, p.err);
-          if ((cc & 1) == 0 && round > 0 && alive) alive = mp_wait_all(bar_rempty, (round - 1) & 1, p.err);
+          if (cc == 0) alive = mbar_wait_warp(bar_a, c & 1, p.err);
+          if ((cc & 1) == 0 && round > 0 && alive) alive = mbar_wait_warp(bar_rempty, (round - 1) & 1, p.err);
           if (!alive) break;
           tc_fence_after();
           const uint64_t b = mp_desc_mn(k_sm + slot * stage_bytes + i * kMpChunk);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            mp_mma_ss(tmem_base + s_col + (cc & 1) * 64, q_desc + (kk >> 2) * (kMpChunk >> 4) + 2 * (kk & 3), b + kk * (2048 >> 4),
+            tc_mma_f16_elected(tmem_base + s_col + (cc & 1) * 64, q_desc + (kk >> 2) * (kMpChunk >> 4) + 2 * (kk & 3), b + kk * (2048 >> 4),
                       idesc_mix, kk > 0 ? 1u : 0u);
           const bool last = cc + 1 == p.dk_chunks;
           if ((cc & 1) != 0 || last) {
-            mp_commit(bar_rfull);
+            tc_commit_elected(bar_rfull);
             ++round;
           }
           cc = last ? 0 : cc + 1;
           c += last ? 1 : 0;
         }
-        mp_commit(bar_kempty + 8 * slot);
+        tc_commit_elected(bar_kempty + 8 * slot);
         if (++slot == static_cast<uint32_t>(p.stages)) {
           slot = 0;
           kphase ^= 1;
         }
       }
-      if (alive) alive = mp_wait_all(bar_rempty, (round - 1) & 1, p.err);  // the last of Q' is in place
+      if (alive) alive = mbar_wait_warp(bar_rempty, (round - 1) & 1, p.err);  // the last of Q' is in place
     } else {
-      alive = mp_wait_all(bar_q, 0, p.err);
+      alive = mbar_wait_warp(bar_q, 0, p.err);
     }
     auto scores = [&](int t) {
       const int sb = s_bufs == 2 ? t & 1 : 0;
       const uint32_t ph = (s_bufs == 2 ? t >> 1 : t) & 1, s_acc = tmem_base + s_col + sb * kMpKeys;
-      if (alive) alive = mp_wait_all(bar_sempty + 8 * sb, ph ^ 1, p.err);
-      if (kAlias && t >= 2 && alive) alive = mp_wait_all(bar_odone, (t - 2) & 1, p.err);  // P(t - 2) lies there
+      if (alive) alive = mbar_wait_warp(bar_sempty + 8 * sb, ph ^ 1, p.err);
+      if (kAlias && t >= 2 && alive) alive = mbar_wait_warp(bar_odone, (t - 2) & 1, p.err);  // P(t - 2) lies there
 #pragma unroll 1
       for (int c = 0; c < p.k_chunks && alive; c += p.nc) {
-        alive = mp_wait_all(bar_kfull + 8 * slot, kphase, p.err);
+        alive = mbar_wait_warp(bar_kfull + 8 * slot, kphase, p.err);
         if (!alive) break;
         tc_fence_after();
 #pragma unroll 1
@@ -335,34 +314,34 @@ mixed_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             if (QTMEM) mp_mma_ts(s_acc, tmem_base + q_col + (c + i) * 32 + k * 8, b0 + 2 * k, idesc_s, (c + i + k) > 0 ? 1u : 0u);
-            else mp_mma_ss(s_acc, a0 + 2 * k, b0 + 2 * k, idesc_s, (c + i + k) > 0 ? 1u : 0u);
+            else tc_mma_f16_elected(s_acc, a0 + 2 * k, b0 + 2 * k, idesc_s, (c + i + k) > 0 ? 1u : 0u);
           }
         }
-        mp_commit(bar_kempty + 8 * slot);
+        tc_commit_elected(bar_kempty + 8 * slot);
         if (++slot == static_cast<uint32_t>(p.stages)) {
           slot = 0;
           kphase ^= 1;
         }
       }
-      if (alive) mp_commit(bar_sfull + 8 * sb);
+      if (alive) tc_commit_elected(bar_sfull + 8 * sb);
     };
     scores(0);
 #pragma unroll 1
     for (int j = 0; j < n_tiles && alive; ++j) {
       if (j + 1 < n_tiles) scores(j + 1);
-      if (alive) alive = mp_wait_all(bar_vfull, j & 1, p.err);
-      if (alive) alive = mp_wait_all(bar_pfull, j & 1, p.err);
+      if (alive) alive = mbar_wait_warp(bar_vfull, j & 1, p.err);
+      if (alive) alive = mbar_wait_warp(bar_pfull, j & 1, p.err);
       if (!alive) break;
       tc_fence_after();
       const uint32_t pa = tmem_base + (kAlias ? static_cast<uint32_t>((j & 1) * kMpKeys) : 448u);
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
         const uint64_t b = v_desc + kk * ((kVChunks * 2048) >> 4);  // a page
-        if (QTMEM) mp_mma_ss(tmem_o, q_desc + (kk >> 2) * (kMpChunk >> 4) + 2 * (kk & 3), b, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+        if (QTMEM) tc_mma_f16_elected(tmem_o, q_desc + (kk >> 2) * (kMpChunk >> 4) + 2 * (kk & 3), b, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
         else mp_mma_ts(tmem_o, pa + kk * 8, b, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
       }
-      mp_commit(bar_odone);
-      mp_commit(bar_vempty);
+      tc_commit_elected(bar_odone);
+      tc_commit_elected(bar_vempty);
     }
   } else if (warp == 2) {
     // ------------------------------------------- slices of the distance table ------
@@ -372,7 +351,7 @@ mixed_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
     const int span = kMpKeys + QT - 1;
 #pragma unroll 1
     for (int j = 0; j < n_tiles && alive; ++j) {
-      alive = mp_wait_all(bar_bempty + 8 * (j & 1), ((j >> 1) & 1) ^ 1, p.err);
+      alive = mbar_wait_warp(bar_bempty + 8 * (j & 1), ((j >> 1) & 1) ^ 1, p.err);
       if (!alive) break;
       const int at = kDistPad + p0 - (kt0 + j) * kMpKeys - (kMpKeys - 1);
       const uint32_t bytes = static_cast<uint32_t>(((at & 3) + span + 3) & ~3) * 4u;

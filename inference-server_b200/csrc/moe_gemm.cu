@@ -106,6 +106,12 @@ moe_fp8_gemm_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_cons
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  if (threadIdx.x == 64) {  // warm the descriptor cache while the barriers and TMEM are being set up
+    tma_prefetch_desc(&a_map);
+    tma_prefetch_desc(&a_map64);
+    tma_prefetch_desc(&a_map32);
+    tma_prefetch_desc(&b_map);
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < kGemmStages; ++s) {
       mbar_init(bar_full + 8 * s, 1);
@@ -139,75 +145,67 @@ moe_fp8_gemm_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_cons
   asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
   if (warp == 0) {
     // ------------------------------------------------------------ TMA ------
-    if (lane == 0) {
-      tma_prefetch_desc(&a_map);
-      tma_prefetch_desc(&a_map64);
-      tma_prefetch_desc(&a_map32);
-      tma_prefetch_desc(&b_map);
-      uint32_t it = 0;
-      bool alive = true;
-      for (int w = blockIdx.x; w < total && alive; w += gridDim.x) {
-        const MoeTile tile = p.tiles[w / p.n_tiles];
-        if (!tile_ok(tile, p)) {
-          set_error(p.err, kErrDevBadExpert);
-          continue;
-        }
-        const int j = w % p.n_tiles;
-        // the two 128-row blocks of W this tile multiplies with: block index inside the expert
-        int nb0, nb1;
-        if (MODE == kModeGateUp) {
-          nb0 = j;
-          nb1 = p.inter / 128 + j;
-        } else {
-          nb0 = 2 * j;
-          nb1 = 2 * j + 1;
-        }
-        const int sblocks = p.n_rows / 128;
-        // row-major weights: block (nb, kb) starts at row expert*n_rows + nb*128, column kb*128;
-        // tiled weights: it is the contiguous 16 KiB block number (expert*sblocks + nb)*k_blocks + kb
-        const int b_row0 = p.tiled ? (tile.expert * sblocks + nb0) * p.k_blocks * 128 : tile.expert * p.n_rows + nb0 * 128;
-        const int b_row1 = p.tiled ? (tile.expert * sblocks + nb1) * p.k_blocks * 128 : tile.expert * p.n_rows + nb1 * 128;
-        // The A box only needs the tile's own rows.  The MMA still reads 128 rows of the stage; what an earlier
-        // tile left in the rows below the box only reaches accumulator rows that are never stored.
-        const CUtensorMap* amap = tile.rows <= 32 ? &a_map32 : (tile.rows <= 64 ? &a_map64 : &a_map);
-        const uint32_t stage_bytes = (tile.rows <= 32 ? 32u : (tile.rows <= 64 ? 64u : 128u)) * kBlockK + kBBytes;
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
-          const uint32_t slot = it % kGemmStages, phase = (it / kGemmStages) & 1;
-          alive = mbar_wait(bar_empty + 8 * slot, phase ^ 1, p.err);
-          if (!alive) break;
-          const uint32_t sa = ring + slot * kStageBytesG, sb = sa + kABytes;
-          mbar_arrive_expect_tx(bar_full + 8 * slot, stage_bytes);
-          tma_load_2d(sa, amap, bar_full + 8 * slot, kb * kBlockK, tile.row0);
-          const int bx = p.tiled ? 0 : kb * kBlockK, by = p.tiled ? kb * 128 : 0;
-          tma_load_2d(sb, &b_map, bar_full + 8 * slot, bx, b_row0 + by);
-          tma_load_2d(sb + kBBytes / 2, &b_map, bar_full + 8 * slot, bx, b_row1 + by);
-        }
+    uint32_t it = 0;
+    bool alive = true;
+    for (int w = blockIdx.x; w < total && alive; w += gridDim.x) {
+      const MoeTile tile = p.tiles[w / p.n_tiles];
+      if (!tile_ok(tile, p)) {
+        set_error(p.err, kErrDevBadExpert);
+        continue;
+      }
+      const int j = w % p.n_tiles;
+      // the two 128-row blocks of W this tile multiplies with: block index inside the expert
+      int nb0, nb1;
+      if (MODE == kModeGateUp) {
+        nb0 = j;
+        nb1 = p.inter / 128 + j;
+      } else {
+        nb0 = 2 * j;
+        nb1 = 2 * j + 1;
+      }
+      const int sblocks = p.n_rows / 128;
+      // row-major weights: block (nb, kb) starts at row expert*n_rows + nb*128, column kb*128;
+      // tiled weights: it is the contiguous 16 KiB block number (expert*sblocks + nb)*k_blocks + kb
+      const int b_row0 = p.tiled ? (tile.expert * sblocks + nb0) * p.k_blocks * 128 : tile.expert * p.n_rows + nb0 * 128;
+      const int b_row1 = p.tiled ? (tile.expert * sblocks + nb1) * p.k_blocks * 128 : tile.expert * p.n_rows + nb1 * 128;
+      // The A box only needs the tile's own rows.  The MMA still reads 128 rows of the stage; what an earlier
+      // tile left in the rows below the box only reaches accumulator rows that are never stored.
+      const CUtensorMap* amap = tile.rows <= 32 ? &a_map32 : (tile.rows <= 64 ? &a_map64 : &a_map);
+      const uint32_t stage_bytes = (tile.rows <= 32 ? 32u : (tile.rows <= 64 ? 64u : 128u)) * kBlockK + kBBytes;
+      for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+        const uint32_t slot = it % kGemmStages, phase = (it / kGemmStages) & 1;
+        alive = mbar_wait_warp(bar_empty + 8 * slot, phase ^ 1, p.err);
+        if (!alive) break;
+        const uint32_t sa = ring + slot * kStageBytesG, sb = sa + kABytes;
+        mbar_arrive_expect_tx_elected(bar_full + 8 * slot, stage_bytes);
+        tma_load_2d_elected(sa, amap, bar_full + 8 * slot, kb * kBlockK, tile.row0);
+        const int bx = p.tiled ? 0 : kb * kBlockK, by = p.tiled ? kb * 128 : 0;
+        tma_load_2d_elected(sb, &b_map, bar_full + 8 * slot, bx, b_row0 + by);
+        tma_load_2d_elected(sb + kBBytes / 2, &b_map, bar_full + 8 * slot, bx, b_row1 + by);
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA ------
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_f8(kTileM, kTileN);
-      uint32_t it = 0;
-      bool alive = true;
-      for (int w = blockIdx.x; w < total && alive; w += gridDim.x) {
-        if (!tile_ok(p.tiles[w / p.n_tiles], p)) continue;
-        for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
-          const uint32_t slot = it % kGemmStages, phase = (it / kGemmStages) & 1;
-          const uint32_t buf = it & 1, aphase = (it >> 1) & 1;
-          alive = mbar_wait(bar_full + 8 * slot, phase, p.err);
-          alive = alive && mbar_wait(bar_tempty + 8 * buf, aphase ^ 1, p.err);
-          if (!alive) break;
-          tc_fence_after();
-          const uint32_t sa = ring + slot * kStageBytesG, sb = sa + kABytes;
-          const uint64_t a_desc = umma_desc_k128(sa), b_desc = umma_desc_k128(sb);
-          const uint32_t d = tmem_base + buf * kTileN;
+    constexpr uint32_t idesc = umma_idesc_f8(kTileM, kTileN);
+    uint32_t it = 0;
+    bool alive = true;
+    for (int w = blockIdx.x; w < total && alive; w += gridDim.x) {
+      if (!tile_ok(p.tiles[w / p.n_tiles], p)) continue;
+      for (int kb = 0; kb < p.k_blocks; ++kb, ++it) {
+        const uint32_t slot = it % kGemmStages, phase = (it / kGemmStages) & 1;
+        const uint32_t buf = it & 1, aphase = (it >> 1) & 1;
+        alive = mbar_wait_warp(bar_full + 8 * slot, phase, p.err);
+        alive = alive && mbar_wait_warp(bar_tempty + 8 * buf, aphase ^ 1, p.err);
+        if (!alive) break;
+        tc_fence_after();
+        const uint32_t sa = ring + slot * kStageBytesG, sb = sa + kABytes;
+        const uint64_t a_desc = umma_desc_k128(sa), b_desc = umma_desc_k128(sb);
+        const uint32_t d = tmem_base + buf * kTileN;
 #pragma unroll
-          for (int k = 0; k < kBlockK / 32; ++k)
-            tc_mma_f8(d, a_desc + 2 * k, b_desc + 2 * k, idesc, k > 0 ? 1u : 0u);
-          tc_commit(bar_empty + 8 * slot);
-          tc_commit(bar_tfull + 8 * buf);
-        }
+        for (int k = 0; k < kBlockK / 32; ++k)
+          tc_mma_f8_elected(d, a_desc + 2 * k, b_desc + 2 * k, idesc, k > 0 ? 1u : 0u);
+        tc_commit_elected(bar_empty + 8 * slot);
+        tc_commit_elected(bar_tfull + 8 * buf);
       }
     }
   }
