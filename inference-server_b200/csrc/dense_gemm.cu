@@ -35,9 +35,11 @@
 //               times slower: about 12 bytes per clock per SM against the 128 KiB each CTA must move.)
 //               The split is chosen so that all clusters of the launch are resident at once
 //               (cudaOccupancyMaxActiveClusters).
-//   two tiles   lm_head has 1187 weight tiles and needs no split; there a CTA takes two adjacent
-//               128-row tiles of W against one X box (two accumulators), which halves how often X
-//               is pulled from L2, and walks its share of the vocabulary persistently.
+//   one pass    lm_head has 1187 weight tiles and needs no split; a CTA walks its share of them persistently, the
+//               accumulators alternating, so that one tile's arg-max (and logits) overlap the next tile's MMAs.  (Two
+//               tiles per item, one X box for both, fill TMEM: nothing overlaps, and 594 items leave 2 of 148 CTAs a
+//               fifth round: 256 rows with logits 256 us that way, 155 us this way; one row 102 us
+//               either way.)
 //
 // Groups: a launch may cover several independent products that sit side by side (one per attention head): group g
 // multiplies the columns [g * x_step, + K) of X with the weight rows [g * w_step, + N) into the columns
@@ -1432,11 +1434,11 @@ static int lm_head_any(const void* x, const void* w, int64_t* next_tokens, __nv_
   p.N = vocab_size;
   p.K = hidden;
   p.m_tiles = 1;
-  p.n_tiles = (vocab_size + 255) / 256;
+  p.n_tiles = (vocab_size + 127) / 128;
   p.xbox = pick_xbox(num_rows);
   p.ksplit = 1;
   const int grid = p.n_tiles < sms ? p.n_tiles : (sms < 256 ? sms : 256);
-  B200_REQUIRE((p.n_tiles + grid - 1) / grid <= 16, "lm_head_argmax: vocabulary of %d needs more than 32 weight tiles "
+  B200_REQUIRE((p.n_tiles + grid - 1) / grid <= 32, "lm_head_argmax: vocabulary of %d needs more than 32 weight tiles "
                "per CTA on this device", vocab_size);
   p.part_val = static_cast<float*>(workspace);
   p.part_idx = reinterpret_cast<int*>(static_cast<uint8_t*>(workspace) + static_cast<size_t>(256) * 4 * kDenseMaxRows * 4);
@@ -1445,7 +1447,7 @@ static int lm_head_any(const void* x, const void* w, int64_t* next_tokens, __nv_
   if (rc) return rc;
   rc = get_tensor_map_2d(x, num_rows, hidden, 2, p.xbox, 64, &x_map);
   if (rc) return rc;
-  rc = launch_dense<2, kEpiArgmax>(w_map, x_map, p, grid, as_stream(stream));
+  rc = launch_dense<1, kEpiArgmax>(w_map, x_map, p, grid, as_stream(stream));
   if (rc) return rc;
   B200_CUDA(launch_overlapped(argmax_fold_kernel, dim3((num_rows + 3) / 4), dim3(128), 0, as_stream(stream), p.part_val,
                               p.part_idx, grid, num_rows, reinterpret_cast<long long*>(next_tokens)));
