@@ -122,17 +122,20 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, in
   set_error(err, kErrDevWaitTimeout);
   return false;
 }
-// The *_elected forms are called by a converged warp and sent by one lane of it, always the same one.  Loops that issue TMA copies
-// or tensor-core instructions are written with them and not inside a branch on the lane number: there the compiler cannot know
-// that a single thread is active and wraps every such instruction, whose operands are the warp's, in code that serialises
-// lanes.  A K block of dense_gemm.cu (a wait, four MMAs, a commit) then takes about 500 cycles to issue, more than its MMAs
-// take at any width.
-__device__ __forceinline__ void mbar_arrive_expect_tx_elected(uint32_t bar, uint32_t bytes) {
+// One lane of a converged warp, always the same one.  Loops that issue TMA copies or tensor-core instructions run inside
+// if (elect_one()) and not inside a branch on the lane number: from this form the compiler knows that a single thread is active,
+// from the other it does not and wraps every such instruction, whose operands are the warp's, in code that serialises
+// lanes.  A K block of dense_gemm.cu (a wait, four MMAs, a commit) then took about 500 cycles to issue, more than its
+// MMAs take at any width.  (Issuing from all lanes with an elected lane per instruction is as cheap to issue, but 32 lanes
+// then poll every barrier: the FP8 expert products at 4096 tokens took 150 + 122 us against 146 + 119 us.)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
   asm volatile(
-      "{\n\t.reg .pred e;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes)
-      : "memory");
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(e));
+  return e != 0;
 }
 
 // --------------------------------------------------------------------- TMA --
@@ -145,14 +148,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
       "[%0], [%1, {%3, %4}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_elected(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-  asm volatile(
-      "{\n\t.reg .pred e;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "@e cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
 // Asks a 2-D box of global memory into L2; a hint, nothing waits for it.
@@ -227,8 +222,14 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// Arrives once on `bar` when every tcgen05.mma issued so far by the elected thread has finished (implies
-// tcgen05.fence::before_thread_sync).
+// Arrives once on `bar` when every tcgen05.mma issued so far by this thread has
+// finished (implies tcgen05.fence::before_thread_sync).
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                   bar)
+               : "memory");
+}
+// The same from a converged warp, by its elected lane.
 __device__ __forceinline__ void tc_commit_elected(uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred e;\n\t"
@@ -237,17 +238,25 @@ __device__ __forceinline__ void tc_commit_elected(uint32_t bar) {
       : "memory");
 }
 // D[tmem] (+)= A[smem] * B[smem], e4m3 x e4m3 -> f32, one K=32 slice.
-__device__ __forceinline__ void tc_mma_f8_elected(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                  uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                          uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
+      "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc),
-      "r"(accumulate)
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // f16 x f16 or bf16 x bf16 -> f32 (the instruction descriptor says which), one K=16 slice.
+__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 __device__ __forceinline__ void tc_mma_f16_elected(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                    uint32_t accumulate) {
   asm volatile(

@@ -309,60 +309,64 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA ------
-    uint32_t slot = 0, phase = 0;
-    bool alive = true;
-    for (int w = blockIdx.x; w < total && alive; w += gridDim.x) {
-      const int tile = w / ks, kidx = w - tile * ks;
-      const DenseItem item = dense_item(p, tile);
-      const int g = item.g, nt = item.nt;
-      for (int kb = 0; kb < kb_per; ++kb) {
-        alive = mbar_wait_warp(bar_empty + 8 * slot, phase ^ 1, p.err);
-        if (!alive) break;
-        const uint32_t sw = ring + slot * stage_bytes, sx = sw + A_TILES * kDenseWBytes;
-        const int kx = (kidx * kb_per + kb) * kDenseBlockK;
-        mbar_arrive_expect_tx_elected(bar_full + 8 * slot, stage_tx);
+    if (elect_one()) {
+      uint32_t slot = 0, phase = 0;
+      bool alive = true;
+      for (int w = blockIdx.x; w < total && alive; w += gridDim.x) {
+        const int tile = w / ks, kidx = w - tile * ks;
+        const DenseItem item = dense_item(p, tile);
+        const int g = item.g, nt = item.nt;
+        for (int kb = 0; kb < kb_per; ++kb) {
+          alive = mbar_wait(bar_empty + 8 * slot, phase ^ 1, p.err);
+          if (!alive) break;
+          const uint32_t sw = ring + slot * stage_bytes, sx = sw + A_TILES * kDenseWBytes;
+          const int kx = (kidx * kb_per + kb) * kDenseBlockK;
+          mbar_arrive_expect_tx(bar_full + 8 * slot, stage_tx);
 #pragma unroll
-        for (int a = 0; a < A_TILES; ++a)
-          tma_load_2d_elected(sw + a * kDenseWBytes, &w_map, bar_full + 8 * slot, kx,
-                      g * p.w_step + (nt * A_TILES + a) * 128);
-        tma_load_2d_elected(sx, &x_map, bar_full + 8 * slot, g * p.x_step + kx, item.m0);
-        if (++slot == stages) {
-          slot = 0;
-          phase ^= 1;
+          for (int a = 0; a < A_TILES; ++a)
+            tma_load_2d(sw + a * kDenseWBytes, &w_map, bar_full + 8 * slot, kx,
+                        g * p.w_step + (nt * A_TILES + a) * 128);
+          tma_load_2d(sx, &x_map, bar_full + 8 * slot, g * p.x_step + kx, item.m0);
+          if (++slot == stages) {
+            slot = 0;
+            phase ^= 1;
+          }
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA ------
-    const uint32_t idesc = umma_idesc_bf16(128, static_cast<uint32_t>(p.xbox));
-    uint32_t slot = 0, phase = 0, item = 0;
-    bool alive = true;
-    for (int w = blockIdx.x; w < total && alive; w += gridDim.x, ++item) {
-      const uint32_t buf = item % kBufs, aphase = (item / kBufs) & 1;
-      alive = mbar_wait_warp(bar_tempty + 8 * buf, aphase ^ 1, p.err);
-      if (!alive) break;
-      tc_fence_after();
-      for (int kb = 0; kb < kb_per; ++kb) {
-        alive = mbar_wait_warp(bar_full + 8 * slot, phase, p.err);
+    if (elect_one()) {
+      const uint32_t idesc = umma_idesc_bf16(128, static_cast<uint32_t>(p.xbox));
+      uint32_t slot = 0, phase = 0, item = 0;
+      bool alive = true;
+      for (int w = blockIdx.x; w < total && alive; w += gridDim.x, ++item) {
+        const uint32_t buf = item % kBufs, aphase = (item / kBufs) & 1;
+        alive = mbar_wait(bar_tempty + 8 * buf, aphase ^ 1, p.err);
         if (!alive) break;
         tc_fence_after();
-        const uint32_t sw = ring + slot * stage_bytes, sx = sw + A_TILES * kDenseWBytes;
-        const uint64_t b_desc = umma_desc_k128(sx);
+        for (int kb = 0; kb < kb_per; ++kb) {
+          alive = mbar_wait(bar_full + 8 * slot, phase, p.err);
+          if (!alive) break;
+          tc_fence_after();
+          const uint32_t sw = ring + slot * stage_bytes, sx = sw + A_TILES * kDenseWBytes;
+          const uint64_t b_desc = umma_desc_k128(sx);
 #pragma unroll
-        for (int a = 0; a < A_TILES; ++a) {
-          const uint64_t a_desc = umma_desc_k128(sw + a * kDenseWBytes);
-          const uint32_t d = tmem_base + (A_TILES == 1 ? buf : static_cast<uint32_t>(a)) * kDenseMaxRows;
+          for (int a = 0; a < A_TILES; ++a) {
+            const uint64_t a_desc = umma_desc_k128(sw + a * kDenseWBytes);
+            const uint32_t d = tmem_base + (A_TILES == 1 ? buf : static_cast<uint32_t>(a)) * kDenseMaxRows;
 #pragma unroll
-          for (int k = 0; k < kDenseBlockK / 16; ++k)
-            tc_mma_f16_elected(d, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < kDenseBlockK / 16; ++k)
+              tc_mma_f16(d, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          }
+          tc_commit(bar_empty + 8 * slot);
+          if (++slot == stages) {
+            slot = 0;
+            phase ^= 1;
+          }
         }
-        tc_commit_elected(bar_empty + 8 * slot);
-        if (++slot == stages) {
-          slot = 0;
-          phase ^= 1;
-        }
+        if (alive) tc_commit(bar_tfull + 8 * buf);
       }
-      if (alive) tc_commit_elected(bar_tfull + 8 * buf);
     }
   } else if (EPI == kEpiStore && ks > 1) {
     // ------------------------------------- epilogue, split K: wait only ------

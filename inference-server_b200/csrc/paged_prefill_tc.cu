@@ -230,54 +230,58 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __
     }
   } else if (warp == 1) {
     // ---------------------------------------------------- S = Q K^T ------
-    constexpr uint32_t idesc_s = tc_idesc_bf16(kTcRows, kTcKeys, 0);  // B = K, K-major
-    bool alive = mbar_wait_warp(bar_q, 0, err);
-    const uint64_t a0 = umma_desc_k128(q_sm);
+    if (elect_one()) {
+      constexpr uint32_t idesc_s = tc_idesc_bf16(kTcRows, kTcKeys, 0);  // B = K, K-major
+      bool alive = mbar_wait(bar_q, 0, err);
+      const uint64_t a0 = umma_desc_k128(q_sm);
 #pragma unroll 1
-    for (int t = 0; t < n_tiles && alive; ++t) {
-      const int st = t & 1;
-      const uint32_t ph = (t >> 1) & 1;
-      alive = mbar_wait_warp(bar_kfull + 8 * st, ph, err);
-      if (!alive) break;
-      alive = mbar_wait_warp(bar_sempty + 8 * st, ph ^ 1, err);  // the softmax warps have read tile t - 2
-      if (!alive) break;
-      tc_fence_after();
-      const uint64_t b0 = umma_desc_k128(k_sm + st * kTcTileBytes);
+      for (int t = 0; t < n_tiles && alive; ++t) {
+        const int st = t & 1;
+        const uint32_t ph = (t >> 1) & 1;
+        alive = mbar_wait(bar_kfull + 8 * st, ph, err);
+        if (!alive) break;
+        alive = mbar_wait(bar_sempty + 8 * st, ph ^ 1, err);  // the softmax warps have read tile t - 2
+        if (!alive) break;
+        tc_fence_after();
+        const uint64_t b0 = umma_desc_k128(k_sm + st * kTcTileBytes);
 #pragma unroll
-      for (int k = 0; k < D / 16; ++k) {  // 16 of the head dimensions each
-        const uint32_t off = ((k >> 2) * kTcHalfBytes + (k & 3) * 32) >> 4;
-        tc_mma_f16_elected(tmem_base + st * kTcKeys, a0 + off, b0 + off, idesc_s, k > 0 ? 1u : 0u);
+        for (int k = 0; k < D / 16; ++k) {  // 16 of the head dimensions each
+          const uint32_t off = ((k >> 2) * kTcHalfBytes + (k & 3) * 32) >> 4;
+          tc_mma_f16(tmem_base + st * kTcKeys, a0 + off, b0 + off, idesc_s, k > 0 ? 1u : 0u);
+        }
+        tc_commit(bar_sfull + 8 * st);
+        tc_commit(bar_kempty + 8 * st);
       }
-      tc_commit_elected(bar_sfull + 8 * st);
-      tc_commit_elected(bar_kempty + 8 * st);
     }
   } else if (warp == 2) {
     // ---------------------------------------------------- O += P V ------
-    constexpr uint32_t idesc_o = tc_idesc_bf16(kTcRows, D, 1);  // B = V, MN-major
-    const uint32_t tmem_o = tmem_base + 2 * kTcKeys;
-    bool alive = true;
+    if (elect_one()) {
+      constexpr uint32_t idesc_o = tc_idesc_bf16(kTcRows, D, 1);  // B = V, MN-major
+      const uint32_t tmem_o = tmem_base + 2 * kTcKeys;
+      bool alive = true;
 #pragma unroll 1
-    for (int j = 0; j < n_tiles && alive; ++j) {
-      const int st = j & 1;
-      alive = mbar_wait_warp(bar_vfull + 8 * st, (j >> 1) & 1, err);
-      if (!alive) break;
-      alive = mbar_wait_warp(bar_rescaled + 8 * (j & 1), (j >> 1) & 1, err);  // nobody is rewriting O any more
-      if (!alive) break;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        alive = mbar_wait_warp(bar_pfull + 8 * half, j & 1, err);
+      for (int j = 0; j < n_tiles && alive; ++j) {
+        const int st = j & 1;
+        alive = mbar_wait(bar_vfull + 8 * st, (j >> 1) & 1, err);
         if (!alive) break;
-        tc_fence_after();
-        const uint64_t a0 = umma_desc_k128(p_sm + half * kTcHalfBytes);
+        alive = mbar_wait(bar_rescaled + 8 * (j & 1), (j >> 1) & 1, err);  // nobody is rewriting O any more
+        if (!alive) break;
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {  // 16 keys each
-          const uint64_t b = umma_desc_mn128(v_sm + st * kTcTileBytes + (half * 4 + kk) * (16 * 128), kTcHalfBytes, 1024);
-          tc_mma_f16_elected(tmem_o, a0 + ((kk * 32) >> 4), b, idesc_o, (j > 0 || half > 0 || kk > 0) ? 1u : 0u);
+        for (int half = 0; half < 2; ++half) {
+          alive = mbar_wait(bar_pfull + 8 * half, j & 1, err);
+          if (!alive) break;
+          tc_fence_after();
+          const uint64_t a0 = umma_desc_k128(p_sm + half * kTcHalfBytes);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {  // 16 keys each
+            const uint64_t b = umma_desc_mn128(v_sm + st * kTcTileBytes + (half * 4 + kk) * (16 * 128), kTcHalfBytes, 1024);
+            tc_mma_f16(tmem_o, a0 + ((kk * 32) >> 4), b, idesc_o, (j > 0 || half > 0 || kk > 0) ? 1u : 0u);
+          }
+          tc_commit(bar_odone + 8 * half);
         }
-        tc_commit_elected(bar_odone + 8 * half);
+        if (!alive) break;
+        tc_commit(bar_vempty + 8 * st);
       }
-      if (!alive) break;
-      tc_commit_elected(bar_vempty + 8 * st);
     }
   } else {
     // -------------------------------------------------------- softmax ------
