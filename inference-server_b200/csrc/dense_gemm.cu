@@ -990,9 +990,12 @@ template <int A_TILES, int EPI>
 static int launch_dense(const CUtensorMap& w_map, const CUtensorMap& x_map, DenseParams p, int grid, cudaStream_t st) {
   using Cfg = DenseCfg<A_TILES, EPI>;
   p.stages = Cfg::stages(p.xbox);
-  // W's share of L2 while the kernel before runs: at most half of it, and where row tiles share a W tile it comes once anyway
+  // What a CTA asks of its W while the kernel before runs: 256 KB, about what the gap gives time for.  The requests share the
+  // copy engine's queue with the loads: all of a 1 MB item (12288 features, width 2048, one row) cost 16.6 us against
+  // 13.8 without any, while 256 KB items gain (4096 -> 2048, behind a small kernel: 7.7 against 8.4).  Where row tiles share
+  // a W tile it comes once anyway.
   const int k_blocks = (p.K + kDenseBlockK - 1) / kDenseBlockK / p.ksplit;
-  const int fits = (64 << 20) / (grid * A_TILES * kDenseWBytes);
+  constexpr int fits = (256 << 10) / (A_TILES * kDenseWBytes);
   p.prefetch = p.m_tiles == 1 && p.tiles == nullptr ? (k_blocks < fits ? k_blocks : fits) : 0;
   const void* fn = reinterpret_cast<const void*>(&dense_gemm_kernel<A_TILES, EPI>);
   int rc = ensure_dynamic_smem(fn, Cfg::kSmemBytes);
