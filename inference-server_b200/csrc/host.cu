@@ -113,12 +113,13 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 struct MapKey {
   int device;
   const void* base;
-  uint64_t dim[3];  // innermost first
+  uint64_t dim[4];  // innermost first
   int elem_bytes;
-  uint32_t box[3];
+  uint32_t box[4];
+  uint64_t stride[3];  // bytes, of dim[1..]
   bool operator==(const MapKey& o) const {
-    for (int i = 0; i < 3; ++i)
-      if (dim[i] != o.dim[i] || box[i] != o.box[i]) return false;
+    for (int i = 0; i < 4; ++i)
+      if (dim[i] != o.dim[i] || box[i] != o.box[i] || (i < 3 && stride[i] != o.stride[i])) return false;
     return device == o.device && base == o.base && elem_bytes == o.elem_bytes;
   }
 };
@@ -131,7 +132,7 @@ static std::mutex g_map_mu;
 static std::vector<MapEntry> g_maps;
 static EncodeTiledFn g_encode = nullptr;
 
-// Dense row-major tensor of `rank` 2 or 3 dimensions.
+// Tensor of `rank` 2 to 4 dimensions.
 static int get_tensor_map(int rank, MapKey key, CUtensorMap* out) {
   cudaError_t ce = cudaGetDevice(&key.device);
   if (ce != cudaSuccess) return cuda_fail(ce, "cudaGetDevice");
@@ -154,15 +155,15 @@ static int get_tensor_map(int rank, MapKey key, CUtensorMap* out) {
   }
   const unsigned long long cols = key.dim[0], rows = key.dim[1];
   if (key.box[0] * static_cast<uint32_t>(key.elem_bytes) != 128u || key.box[1] == 0 || key.box[1] > 256 || key.box[2] == 0 ||
-      key.box[2] > 256 || (reinterpret_cast<uintptr_t>(key.base) & 15) != 0 || (cols * key.elem_bytes) % 16 != 0) {
+      key.box[2] > 256 || key.box[3] == 0 || key.box[3] > 256 || (reinterpret_cast<uintptr_t>(key.base) & 15) != 0 || key.stride[0] % 16 != 0) {
     set_detail("tensor map: base %p rows %llu cols %llu elem %d box %ux%ux%u is not encodable", key.base, rows, cols,
                key.elem_bytes, key.box[2], key.box[1], key.box[0]);
     return -kErrTensorMap;
   }
-  cuuint64_t gdim[3] = {key.dim[0], key.dim[1], key.dim[2]};
-  cuuint64_t gstride[2] = {cols * static_cast<uint64_t>(key.elem_bytes), cols * rows * static_cast<uint64_t>(key.elem_bytes)};
-  cuuint32_t box[3] = {key.box[0], key.box[1], key.box[2]};
-  cuuint32_t estr[3] = {1, 1, 1};
+  cuuint64_t gdim[4] = {key.dim[0], key.dim[1], key.dim[2], key.dim[3]};
+  cuuint64_t gstride[3] = {key.stride[0], key.stride[1], key.stride[2]};
+  cuuint32_t box[4] = {key.box[0], key.box[1], key.box[2], key.box[3]};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
   MapEntry entry;
   entry.key = key;
   CUresult r = g_encode(&entry.map,
@@ -182,12 +183,30 @@ static int get_tensor_map(int rank, MapKey key, CUtensorMap* out) {
 
 int get_tensor_map_2d(const void* base, uint64_t rows, uint64_t cols, int elem_bytes,
                       uint32_t box_rows, uint32_t box_cols, CUtensorMap* out) {
-  return get_tensor_map(2, MapKey{0, base, {cols, rows, 1}, elem_bytes, {box_cols, box_rows, 1}}, out);
+  return get_tensor_map(2, MapKey{0, base, {cols, rows, 1, 1}, elem_bytes, {box_cols, box_rows, 1, 1}, {cols * elem_bytes, 0, 0}}, out);
 }
 
 int get_tensor_map_3d(const void* base, uint64_t planes, uint64_t rows, uint64_t cols, int elem_bytes, uint32_t box_planes,
                       uint32_t box_rows, uint32_t box_cols, CUtensorMap* out) {
-  return get_tensor_map(3, MapKey{0, base, {cols, rows, planes}, elem_bytes, {box_cols, box_rows, box_planes}}, out);
+  return get_tensor_map(3, MapKey{0, base, {cols, rows, planes, 1}, elem_bytes, {box_cols, box_rows, box_planes, 1},
+                                  {cols * elem_bytes, cols * rows * elem_bytes, 0}}, out);
+}
+
+int get_tensor_map_atoms(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out) {
+  const uint64_t pitch = cols * 2;
+  return get_tensor_map(4, MapKey{0, base, {64, 8, cols / 64, rows / 8}, 2, {64, 8, static_cast<uint32_t>(cols / 64), box_rows / 8},
+                                  {pitch, 128, 8 * pitch}}, out);
+}
+
+int get_tensor_map_columns(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out) {
+  return get_tensor_map(3, MapKey{0, base, {64, rows, cols / 64, 1}, 2, {64, box_rows, static_cast<uint32_t>(cols / 64), 1},
+                                  {cols * 2, 128, 0}}, out);
+}
+
+int get_tensor_map_atoms_of(const void* base, uint64_t planes, uint64_t rows, uint64_t cols, uint32_t box_planes, CUtensorMap* out) {
+  const uint64_t pitch = cols * 2;
+  return get_tensor_map(4, MapKey{0, base, {64, rows, cols / 64, planes}, 2, {64, 8, static_cast<uint32_t>(cols / 64), box_planes},
+                                  {pitch, 128, rows * pitch}}, out);
 }
 
 }  // namespace b200

@@ -32,6 +32,19 @@ int get_tensor_map_2d(const void* base, uint64_t rows, uint64_t cols, int elem_b
 int get_tensor_map_3d(const void* base, uint64_t planes, uint64_t rows, uint64_t cols, int elem_bytes, uint32_t box_planes,
                       uint32_t box_rows, uint32_t box_cols, CUtensorMap* out);
 
+// A bf16 [rows, cols] tensor (rows a multiple of 8, cols of 64) as swizzled atoms of 8 rows x 128 bytes: a box holds all columns
+// of `box_rows` rows (a multiple of 8), the atoms of 8 rows one after the other, then those of the next 8.  Coordinates:
+// (0, 0, 0, row / 8).
+int get_tensor_map_atoms(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out);
+
+// The same atoms for a dense [planes, rows, cols] tensor: a box holds all columns of 8 rows of `box_planes` planes.  Coordinates:
+// (0, row, 0, plane).
+int get_tensor_map_atoms_of(const void* base, uint64_t planes, uint64_t rows, uint64_t cols, uint32_t box_planes, CUtensorMap* out);
+
+// A bf16 [rows, cols] tensor (cols a multiple of 64): a box holds all columns of `box_rows` rows, 64 columns of all its rows
+// one after the other.  Coordinates: (0, row, 0).
+int get_tensor_map_columns(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, CUtensorMap* out);
+
 // Records the last CUDA error text for b200_last_error_detail().
 int cuda_fail(cudaError_t e, const char* where);
 void set_detail(const char* fmt, ...);

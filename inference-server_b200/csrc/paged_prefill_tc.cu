@@ -7,16 +7,18 @@
 //   grid     (query tiles, kv heads).  A CTA owns 128 rows of the score matrix: 128 / G consecutive prompt
 //            positions x the G query heads of its kv head, and walks the key tiles (128 keys = 8 pages) of
 //            the context up to its last position.  Heavy tiles (late positions) are issued first.
-//   warp 0   TMA producer: the Q tile once (boxes of G rows x 128 B), then per key tile the 8 K pages and
-//            the 8 V pages of the kv head (boxes of 16 tokens x 128 B, two column halves each) into two
-//            two-stage rings, 128-byte swizzle, mbarrier hand-over.  The 16 boxes of a tile are issued by 16
-//            lanes side by side.
+//   warp 0   TMA producer: the Q tile once, then per key tile the 8 K pages of the kv
+//            head into a two-stage ring; warp 11 does the same with V.  A page (16 tokens) is one box of 8-row
+//            swizzled atoms.  A TMA copy costs about 100 cycles to issue whatever its size, and 32 copies of
+//            2 KB per key tile from one warp were what the kernel waited for: 3300 cycles per key tile, with or
+//            without its exponentials, its products or its P stores. With a box per page and two warps
+//            1024 tokens behind 14 k, 32 / 4 heads: 400 -> 330 us, 2048 tokens in two chunks 47 -> 39 us each, 91
+//            tokens 12.9 -> 11.6 us.
 //   warp 1   score issuer (one thread): S = Q K^T as 8 x tcgen05.mma M128 N128 K16 (kind::f16, bf16, both
 //            operands K-major) into one of two S accumulators in TMEM, as far ahead as those allow.
 //   warp 2   P V issuer (one thread): O += P V as 2 x 4 tcgen05.mma M128 N128 K16, P (bf16, written by the
 //            softmax warps) as the K-major A operand and V as an MN-major B operand straight from its page
-//            layout [key][head_dim].  A thread gets a tcgen05.mma on its way about every 95 cycles whatever
-//            its N (measured), which is why the two products have an issuer each, and the P tile is handed
+//            layout [key][head_dim].  The P tile is handed
 //            over in two halves of 64 keys so that the first half's product starts while the second half's
 //            exponentials are still being taken.
 //   warps 3-10  softmax: a thread owns one score row and 64 of the tile's 128 key columns (two threads per
@@ -58,7 +60,7 @@ constexpr int kTcPages = kTcKeys / kTcPage;
 constexpr int kTcHalfBytes = 128 * 128;      // 128 rows x 64 bf16: one swizzled column half of a tile
 constexpr int kTcPBytes = 2 * kTcHalfBytes;  // P: 128 rows x 128 keys
 constexpr int kTcSoftmaxWarps = 8;
-constexpr int kTcThreads = (3 + kTcSoftmaxWarps) * 32;
+constexpr int kTcThreads = (4 + kTcSoftmaxWarps) * 32;
 constexpr int kTcExtraBytes = 256 /* barriers, tmem base */ + 2 * 2 * kTcRows * 4 /* max exchange */ +
                               2 * kTcRows * 4 /* sum exchange */;
 template <int D>
@@ -80,6 +82,16 @@ __device__ __forceinline__ uint64_t umma_desc_mn128(uint32_t smem_addr, uint32_t
   uint64_t d = 0;
   d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
   d |= static_cast<uint64_t>(lbo >> 4) << 16;
+  d |= static_cast<uint64_t>(sbo >> 4) << 32;
+  d |= static_cast<uint64_t>(1) << 46;  // descriptor version (sm_100)
+  d |= static_cast<uint64_t>(2) << 61;  // 128-byte swizzle
+  return d;
+}
+// Descriptor of a K-major operand tile of 8 x 128 B swizzled atoms; groups of 8 rows `sbo` bytes apart.
+__device__ __forceinline__ uint64_t tc_desc_k_atoms(uint32_t smem_addr, uint32_t sbo) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
+  d |= static_cast<uint64_t>(1) << 16;  // leading byte offset (unused)
   d |= static_cast<uint64_t>(sbo >> 4) << 32;
   d |= static_cast<uint64_t>(1) << 46;  // descriptor version (sm_100)
   d |= static_cast<uint64_t>(2) << 61;  // 128-byte swizzle
@@ -126,6 +138,8 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __
 #ifdef B200_DEVICE_OK
   constexpr int kTcTileBytes = TcCfg<D>::kTileBytes;
   constexpr int kHalves = D / 64;
+  constexpr int kTcPageBytes = kTcPage * D * 2;
+  constexpr uint32_t kAtomGroup = kHalves * 1024;  // Q, K and V: 8 rows x 128 B atoms of the same 8 rows side by side
   const int gr = G > 0 ? G : group;
   const int QT = kTcRows / gr;  // prompt positions per CTA
   extern __shared__ uint8_t smem_raw[];
@@ -192,22 +206,28 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA ------
-    // The first 8 * kHalves lanes each own one box of a tile: page lane / kHalves, column half lane % kHalves.
     if (G > 0) {
       if (lane == 0) mbar_arrive_expect_tx(bar_q, kTcTileBytes);
       __syncwarp();
-      for (int i = lane; i < kHalves * QT; i += 32) {
-        const int tl = i / kHalves, hf = i % kHalves;
-        tma_load_2d(q_sm + hf * kTcHalfBytes + tl * gr * 128, &q_map, bar_q, hf * 64,
-                    (t0 + tl) * num_q_heads + h * gr);  // rows past the chunk are filled with zeros
+      // rows past the chunk are filled with zeros
+      if (G == 8) {
+        if (lane == 0) tma_load_4d(q_sm, &q_map, bar_q, 0, h * 8, 0, t0);
+      } else if (lane < QT) {
+        tma_load_4d(q_sm + lane * (G / 8) * kAtomGroup, &q_map, bar_q, 0, 0, 0, ((t0 + lane) * num_q_heads + h * gr) / 8);
       }
     }
-    const int pg = (lane / kHalves) & 7, hf = lane % kHalves;
+  }
+  if (warp == 0 || warp == kTcSoftmaxWarps + 3) {
+    // -------------------------------------------- K (warp 0), V (warp 11) ------
+    // Lane i of the first 8 owns page i of a tile.
+    const bool is_k = warp == 0;
+    const uint32_t ring = is_k ? k_sm : v_sm, full = is_k ? bar_kfull : bar_vfull, empty = is_k ? bar_kempty : bar_vempty;
+    const CUtensorMap* map = is_k ? &k_map : &v_map;
+    const int pg = lane & 7;
     bool alive = true;
 #pragma unroll 1
     for (int j = 0; j < n_tiles; ++j) {
       const int st = j & 1;
-      const uint32_t ph = (j >> 1) & 1;
       // pages past the tile's last position hold nothing this CTA may read; the last valid page stands in so that
       // every stage is the same number of bytes and holds finite numbers (their scores are masked)
       int page = __ldg(table_row + min((kt0 + j) * kTcPages + pg, last_page));
@@ -215,25 +235,20 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __
         set_error(err, kErrDevBadBlockId);
         page = 0;
       }
-      const int row = (page * num_kv_heads + h) * kTcPage;
-      const uint32_t dst = st * kTcTileBytes + hf * kTcHalfBytes + pg * (kTcPage * 128);
-      if (alive) alive = mbar_wait(bar_kempty + 8 * st, ph ^ 1, err);
+      if (alive) alive = mbar_wait(empty + 8 * st, ((j >> 1) & 1) ^ 1, err);
       if (!__all_sync(0xffffffffu, alive)) break;
-      if (lane == 0) mbar_arrive_expect_tx(bar_kfull + 8 * st, kTcTileBytes);
+      if (lane == 0) mbar_arrive_expect_tx(full + 8 * st, kTcTileBytes);
       __syncwarp();
-      if (lane < 8 * kHalves) tma_load_2d(k_sm + dst, &k_map, bar_kfull + 8 * st, hf * 64, row);
-      if (alive) alive = mbar_wait(bar_vempty + 8 * st, ph ^ 1, err);
-      if (!__all_sync(0xffffffffu, alive)) break;
-      if (lane == 0) mbar_arrive_expect_tx(bar_vfull + 8 * st, kTcTileBytes);
-      __syncwarp();
-      if (lane < 8 * kHalves) tma_load_2d(v_sm + dst, &v_map, bar_vfull + 8 * st, hf * 64, row);
+      if (lane < kTcPages)
+        tma_load_4d(ring + st * kTcTileBytes + pg * kTcPageBytes, map, full + 8 * st, 0, 0, 0,
+                    (page * num_kv_heads + h) * (kTcPage / 8));
     }
   } else if (warp == 1) {
     // ---------------------------------------------------- S = Q K^T ------
     if (elect_one()) {
       constexpr uint32_t idesc_s = tc_idesc_bf16(kTcRows, kTcKeys, 0);  // B = K, K-major
       bool alive = mbar_wait(bar_q, 0, err);
-      const uint64_t a0 = umma_desc_k128(q_sm);
+      const uint64_t a0 = tc_desc_k_atoms(q_sm, kAtomGroup);
 #pragma unroll 1
       for (int t = 0; t < n_tiles && alive; ++t) {
         const int st = t & 1;
@@ -243,10 +258,10 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __
         alive = mbar_wait(bar_sempty + 8 * st, ph ^ 1, err);  // the softmax warps have read tile t - 2
         if (!alive) break;
         tc_fence_after();
-        const uint64_t b0 = umma_desc_k128(k_sm + st * kTcTileBytes);
+        const uint64_t b0 = tc_desc_k_atoms(k_sm + st * kTcTileBytes, kAtomGroup);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {  // 16 of the head dimensions each
-          const uint32_t off = ((k >> 2) * kTcHalfBytes + (k & 3) * 32) >> 4;
+          const uint32_t off = ((k >> 2) * 1024 + (k & 3) * 32) >> 4;
           tc_mma_f16(tmem_base + st * kTcKeys, a0 + off, b0 + off, idesc_s, k > 0 ? 1u : 0u);
         }
         tc_commit(bar_sfull + 8 * st);
@@ -274,7 +289,7 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __
           const uint64_t a0 = umma_desc_k128(p_sm + half * kTcHalfBytes);
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {  // 16 keys each
-            const uint64_t b = umma_desc_mn128(v_sm + st * kTcTileBytes + (half * 4 + kk) * (16 * 128), kTcHalfBytes, 1024);
+            const uint64_t b = umma_desc_mn128(v_sm + st * kTcTileBytes + (half * 4 + kk) * kTcPageBytes, 1024, kAtomGroup);
             tc_mma_f16(tmem_o, a0 + ((kk * 32) >> 4), b, idesc_o, (j > 0 || half > 0 || kk > 0) ? 1u : 0u);
           }
           tc_commit(bar_odone + 8 * half);
@@ -302,7 +317,7 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __
         if (qt_l < QT && t0 + qt_l < num_tokens)
           v = *reinterpret_cast<const uint4*>(
               q + (static_cast<size_t>(t0 + qt_l) * num_q_heads + h * gr + (qr - qt_l * gr)) * D + ch * 8);
-        *reinterpret_cast<uint4*>(base_ptr + (ch >> 3) * kTcHalfBytes + swz128(qr, ch & 7)) = v;
+        *reinterpret_cast<uint4*>(base_ptr + (qr >> 3) * kAtomGroup + (ch >> 3) * 1024 + swz128(qr & 7, ch & 7)) = v;
       }
       fence_proxy_async();  // the tensor core reads Q through the async proxy
       __syncwarp();
@@ -456,13 +471,15 @@ int launch_prefill_tc(const void* q, const void* k_pool, const void* v_pool, con
   const int group = hq / hkv;
   CUtensorMap qmap, kmap, vmap;
   const uint64_t rows = static_cast<uint64_t>(num_blocks) * hkv * kTcPage;
-  int rc = get_tensor_map_2d(k_pool, rows, head_dim, 2, kTcPage, 64, &kmap);
+  int rc = get_tensor_map_atoms(k_pool, rows, head_dim, kTcPage, &kmap);
   if (rc) return rc;
-  rc = get_tensor_map_2d(v_pool, rows, head_dim, 2, kTcPage, 64, &vmap);
+  rc = get_tensor_map_atoms(v_pool, rows, head_dim, kTcPage, &vmap);
   if (rc) return rc;
   const bool q_tma = head_dim == 128 && (group == 8 || group == 16);
   if (q_tma) {
-    rc = get_tensor_map_2d(q, static_cast<uint64_t>(num_tokens) * hq, head_dim, 2, group, 64, &qmap);
+    // 8 query heads per kv head: the CTA's positions in one box; 16: a box per position
+    rc = group == 8 ? get_tensor_map_atoms_of(q, num_tokens, hq, head_dim, kTcRows / 8, &qmap)
+                    : get_tensor_map_atoms(q, static_cast<uint64_t>(num_tokens) * hq, head_dim, 16, &qmap);
     if (rc) return rc;
   } else {
     qmap = kmap;  // not read
