@@ -12,7 +12,7 @@
 //
 //   grid     (batch x head groups of 16 * MT, splits): the head groups of a row are neighbours, so the second finds the
 //            row's pages in L2
-//   load     tiles of tokens by TMA (boxes of 16 tokens x 128 B, 128-byte swizzle, one box per lane of warp 0) into a ring
+//   load     tiles of tokens by TMA (a box per page: its 64-column halves one after the other, 128-byte swizzle) into a ring
 //            of stages; a stage is refilled right after the barrier that every warp reaches only when it is done with the
 //            tile before, so no "empty" barriers and no producer warp are needed
 //   scores   the groups of 8 tokens of a tile are dealt to the warps; S[heads x 8 tokens] over the whole rank by mma.sync
@@ -41,16 +41,15 @@ template <int R_, int MT_, int WARPS_, int TILE_, int STAGES_, int CTAS_>
 struct LatentCfg {
   static constexpr int R = R_, MT = MT_, kWarps = WARPS_, kTile = TILE_, kStages = STAGES_, kCtas = CTAS_;
   static constexpr int kPages = kTile / kLatPage;
-  static constexpr int kHalf = kTile * 128;  // 64 columns of a tile
+  static constexpr int kPageHalf = kLatPage * 128;  // 64 columns of a page
   static constexpr int kHalves = R / 64;
   static constexpr bool kQRegs = R * MT <= 512;
-  static constexpr int kStageBytes = kHalves * kHalf;
+  static constexpr int kStageBytes = kPages * kHalves * kPageHalf;  // [page][64-column half][16 tokens][128 B]
   static constexpr int kQBytes = kQRegs ? 0 : MT * 16 * R * 2;
   static constexpr int kPBytes = MT * 16 * 128;
   static constexpr int kRedBytes = kWarps * MT * 16 * 4;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kQBytes + kPBytes + kRedBytes + 8 * kStages;
   static constexpr int kThreads = kWarps * 32;
-  static_assert(kPages * kHalves <= 32, "one TMA box per lane");
   static_assert(!kQRegs || MT * 16 * R * 2 <= kStageBytes, "the queries pass through the last stage");
 
   static_assert(kTile <= 64 && kTile % 16 == 0 && R % (kWarps * 16) == 0, "tile shape");
@@ -67,7 +66,8 @@ latent_attn_decode_kernel(const __grid_constant__ CUtensorMap c_map, const __nv_
   grid_dep_wait();
   grid_dep_launch();
   constexpr int R = Cfg::R, MT = Cfg::MT, NW = Cfg::kWarps, STAGES = Cfg::kStages;
-  constexpr int kLatTile = Cfg::kTile, kLatHalf = Cfg::kHalf, kLatPages = Cfg::kPages, kHalves = Cfg::kHalves;
+  constexpr int kLatTile = Cfg::kTile, kLatPages = Cfg::kPages, kPageHalf = Cfg::kPageHalf;
+  constexpr int kPageBytes = Cfg::kHalves * kPageHalf;
   constexpr int kCols = R / NW, kNt = kCols / 8;  // output columns of a warp, n tiles of 8
   extern __shared__ uint8_t smem_raw[];
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -113,11 +113,13 @@ latent_attn_decode_kernel(const __grid_constant__ CUtensorMap c_map, const __nv_
   __syncthreads();
 
   // ---------------------------------------------------------------- loads --
-  // Lane of warp 0 -> one box of a tile.  The page id of the next tile to load is fetched one step ahead.  Pages past the
+  // Lane of warp 0 -> one page of a tile, a box of all its columns: a copy costs about 100 cycles to issue whatever its size, and
+  // between two barriers every warp waits for this one (with a box per 64 columns of a page, rank 512, 256 rows of 512
+  // to 4096 tokens, 16 heads: 131 us, now 117).  The page id of the next tile to load is fetched one step ahead.  Pages past the
   // split's end hold nothing that may be read; the last valid page stands in (its scores are masked).
   const int* table_row = block_table + static_cast<size_t>(b) * max_pages;
-  const int pg = lane / kHalves, half = lane % kHalves;
-  const bool issuer = warp == 0 && lane < kLatPages * kHalves;
+  const int pg = lane;
+  const bool issuer = warp == 0 && lane < kLatPages;
   int next_id = 0;
   auto fetch_id = [&](int tile) {
     if (issuer) next_id = table_row[min(first_page + tile * kLatPages + pg, last_page)];
@@ -132,8 +134,7 @@ latent_attn_decode_kernel(const __grid_constant__ CUtensorMap c_map, const __nv_
     if (lane == 0) mbar_arrive_expect_tx(bars + 8 * slot, Cfg::kStageBytes);
     __syncwarp();
     if (issuer)
-      tma_load_2d(ring + slot * Cfg::kStageBytes + half * kLatHalf + pg * (kLatPage * 128), &c_map, bars + 8 * slot,
-                  half * 64, id * kLatPage);
+      tma_load_3d(ring + slot * Cfg::kStageBytes + pg * kPageBytes, &c_map, bars + 8 * slot, 0, id * kLatPage, 0);
   };
   if (warp == 0) {
     for (int t = 0; t < min(STAGES - 1, n_tiles); ++t) {
@@ -195,7 +196,7 @@ latent_attn_decode_kernel(const __grid_constant__ CUtensorMap c_map, const __nv_
         for (int kk = 0; kk < R / 32; ++kk) {  // 32 latent columns: two k steps
           uint32_t b0, b1, b2, b3;
           const int ch = kk * 4 + lj;
-          ldmatrix_x4(cbase + (ch >> 3) * kLatHalf + swz128(n8 * 8 + lr, ch & 7), b0, b1, b2, b3);
+          ldmatrix_x4(cbase + (n8 >> 1) * kPageBytes + (ch >> 3) * kPageHalf + swz128((n8 & 1) * 8 + lr, ch & 7), b0, b1, b2, b3);
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt) {
             if (Cfg::kQRegs) {
@@ -298,7 +299,7 @@ latent_attn_decode_kernel(const __grid_constant__ CUtensorMap c_map, const __nv_
       for (int np = 0; np < kNt / 2; ++np) {
         uint32_t v0, v1, v2, v3;
         const int ch = warp * (kCols / 8) + np * 2 + v_sub;
-        ldmatrix_x4_trans(cbase + (ch >> 3) * kLatHalf + swz128(ks * 16 + v_tok, ch & 7), v0, v1, v2, v3);
+        ldmatrix_x4_trans(cbase + ks * kPageBytes + (ch >> 3) * kPageHalf + swz128(v_tok, ch & 7), v0, v1, v2, v3);
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
           mma_bf16_16816(o[mt][2 * np], pa[mt], v0, v1);
@@ -391,7 +392,7 @@ static int launch_latent(const void* q, const void* c_pool, const int* block_tab
                          int split_tokens, int max_splits, const float* gate, cudaStream_t st) {
   static_assert(Cfg::kSmemBytes <= 232448, "more shared memory than a CTA may have");
   CUtensorMap cmap;
-  int rc = get_tensor_map_2d(c_pool, static_cast<uint64_t>(num_blocks) * kLatPage, Cfg::R, 2, kLatPage, 64, &cmap);
+  int rc = get_tensor_map_columns(c_pool, static_cast<uint64_t>(num_blocks) * kLatPage, Cfg::R, kLatPage, &cmap);
   if (rc) return rc;
   rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&latent_attn_decode_kernel<Cfg>), Cfg::kSmemBytes);
   if (rc) return rc;
