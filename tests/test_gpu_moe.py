@@ -262,3 +262,21 @@ def test_padding_rows_get_no_expert_and_drop_out_of_the_layer(ops):
     ops.read_status(q2.workspace, "permute with padding rows")
     assert bool((q2.row_of_pair[rows:] == -1).all())
     np.testing.assert_array_equal(q2.row_of_pair.cpu().numpy()[:rows], r["row_of_pair"])
+
+
+@pytest.mark.parametrize("T", [192, 201, 449])
+def test_many_rows_per_expert_give_the_bits_of_few(ops, T):
+    """With at least 96 rows per expert the down product stores its rows through shared memory: the same values, in full and short
+    tiles (an expert left with a single row or none of a tile's quarters included)."""
+    E, K, H, I = 4, 2, 256, 128
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, H, generator=g).bfloat16().to(DEV)
+    logits = torch.randn(T, E, generator=g).to(DEV)
+    w13, s13 = (t.to(DEV) for t in oracle.quantize_weight_ref(torch.randn(E, 2 * I, H, generator=g) * 0.05))
+    w2, s2 = (t.to(DEV) for t in oracle.quantize_weight_ref(torch.randn(E, H, I, generator=g) * 0.05))
+    ws = ops.moe_fp8_workspace(T, E, K, H, I, DEV)
+
+    def run(lo, hi):
+        return ops.moe_fp8_forward(x[lo:hi].contiguous(), logits[lo:hi].contiguous(), w13, s13, w2, s2, K, True, ws).clone()
+    parts = [run(lo, min(T, lo + 100)) for lo in range(0, T, 100)]
+    assert torch.equal(run(0, T), torch.cat(parts))

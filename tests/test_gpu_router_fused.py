@@ -68,6 +68,20 @@ def test_repeatable_and_independent_of_the_batch_around_a_row(ops):
         assert torch.equal(u[:19], v)
 
 
+@pytest.mark.parametrize("T,H,E", [(513, 2048, 128), (545, 512, 16)])
+def test_long_chunks_give_the_bits_of_short_ones(ops, T, H, E):
+    """More than 512 rows run with 32 rows per cluster (a last cluster of one row included): the same sums in the same order."""
+    x, delta, nw, rw = make(T, H, E, seed=4)
+    K = 4
+
+    def run(lo, hi):
+        xs = x[lo:hi].contiguous().to(DEV)
+        return (xs, *ops.add_rmsnorm_route(xs, delta[lo:hi].contiguous().to(DEV), nw.to(DEV), 1e-6, rw.to(DEV), K, True,
+                                           want_logits=True))
+    for whole, first, rest in zip(run(0, T), run(0, 300), run(300, T)):
+        assert torch.equal(whole, torch.cat([first, rest]))
+
+
 def test_unsupported_shapes_are_refused(ops):
     assert not ops.add_rmsnorm_route_supported(768, 128, 8)     # hidden not a multiple of 512
     assert not ops.add_rmsnorm_route_supported(2048, 256, 8)    # more than 128 experts
