@@ -326,7 +326,6 @@ class LayeredEngine(gated.GatedMechanisms, PagedEngine):
     """A layer-list decoder on the paged step: weights, pools and one pass over the layers."""
 
     logits_dtype = torch.float32
-    prompt_chunk = 2048
 
     def __init__(self, cfg: LayeredConfig, num_blocks: int, max_batch: int, max_pages_per_seq: int, device="cuda", seed: int = 0,
                  tensors: dict[str, torch.Tensor] | None = None, dtype: torch.dtype = torch.bfloat16, use_graphs: bool = True,
