@@ -748,10 +748,12 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
       }
       asm volatile("bar.sync 1, 256;" ::: "memory");
       const int col = (warp - 2) * 32 + lane;
-      float val = quarter_val[col];
-      int idx = quarter_idx[col];
+      // From nothing, as the fold below starts: a quarter whose candidate is a NaN (a NaN logit, or only logits of -inf, whose
+      // cut key is one) must not stand for the others.
+      float val = -INFINITY;
+      int idx = 0x7fffffff;
 #pragma unroll
-      for (int q = 1; q < 4; ++q) {
+      for (int q = 0; q < 4; ++q) {
         const float v = quarter_val[q * kDenseMaxRows + col];
         const int i = quarter_idx[q * kDenseMaxRows + col];
         if (v > val || (v == val && i < idx)) {

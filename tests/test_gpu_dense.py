@@ -104,6 +104,24 @@ def test_lm_head_argmax_agrees_with_argmax_of_the_written_logits(ops):
     assert bool((picked == logits.max(dim=1).values).all())
 
 
+@pytest.mark.parametrize("lost", [float("-inf"), float("nan")])
+@pytest.mark.parametrize("quarter", [0, 2])
+@pytest.mark.parametrize("M,V,K", [(3, 4096, 128), (65, 40000, 64)])
+def test_lm_head_argmax_with_a_lane_quarter_of_infinities_or_nans(ops, M, V, K, quarter, lost):
+    """32 neighbouring features of every weight tile have logits of -inf (or NaN), a column of weights that masks them: the token
+    is the arg-max over the others."""
+    x, w, _ = make(M, V, K, seed=V)
+    x[:, 0] = 1
+    gone = (torch.arange(V) % 128) // 32 == quarter
+    want = (x.float() @ w.float().t()).masked_fill(gone, float("-inf"))
+    w[gone, 0] = lost
+    tok = ops.lm_head_argmax(x.to(DEV), w.to(DEV)).cpu()
+    assert not gone[tok].any()
+    picked, best = want[torch.arange(M), tok], want.max(dim=1).values
+    # keys drop 5 of 24 bits; the two sums of K products differ by at most K roundings
+    assert bool((best - picked <= 2.0 ** -17 * best.abs() + K * 2.0 ** -23 * (x.float().abs() @ w[~gone].float().abs().t()).amax(1)).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M,V,K", [(1, 8192, 1024), (33, 1001, 512), (256, 3000, 128), (300, 129, 64)])
 def test_lm_head_argmax_writes_the_logits_of_the_plain_product(ops, M, V, K, dtype):
