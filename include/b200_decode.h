@@ -360,9 +360,10 @@ int b200_qk_norm_rope_append(const void* qkv, const void* q_norm_weight, const v
  * Replaces, in one kernel: the residual add and post-attention RMSNorm of the decoder layer, the router's
  * linear layer (`gate`) and Qwen3MoeTopKRouter (fp32 softmax, top-k, renormalisation) of the forward called at
  * torch_backend.py:314-320 - b200_add_rmsnorm, the router projection and b200_moe_route back to back, with the
- * router logits kept on the chip in fp32.  A cluster of 8 CTAs owns 16 rows; each CTA takes an eighth of the
- * hidden dimension and the partial sums of squares and partial logits meet through distributed shared memory,
- * summed in rank order.
+ * router logits kept on the chip in fp32.  A cluster of 8 CTAs owns 16 rows or 32
+ * (b200_add_rmsnorm_route_rows says which, < 0 on error; the results are the same); each CTA takes an eighth of
+ * the hidden dimension and the partial sums of squares and partial logits meet through distributed shared
+ * memory, summed in rank order.
  *
  *   x [num_rows, hidden] bf16, updated in place to x + delta when delta is not NULL
  *   normed_out [num_rows, hidden] bf16 = norm_weight * normalise(x)   (the MoE layer's input)
@@ -372,6 +373,7 @@ int b200_qk_norm_rope_append(const void* qkv, const void* q_norm_weight, const v
  * hidden a multiple of 512, num_experts a multiple of 16 and at most 128: b200_add_rmsnorm_route_supported.
  */
 int b200_add_rmsnorm_route_supported(int hidden, int num_experts, int top_k);
+int b200_add_rmsnorm_route_rows(int num_rows, int hidden, int num_experts);
 int b200_add_rmsnorm_route(void* x, const void* delta, const void* norm_weight, float eps,
                            const void* router_weight, int num_rows, int hidden, int num_experts, int top_k,
                            int renormalize, const int32_t* num_valid_rows, void* normed_out, int32_t* topk_ids,

@@ -79,6 +79,7 @@ SIGNATURES = {
     "b200_lm_head_argmax_logits": (c_int, [c_void_p] * 4 + [c_int, c_void_p, c_size_t, c_void_p] + [c_int] * 3 + [c_void_p]),
     "b200_lm_head_argmax": (c_int, [c_void_p] * 4 + [c_size_t, c_void_p] + [c_int] * 3 + [c_void_p]),
     "b200_add_rmsnorm_route_supported": (c_int, [c_int] * 3),
+    "b200_add_rmsnorm_route_rows": (c_int, [c_int] * 3),
     "b200_add_rmsnorm_route": (c_int, [c_void_p] * 3 + [c_float, c_void_p] + [c_int] * 5 + [c_void_p] * 6),
     "b200_add_rmsnorm": (c_int, [c_void_p, c_void_p, c_void_p, c_float, c_int, c_int, c_void_p, c_void_p]),
     "b200_qk_norm_rope_append": (c_int, [c_void_p] * 11 + [c_int] * 4 + [c_float] + [c_int] * 4 + [c_void_p]),

@@ -8,19 +8,21 @@
 //
 //   x += delta (bf16);  h = weight * rmsnorm(x);  logits = h W_r^T (fp32);  ids, weights = top-k
 //
-//   grid   = (rows / ROWS) clusters of 8 CTAs.  A cluster owns ROWS = 16 rows, or 32 of a long prompt
-//            chunk, whose 16-row clusters do not all fit the GPU at once; CTA r of it owns the r-th
+//   grid   = (rows / ROWS) clusters of 8 CTAs.  A cluster owns ROWS = 16 rows, or 32 where that saves
+//            enough waves of clusters (route_rows); CTA r of it owns the r-th
 //            eighth of the hidden dimension, so the router matrix [E, H] (0.5 MiB at E = 128,
 //            H = 2048, too much for one CTA to pull in time) is read as eight 64 KiB slices.
-//   norm   = each CTA adds and squares its slice of the 16 rows; the eight partial sums of squares
-//            meet through distributed shared memory (16 floats per CTA) and are added in rank order.
-//   gemm   = [16 x H/8] x [H/8 x E] per CTA by mma.sync m16n8k16 (bf16 in, fp32 out): 134 MFLOP for
+//   norm   = each CTA adds and squares its slice of the rows; the eight partial sums of squares
+//            meet through distributed shared memory (ROWS floats per CTA) and are added in rank order.
+//   gemm   = [ROWS x H/8] x [H/8 x E] per CTA by mma.sync m16n8k16 (bf16 in, fp32 out): 134 MFLOP for
 //            256 rows, far too little for the tcgen05 path to pay its set-up; warp w takes experts
-//            16w..16w+15.  The eight partial logit tiles (16 x E fp32) meet through distributed
+//            16w..16w+15.  The eight partial logit tiles (ROWS x E fp32) meet through distributed
 //            shared memory: CTA r sums rows ROWS/8 * r ... in rank order.
 //   route  = those rows are routed by a warp each exactly as moe_route_kernel does (selection on
 //            the logits, ties to the lower expert id), on fp32 logits that never leave the chip.
 // Everything is deterministic (fixed summation orders, no atomics).
+
+#include <mutex>
 
 #include "common.cuh"
 #include "host.h"
@@ -299,26 +301,88 @@ static size_t router_fused_smem(int H, int E, int rows) {
   return (rows + static_cast<size_t>(E)) * pitch * 2 + (2 * rows + rows * static_cast<size_t>(E) + rows / kRfCluster * E) * 4;
 }
 
+static void route_launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int clusters, size_t smem, cudaStream_t st) {
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3(static_cast<unsigned>(clusters) * kRfCluster);
+  cfg->blockDim = dim3(kRfThreads);
+  cfg->dynamicSmemBytes = smem;
+  cfg->stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kRfCluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+}
+
 template <int ROWS>
 static int launch_route(const RouterFusedParams& p, cudaStream_t st) {
   const size_t smem = router_fused_smem(p.H, p.E, ROWS);
   int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&add_rmsnorm_route_kernel<ROWS>), static_cast<int>(smem));
   if (rc) return rc;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>((p.T + ROWS - 1) / ROWS) * kRfCluster);
-  cfg.blockDim = dim3(kRfThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
+  cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kRfCluster;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  route_launch_config(&cfg, attr, (p.T + ROWS - 1) / ROWS, smem, st);
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = overlapped_launch_enabled() ? 2 : 1;
+  if (overlapped_launch_enabled()) cfg.numAttrs = 2;
   B200_CUDA(cudaLaunchKernelEx(&cfg, add_rmsnorm_route_kernel<ROWS>, p));
+  return 0;
+}
+
+// How many clusters of ROWS rows the current device holds at once; asked once per device and size of shared memory.
+template <int ROWS>
+static int resident_route_clusters(int H, int E, int* out) {
+  struct Entry {
+    int dev;
+    size_t smem;
+    int n;
+  };
+  static std::mutex mu;
+  static Entry cache[32];
+  static int used = 0;
+  const size_t smem = router_fused_smem(H, E, ROWS);
+  int dev = 0;
+  B200_CUDA(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    for (int i = 0; i < used; ++i)
+      if (cache[i].dev == dev && cache[i].smem == smem) {
+        *out = cache[i].n;
+        return 0;
+      }
+  }
+  int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&add_rmsnorm_route_kernel<ROWS>), static_cast<int>(smem));
+  if (rc) return rc;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[1];
+  route_launch_config(&cfg, attr, 1, smem, nullptr);
+  int n = 0;
+  B200_CUDA(cudaOccupancyMaxActiveClusters(&n, add_rmsnorm_route_kernel<ROWS>, &cfg));
+  if (n < 1) n = 1;
+  std::lock_guard<std::mutex> lock(mu);
+  if (used < static_cast<int>(sizeof(cache) / sizeof(cache[0]))) cache[used++] = Entry{dev, smem, n};
+  *out = n;
+  return 0;
+}
+
+// Rows per cluster: 16, or 32 where that leaves at most three waves of clusters in place of four.  A wave of 32-row clusters takes
+// 1.15-1.3 times one of 16-row clusters (128 experts: width 512 14.2 and 12.1 us, 2048 14.6 and 11.4, 4096 13.9 and 10.6), and how many of either
+// the GPU holds depends on their shared memory, so on width and experts.  us with 16 and with 32, 128 experts:
+//   width 2048   513 rows 11.4, 13.2   576: 19.4, 13.6   1024: 22.3, 14.6   2048: 43.7, 28.6
+//   width  512  1024 rows 12.1, 14.2  1500: 21.0, 14.7   2048: 22.9, 25.3   4096: 43.5, 40.6
+//   width 4096   128 rows 10.6, 13.6   256: 20.6, 13.9    512: 31.6, 27.0   1024: 54.2, 41.6
+static int route_rows(int T, int H, int E, int* out) {
+  *out = 16;
+  const int c16 = (T + 15) / 16, c32 = (T + 31) / 32;
+  if (c16 < 2 || router_fused_smem(H, E, 32) > 200 * 1024) return 0;
+  int n16 = 0, n32 = 0;
+  int rc = resident_route_clusters<16>(H, E, &n16);
+  if (rc) return rc;
+  if (c16 <= n16) return 0;
+  rc = resident_route_clusters<32>(H, E, &n32);
+  if (rc) return rc;
+  if (4 * ((c32 + n32 - 1) / n32) <= 3 * ((c16 + n16 - 1) / n16)) *out = 32;
   return 0;
 }
 
@@ -365,9 +429,18 @@ extern "C" int b200_add_rmsnorm_route(void* x, const void* delta, const void* no
   p.E = num_experts;
   p.K = top_k;
   p.renorm = renormalize;
-  // 16-row clusters as long as they are all resident (two CTAs per SM: about 32 clusters); beyond that 32 rows per cluster.
-  // Width 2048, 128 experts: 1024 rows 25.7 us with 16, 18.4 us with 32; up to 512 rows one
-  // wave of 16-row clusters takes 8-13 us.
-  if (num_rows > 32 * 16 && router_fused_smem(hidden, num_experts, 32) <= 200 * 1024) return launch_route<32>(p, as_stream(stream));
-  return launch_route<16>(p, as_stream(stream));
+  int rows = 16;
+  rc = route_rows(num_rows, hidden, num_experts, &rows);
+  if (rc) return rc;
+  return rows == 32 ? launch_route<32>(p, as_stream(stream)) : launch_route<16>(p, as_stream(stream));
+}
+
+extern "C" int b200_add_rmsnorm_route_rows(int num_rows, int hidden, int num_experts) {
+  B200_REQUIRE(num_rows > 0 && b200_add_rmsnorm_route_supported(hidden, num_experts, 1), "add_rmsnorm_route_rows: %d rows of %d, %d experts",
+               num_rows, hidden, num_experts);
+  int rc = check_device(nullptr);
+  if (rc) return rc;
+  int rows = 0;
+  rc = route_rows(num_rows, hidden, num_experts, &rows);
+  return rc ? rc : rows;
 }

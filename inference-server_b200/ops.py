@@ -304,6 +304,14 @@ def add_rmsnorm_route_supported(hidden: int, num_experts: int, top_k: int) -> bo
     return bool(_lib.load().b200_add_rmsnorm_route_supported(int(hidden), int(num_experts), int(top_k)))
 
 
+def add_rmsnorm_route_rows(num_rows: int, hidden: int, num_experts: int) -> int:
+    """Rows per cluster (16 or 32) of add_rmsnorm_route on the current device."""
+    rows = _lib.load().b200_add_rmsnorm_route_rows(int(num_rows), int(hidden), int(num_experts))
+    if rows < 0:
+        check(rows, "b200_add_rmsnorm_route_rows")
+    return rows
+
+
 def add_rmsnorm_route(x: torch.Tensor, delta: torch.Tensor | None, norm_weight: torch.Tensor, eps: float,
                       router_weight: torch.Tensor, top_k: int, renormalize: bool = True,
                       num_valid: torch.Tensor | None = None, want_logits: bool = False):

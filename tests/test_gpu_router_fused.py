@@ -68,18 +68,31 @@ def test_repeatable_and_independent_of_the_batch_around_a_row(ops):
         assert torch.equal(u[:19], v)
 
 
-@pytest.mark.parametrize("T,H,E", [(513, 2048, 128), (545, 512, 16)])
+@pytest.mark.parametrize("T,H,E", [(577, 2048, 128), (1500, 512, 16), (300, 4096, 128)])
 def test_long_chunks_give_the_bits_of_short_ones(ops, T, H, E):
-    """More than 512 rows run with 32 rows per cluster (a last cluster of one row included): the same sums in the same order."""
+    """More rows than the 16-row clusters that fit the GPU at once run with 32 rows per cluster (a last cluster of one row
+    included): the same sums in the same order, rows beyond num_valid without experts."""
     x, delta, nw, rw = make(T, H, E, seed=4)
-    K = 4
+    K, half = 4, (T // 32) * 16
+    assert [ops.add_rmsnorm_route_rows(n, H, E) for n in (T, half, T - half)] == [32, 16, 16]
 
-    def run(lo, hi):
+    def run(lo, hi, **kw):
         xs = x[lo:hi].contiguous().to(DEV)
         return (xs, *ops.add_rmsnorm_route(xs, delta[lo:hi].contiguous().to(DEV), nw.to(DEV), 1e-6, rw.to(DEV), K, True,
-                                           want_logits=True))
-    for whole, first, rest in zip(run(0, T), run(0, 300), run(300, T)):
-        assert torch.equal(whole, torch.cat([first, rest]))
+                                           want_logits=True, **kw))
+    whole = run(0, T)
+    for all_rows, first, rest in zip(whole, run(0, half), run(half, T)):
+        assert torch.equal(all_rows, torch.cat([first, rest]))
+    for n in (T - 31, T - 1, 0):
+        _, h, ids, w, _ = run(0, T, num_valid=torch.tensor([n], dtype=torch.int32, device=DEV))
+        assert torch.equal(h, whole[1]) and torch.equal(ids[:n], whole[2][:n]) and torch.equal(w[:n], whole[3][:n])
+        assert bool((ids[n:] == -1).all()) and bool((w[n:] == 0).all())
+
+
+@pytest.mark.parametrize("T,H,E", [(1024, 512, 16), (1024, 1024, 64), (513, 2048, 128), (1024, 2048, 64), (513, 4096, 64), (2048, 512, 128)])
+def test_rows_that_a_wave_of_short_clusters_takes_stay_there(ops, T, H, E):
+    """Clusters of 32 rows would be as many waves here, each of them longer (3-17 % more time)."""
+    assert ops.add_rmsnorm_route_rows(T, H, E) == 16
 
 
 def test_unsupported_shapes_are_refused(ops):
