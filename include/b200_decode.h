@@ -681,6 +681,9 @@ int b200_moe_fp8_gemm_down(const void* hq, const float* h_scale, const void* w2,
                            void* y_sorted, const int32_t* out_row_map, void* status_word, int num_rows,
                            int num_experts,
                            int hidden, int inter, int weight_layout, void* stream);
+/* 1 if b200_moe_fp8_gemm_down writes its rows by way of shared memory, 0 if straight from registers (the same values): chosen
+ * by the mean rows per expert, which only rows without a row map tell. */
+int b200_moe_fp8_gemm_down_staged(int num_rows, int num_experts, int row_mapped);
 
 /*
  * Replaces: the routing-weight multiply and per-token sum over the top_k expert

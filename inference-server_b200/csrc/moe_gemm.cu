@@ -51,8 +51,8 @@ constexpr int kEpiWarps = 8;
 constexpr int kGemmThreads = (4 + kEpiWarps) * 32;  // warps 2, 3 idle: roles are per warpgroup
 constexpr int kTmemCols = 512;
 // Down, many rows per expert: a promotion thread owns a row, so what it writes straight to memory goes out as 16 bytes in each of
-// 32 rows per instruction.  Each warp then turns its part round in shared memory instead (32 rows x 64 columns at a
-// time) and writes whole 128-byte pieces: 4096 tokens, 8 of 128 experts, 2048 <- 768: 119 -> 101 us.
+// 32 rows per instruction.  Where down_staged says so each warp turns its part round in shared memory instead (32 rows x 64
+// columns at a time) and writes whole 128-byte pieces: 4096 tokens, 8 of 128 experts, 2048 <- 768: 119 -> 101 us.
 constexpr int kStagedWarp = 32 * 128;
 constexpr int kGemmSmem = kGemmStages * kStageBytesG + 1024 /* align */ + 128 /* barriers */ +
                           16 /* tmem base */ + 2 * 2 * kTileM * 4 /* amax exchange */;
@@ -345,20 +345,8 @@ moe_fp8_gemm_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_cons
         const int rows_here = min(32, tile.rows - quarter * 32);  // rows of this warp's quarter that exist (may be negative)
         if (STAGED && rows_here > 0) {
           uint8_t* staged = ring_ptr + kStagedOff + (warp - 4) * kStagedWarp;
-          __nv_bfloat16* row_out[8];  // of the rows this lane writes a piece of
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int i = u * 4 + (lane >> 3);
-            const size_t at = static_cast<size_t>(tile.row0) + quarter * 32 + i;
-            size_t orow = i < rows_here && p.out_row_map ? static_cast<size_t>(__ldg(p.out_row_map + at)) : at;
-            __nv_bfloat16* ybase = p.y;
-            if (p.peer_capacity > 0 && i < rows_here) {
-              const int src = static_cast<int>(orow) / p.peer_capacity;
-              orow = static_cast<size_t>(p.my_rank) * p.peer_capacity + (orow - static_cast<size_t>(src) * p.peer_capacity);
-              ybase = p.y_peers[src];
-            }
-            row_out[u] = ybase + orow * p.n_rows + j * kTileN + half * 128 + (lane & 7) * 8;
-          }
+          __nv_bfloat16* row_out = p.y + (static_cast<size_t>(tile.row0) + quarter * 32 + (lane >> 3)) * p.n_rows + j * kTileN +
+                                   half * 128 + (lane & 7) * 8;  // this lane's piece of the first row it writes
 #pragma unroll
           for (int c0 = 0; c0 < 128; c0 += 64) {
 #pragma unroll
@@ -375,7 +363,7 @@ moe_fp8_gemm_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_cons
             for (int u = 0; u < 8; ++u) {
               const int i = u * 4 + (lane >> 3);
               if (i < rows_here)
-                *reinterpret_cast<uint4*>(row_out[u] + c0) =
+                *reinterpret_cast<uint4*>(row_out + static_cast<size_t>(u * 4) * p.n_rows + c0) =
                     *reinterpret_cast<const uint4*>(staged + i * 128 + (((lane & 7) ^ (i & 7)) << 4));
             }
             __syncwarp();
@@ -492,6 +480,16 @@ extern "C" int b200_moe_fp8_gemm_gate_up(const void* xq, const float* x_scale, c
   return launch_gemm<kModeGateUp>(a_map, b_map, p, as_stream(stream));
 }
 
+// Whether the down product's rows go out by way of shared memory.  Few rows per expert: a tile's epilogue stores little, and the plain
+// form's shorter code streams the weights faster.  us plain and staged:
+//   128 experts, 2048 <- 768: 16 rows per expert 38.6, 41.9   64: 49.4, 47.4   96: 55.3, 51.4   128: 72.1, 62.5   256: 116, 99.5
+//    16 experts, 1024 <- 512:                                  64: 7.02, 7.11                   128: 8.80, 7.87  256: 13.7, 11.7
+//    64 experts, 4096 <- 768: 32: 41.7, 43.6                   64: 48.9, 46.9                   128: 75.1, 64.2  256: 113, 98.2
+// With a row map (expert parallelism) num_rows is the capacity of the receive buffer, twice the mean by default and the same in an
+// idle round, so it does not tell how many rows are there: always the plain form (4096 slots of 16 experts, 2048 <- 768: 64 real rows
+// 8.1 us plain, 9.1 staged; 1024 rows 10.3, 10.1; 2048 rows 19.0, 15.8).
+static bool down_staged(int num_rows, int num_experts, bool row_mapped) { return !row_mapped && num_rows / num_experts >= 96; }
+
 static int gemm_down_impl(const void* hq, const float* h_scale, const void* w2, const float* w2_scale_inv,
                           const void* tiles, const int32_t* num_tiles, void* y_sorted,
                           const int32_t* out_row_map, void* status_word, int num_rows, int num_experts,
@@ -546,10 +544,7 @@ static int gemm_down_impl(const void* hq, const float* h_scale, const void* w2, 
     p.peer_capacity = ep_capacity;
     p.my_rank = ep_rank;
   }
-  // Few rows per expert: a tile's epilogue stores little and the plain form's shorter code streams the weights faster (1024 tokens,
-  // 64 rows per expert: equal; 256 tokens: 37.5 us
-  // plain, 42 us staged).
-  if (num_rows / num_experts >= 96) return launch_gemm<kModeDown, true>(a_map, b_map, p, as_stream(stream));
+  if (down_staged(num_rows, num_experts, out_row_map != nullptr)) return launch_gemm<kModeDown, true>(a_map, b_map, p, as_stream(stream));
   return launch_gemm<kModeDown>(a_map, b_map, p, as_stream(stream));
 }
 
@@ -574,4 +569,9 @@ extern "C" int b200_moe_fp8_gemm_down_p2p(const void* hq, const float* h_scale, 
   return gemm_down_impl(hq, h_scale, w2, w2_scale_inv, tiles, num_tiles, nullptr, out_row_map, status_word,
                         num_rows, num_experts, hidden, inter, weight_layout, y_peers, ep_world, ep_capacity,
                         ep_rank, stream);
+}
+
+extern "C" int b200_moe_fp8_gemm_down_staged(int num_rows, int num_experts, int row_mapped) {
+  B200_REQUIRE(num_rows >= 0 && num_experts > 0, "moe_fp8_gemm_down_staged: bad row/expert count");
+  return down_staged(num_rows, num_experts, row_mapped != 0);
 }

@@ -45,6 +45,14 @@ def test_host_side_calls_that_need_no_gpu():
     assert lib.b200_moe_fp8_workspace_bytes(256, 128, 8, 2048, 768) > 256 * 8 * (2048 * 3 + 768)
 
 
+def test_staged_down_product_goes_by_rows_that_are_there():
+    """A row map comes with a receive buffer, whose capacity (here 8 ranks x 512 slots for 16 experts) may hold a handful of rows."""
+    lib = pkg("_lib").load()
+    assert [lib.b200_moe_fp8_gemm_down_staged(rows, 128, 0) for rows in (0, 2048, 96 * 128 - 1, 96 * 128)] == [0, 0, 0, 1]
+    assert lib.b200_moe_fp8_gemm_down_staged(4096, 16, 1) == 0 and lib.b200_moe_fp8_gemm_down_staged(4096, 16, 0) == 1
+    assert lib.b200_moe_fp8_gemm_down_staged(1, 0, 0) == -1
+
+
 def test_null_pointer_is_rejected_on_the_host():
     lib = pkg("_lib").load()
     rc = lib.b200_moe_route(None, 1, 4, 16, 4, 1, None, None, None, None)

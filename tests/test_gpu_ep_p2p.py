@@ -44,7 +44,7 @@ def test_world_of_one_with_an_arena_matches_the_fused_layer(ops, T, slack):
     assert st.epochs.tolist() == [2, 2]
 
 
-@pytest.mark.parametrize("W,T,cap", [(2, 64, 512), (4, 64, 256), (8, 32, 64)])
+@pytest.mark.parametrize("W,T,cap", [(2, 64, 512), (4, 64, 256), (8, 32, 64), (8, 64, 256)])
 def test_emulated_ranks_match_the_single_gpu_layer(ops, W, T, cap):
     """Every emulated rank must get, for its own tokens, exactly what the whole-model layer gives: a row's
     result does not depend on which other rows share its expert's tile."""

@@ -280,3 +280,21 @@ def test_many_rows_per_expert_give_the_bits_of_few(ops, T):
         return ops.moe_fp8_forward(x[lo:hi].contiguous(), logits[lo:hi].contiguous(), w13, s13, w2, s2, K, True, ws).clone()
     parts = [run(lo, min(T, lo + 100)) for lo in range(0, T, 100)]
     assert torch.equal(run(0, T), torch.cat(parts))
+
+
+@pytest.mark.parametrize("T", [200, 301])
+def test_down_product_with_a_row_map_and_many_rows_per_expert(ops, T):
+    """Row r of the sorted rows goes to row out_row_map[r]: the values of the call without a map, which stores them another way."""
+    E, K, H, I = 4, 2, 256, 128
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, H, generator=g).bfloat16().to(DEV)
+    w13, s13 = (t.to(DEV) for t in oracle.quantize_weight_ref(torch.randn(E, 2 * I, H, generator=g) * 0.05))
+    w2, s2 = (t.to(DEV) for t in oracle.quantize_weight_ref(torch.randn(E, H, I, generator=g) * 0.05))
+    ids, _ = ops.moe_route(torch.randn(T, E, generator=g).to(DEV), K)
+    p = ops.moe_permute(ids, E)
+    xq, xs = ops.act_quant_fp8(x, p.row_of_pair, K)
+    hq, hs = ops.moe_fp8_gemm_gate_up(xq, xs, w13, s13, p)
+    to = torch.randperm(T * K, generator=g).int().to(DEV)
+    want, got = ops.moe_fp8_gemm_down(hq, hs, w2, s2, p), torch.zeros(T * K, H, dtype=torch.bfloat16, device=DEV)
+    ops.moe_fp8_gemm_down(hq, hs, w2, s2, p, out=got, out_row_map=to)
+    assert torch.equal(got[to.long()], want) and bool(want.any())
