@@ -141,6 +141,7 @@ class PagedEngine:
     weights, its page pools (`num_blocks` pages per layer, one more as scratch page) and five hooks:
 
       _decode_hidden(B)                        final normed hidden rows of one decode step of rows [0, B)
+      _default_chunk(n) -> chunk               tokens of a pass of a prompt with n tokens to run, if the caller does not say
       _begin_prompt(chunk) -> chunk            buffers for prompt passes of up to `chunk` tokens
       _prompt_hidden(token_ids, row, lo, chunk, slot)     hidden rows of one chunk at positions lo.. of the sequence with table
                                                `row` (and state slot `slot`)
@@ -154,10 +155,9 @@ class PagedEngine:
     (`_build_graph` does), and a sequence that starts at position 0 must not depend on what its slot holds.
     """
 
-    # Tokens of a prompt pass unless the caller says otherwise.  A pass streams every expert's weights once: 2048 tokens in one
-    # pass and not in two of 1024 cost 5.4 ms instead of 7.0 (qwen3-30b-a3b, 12 layers), and a row's bits do not depend on it
-    # (the attention kernel's rows are grouped by 16 positions either way).  The expert workspace is 115 MB for 2048 tokens.
-    prompt_chunk = 2048
+    prompt_chunk = 2048       # tokens of a prompt pass unless the caller says otherwise
+    # What a default pass falls back to when memory is short; None where a pass must not run its rows twice (recurrent states).
+    short_prompt_chunk = None
     ep_state = None           # expert parallelism (DecodeEngine)
     round_hook = None
     takes_reference_pools = False  # whether a reference BlockManager's K/V pools can stand in for the engine's own
@@ -288,6 +288,17 @@ class PagedEngine:
     def _pick_with_logits(self, h, out=None) -> tuple[torch.Tensor, torch.Tensor]:
         return self._pick(h, out), self._logits(h)
 
+    def _default_chunk(self, tokens: int) -> int:
+        return self.prompt_chunk
+
+    def _may_shorten(self, given: int | None, chunk: int) -> bool:
+        """Whether a prompt pass of `chunk` tokens for which the memory did not suffice may run as shorter ones."""
+        return not given and self.ep_state is None and self.short_prompt_chunk is not None and chunk > self.short_prompt_chunk
+
+    def _begin_shorter(self) -> int:
+        self.prompt_chunk = self.short_prompt_chunk  # later prompts do not try again
+        return self._begin_prompt(self.prompt_chunk)
+
     def _check_slot(self, slot: int) -> None:
         if self.num_slots and not 0 <= slot < self.num_slots:
             raise ValueError(f"state slot {slot} outside [0, {self.num_slots})")
@@ -324,8 +335,18 @@ class PagedEngine:
             raise ValueError("not enough pages for the prompt")
         if len(block_ids) > self.max_pages:
             raise ValueError("sequence needs more pages than the block table is wide")
+        if chunk is not None and chunk < 0:
+            raise ValueError(f"prompt passes of {chunk} tokens")
         self._check_slot(slot)
-        chunk = self._begin_prompt(chunk or self.prompt_chunk)
+        given = chunk
+        chunk = given or self._default_chunk(n - cached_tokens)
+        try:
+            chunk = self._begin_prompt(chunk)
+        except torch.OutOfMemoryError:
+            if not self._may_shorten(given, chunk):
+                raise
+            chunk = 0
+        chunk = chunk or self._begin_shorter()
         row = torch.zeros(self.max_pages, dtype=torch.int32)
         row[: len(block_ids)] = torch.tensor(block_ids, dtype=torch.int32)
         row = row.to(self.device)
@@ -333,14 +354,24 @@ class PagedEngine:
         if want and not all(cached_tokens <= p < n for p in want):
             raise ValueError("logits can be asked for at the positions that are run")
         wanted = None if want is None else torch.empty(len(want), self.vocab_size, dtype=self.logits_dtype, device=self.device)
-        for lo in range(cached_tokens, n, chunk):
+        lo = cached_tokens
+        while lo < n:
             hi = min(n, lo + chunk)
-            h = self._prompt_hidden(token_ids[lo:hi], row, lo, chunk, slot)
+            h = None
+            try:
+                h = self._prompt_hidden(token_ids[lo:hi], row, lo, chunk, slot)
+            except torch.OutOfMemoryError:
+                if not self._may_shorten(given, chunk):
+                    raise
+            if h is None:  # outside the handler, which still holds the failed pass's tensors
+                chunk = self._begin_shorter()
+                continue
             here = [i for i, p in enumerate(want or ()) if lo <= p < hi]
             if here:
                 logits = self._logits(h[torch.tensor([want[i] - lo for i in here], device=self.device)])
                 wanted[torch.tensor(here, device=self.device)] = logits
             h_last = h[hi - lo - 1:hi - lo].contiguous()
+            lo = hi
         if want is not None or not self.keep_logits:
             return int(self._pick(h_last)[0]), wanted
         first, logits = self._pick_with_logits(h_last)
@@ -625,6 +656,23 @@ class DecodeEngine(PagedEngine):
     def _logits(self, h) -> torch.Tensor:
         return ops.dense_gemm(h, self.lm_head, status=self.gemm_status)
 
+    # A pass streams every expert's weights once, so a longer one costs less per token, and its rows need more memory.
+    short_prompt_chunk = 1024
+
+    def _default_chunk(self, tokens: int) -> int:
+        """1024 tokens for prompts of as many or fewer, 2048 beyond.  Milliseconds of a prompt in passes of 1024, 2048 and 4096
+        (qwen3-30b-a3b, 12 layers): 2048 tokens 5.7, 4.6, 4.7; 4096 tokens 12.0, 9.6, 9.7; 16000 tokens 70.3, 58.6, 57.3.
+        The expert workspace takes 57, 115 and 230 MB, a pass's rows 50, 100 and 200 MB more: the second doubling gives
+        little for it.  Once the larger buffers are there they serve every prompt.  Where attention runs a row per token its
+        split partials would double as well: 1024.
+        A row's bits may depend on the length: the o projection of at most about 256 rows is cut along K, so the last 91 rows
+        of 1115 have their sums in another order as a pass of their own (2047 and 1500 tokens give the same bits)."""
+        cfg = self.cfg
+        if not ops.paged_attn_prefill_supported(cfg.q_heads, cfg.kv_heads, cfg.head_dim, PAGE, torch.bfloat16):
+            return self.short_prompt_chunk
+        grown = getattr(self, "_prefill_chunk", 0) == self.prompt_chunk
+        return self.prompt_chunk if grown or tokens > self.short_prompt_chunk else self.short_prompt_chunk
+
     def _begin_prompt(self, chunk: int) -> int:
         ep = self.ep_state is not None
         if ep:
@@ -635,15 +683,22 @@ class DecodeEngine(PagedEngine):
         cfg = self.cfg
         tiled = ops.paged_attn_prefill_supported(cfg.q_heads, cfg.kv_heads, cfg.head_dim, PAGE, torch.bfloat16)
         if getattr(self, "_prefill_chunk", 0) != chunk:
-            self._prefill_chunk = chunk
+            # the buffers make room for the new ones; what their status words (at the start) have recorded stays
+            found = [None if ws is None else ws[:4].clone() for ws in
+                     (getattr(self, "_prefill_attn_ws", None), getattr(self, "_prefill_moe_ws", None))]
+            self._prefill_chunk, self._prefill_attn_ws, self._prefill_moe_ws = 0, None, None
             self._prefill_split = ops.default_split_tokens(chunk, cfg.kv_heads, self.max_pages * PAGE)
             # the tiled kernel needs no workspace beyond a status word; the row-per-token form needs the split
             # partials of `chunk` rows
-            self._prefill_attn_ws = torch.zeros(256, dtype=torch.uint8, device=self.device) if tiled else \
+            attn_ws = torch.zeros(256, dtype=torch.uint8, device=self.device) if tiled else \
                 ops.paged_attn_workspace(chunk, cfg.q_heads, cfg.head_dim, self.max_pages, PAGE, self._prefill_split,
                                          self.device)
-            self._prefill_moe_ws = None if ep else ops.moe_fp8_workspace(chunk, cfg.experts, cfg.top_k, cfg.hidden,
-                                                                         cfg.moe_inter, self.device)
+            moe_ws = None if ep else ops.moe_fp8_workspace(chunk, cfg.experts, cfg.top_k, cfg.hidden, cfg.moe_inter, self.device)
+            for ws, status in zip((attn_ws, moe_ws), found):
+                if ws is not None and status is not None:
+                    ws[:4] = status
+            self._prefill_attn_ws, self._prefill_moe_ws = attn_ws, moe_ws
+            self._prefill_chunk = chunk
         # consecutive prompt tokens share the table, so the row-per-token form takes them two rows per CTA where it can
         self._prefill_tiled = tiled
         self._prefill_pairs = not tiled and ops.paged_attn_pairs_supported(cfg.q_heads, cfg.kv_heads, cfg.head_dim, PAGE, torch.bfloat16)

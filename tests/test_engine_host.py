@@ -1,0 +1,104 @@
+"""Host side of the engines: how long a prompt pass is and what its buffers are sized for (CPU, no kernels)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from conftest import pkg
+
+HIDDEN = 8
+
+
+class HostEngine:
+    """DecodeEngine with the passes played on the host: at most `room_to_run` rows fit in one."""
+
+    def __new__(cls, q_heads=32, kv_heads=4, head_dim=128, room_to_run=1 << 30, ep_state=None):
+        eng = pkg("engine")
+
+        class Engine(eng.DecodeEngine):
+            def __init__(self):
+                self.cfg = SimpleNamespace(q_heads=q_heads, kv_heads=kv_heads, head_dim=head_dim, experts=16, top_k=4, hidden=512,
+                                           moe_inter=256, vocab_size=64)
+                self.device, self.max_pages, self.num_slots, self.keep_logits = torch.device("cpu"), 512, 0, False
+                self.ep_state, self.scratch_block, self.passes = ep_state, 0, []
+
+            def _prompt_hidden(self, token_ids, row, lo, chunk, slot):
+                if len(token_ids) > room_to_run:
+                    raise torch.OutOfMemoryError("rows")
+                self.passes.append((lo, len(token_ids)))
+                return torch.zeros(len(token_ids), HIDDEN)
+
+            def _pick(self, h, out=None):
+                return torch.zeros(h.shape[0], dtype=torch.int64)
+
+        return Engine()
+
+
+@pytest.fixture
+def host_ops(monkeypatch):
+    """Workspaces of one byte per row; more than `room` rows do not fit.  Notes the rows asked for."""
+    ops, box = pkg("ops"), SimpleNamespace(moe=[], attn=[], room=1 << 30)
+
+    def moe(rows, *a):
+        if rows > box.room:
+            raise torch.OutOfMemoryError("workspace")
+        box.moe.append(rows)
+        return torch.zeros(256 + rows, dtype=torch.uint8)
+
+    def attn(rows, *a):
+        box.attn.append(rows)
+        return torch.zeros(256 + rows, dtype=torch.uint8)
+
+    monkeypatch.setattr(ops, "moe_fp8_workspace", moe)
+    monkeypatch.setattr(ops, "paged_attn_workspace", attn)
+    return box
+
+
+def run(e, n, **kw):
+    e.passes.clear()
+    e.prefill(list(range(n)), list(range(-(-n // 16))), **kw)
+    return e.passes
+
+
+def test_prompt_buffers_are_sized_by_the_prompts(host_ops):
+    e = HostEngine()
+    assert run(e, 10) == [(0, 10)] and run(e, 1024) == [(0, 1024)] and host_ops.moe == [1024]
+    assert run(e, 1500, cached_tokens=600) == [(600, 900)] and host_ops.moe == [1024]
+    e._prefill_attn_ws[0], e._prefill_moe_ws[0] = 7, 9  # recorded findings outlive the growth
+    assert run(e, 2500) == [(0, 2048), (2048, 452)] and host_ops.moe == [1024, 2048]
+    assert (int(e._prefill_attn_ws[0]), int(e._prefill_moe_ws[0])) == (7, 9)
+    assert run(e, 10) == [(0, 10)] and host_ops.moe == [1024, 2048]
+    assert run(e, 100, chunk=64) == [(0, 64), (64, 36)] and host_ops.moe == [1024, 2048, 64]
+    with pytest.raises(ValueError):
+        run(e, 100, chunk=-1)
+
+
+def test_shapes_without_the_tiled_kernel_keep_short_passes(host_ops):
+    """Their split partials grow with the pass (32 / 8 heads of 128)."""
+    e = HostEngine(kv_heads=8)
+    assert run(e, 2500) == [(0, 1024), (1024, 1024), (2048, 452)] and host_ops.attn == host_ops.moe == [1024]
+
+
+def test_a_default_pass_that_does_not_fit_runs_as_shorter_ones(host_ops):
+    e = HostEngine()
+    host_ops.room = 1024
+    want = [(0, 1024), (1024, 1024), (2048, 452)]
+    assert run(e, 2500) == want and run(e, 2500) == want and host_ops.moe == [1024]
+    with pytest.raises(torch.OutOfMemoryError):  # asked for
+        run(e, 2500, chunk=2048)
+    host_ops.room = 1 << 30
+    e = HostEngine(room_to_run=1500)  # the buffers fit, the rows do not
+    assert run(e, 2500) == want and run(e, 2500) == want
+    with pytest.raises(torch.OutOfMemoryError):
+        run(e, 2500, chunk=2048)
+    e = HostEngine(room_to_run=1000)
+    with pytest.raises(torch.OutOfMemoryError):
+        run(e, 2500)
+
+
+def test_an_expert_parallel_pass_is_never_run_twice(host_ops):
+    """The other ranks have taken part in the round."""
+    e = HostEngine(room_to_run=1500, ep_state=SimpleNamespace(T=2048))
+    with pytest.raises(torch.OutOfMemoryError):
+        run(e, 2500)
+    assert e.passes == []

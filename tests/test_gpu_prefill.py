@@ -106,3 +106,21 @@ def test_merged_decode_step_and_prompt_chunk_equals_the_two_passes(ops):
     flat_a = [t for a in tr_a for t in a[0] + [a[1]]]
     flat_b = [t for b in tr_b for t in b[0] + [b[1]]]
     assert sum(x == y for x, y in zip(flat_a, flat_b)) >= len(flat_a) - 2, (tr_a, tr_b)  # 9 tokens, near-ties aside
+
+
+@pytest.mark.parametrize("n", [1115, 2047])
+def test_default_pass_agrees_with_passes_of_1024_tokens(ops, n):
+    """A default pass takes more than 1024 tokens at once (for 1115 the o projection of the last 91 rows is cut along K in
+    the one and not in the other): the same model to rounding."""
+    eng = pkg("engine")
+    engine = eng.DecodeEngine(eng.CONFIGS["tiny"], num_blocks=128, max_batch=2, max_pages_per_seq=128, device=DEV, seed=3, keep_logits=True)
+    prompt = torch.randint(0, 4096, (n,), generator=torch.Generator().manual_seed(n)).tolist()
+    blocks, want = list(range(-(-n // 16))), [0, 1023, 1024, n - 1]
+    _, long = engine.prefill(prompt, blocks, want=want)
+    assert engine._prefill_chunk == 2048
+    k_long = [p[blocks].clone() for p in engine.k_pools]
+    _, short = engine.prefill(prompt, blocks, chunk=1024, want=want)
+    engine.check_status("prompt passes")
+    assert rel_err(long, short) < TOL_MODEL
+    for a, p in zip(k_long, engine.k_pools):
+        assert rel_err(p[blocks], a) < TOL_MODEL
