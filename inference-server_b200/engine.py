@@ -650,7 +650,7 @@ class DecodeEngine(PagedEngine):
         return ops.lm_head_argmax(h, self.lm_head, self.argmax_ws, out=out, status=self.gemm_status)
 
     def _pick_with_logits(self, h, out=None) -> tuple[torch.Tensor, torch.Tensor]:
-        logits = torch.empty(h.shape[0], self.vocab_size, dtype=self.logits_dtype, device=self.device)
+        logits = torch.empty(h.shape[0], self.lm_head.shape[0], dtype=self.logits_dtype, device=self.device)
         return ops.lm_head_argmax(h, self.lm_head, self.argmax_ws, out=out, status=self.gemm_status, logits=logits), logits
 
     def _logits(self, h) -> torch.Tensor:

@@ -102,3 +102,16 @@ def test_an_expert_parallel_pass_is_never_run_twice(host_ops):
     with pytest.raises(torch.OutOfMemoryError):
         run(e, 2500)
     assert e.passes == []
+
+
+def test_kept_logits_have_the_rows_of_the_output_matrix(monkeypatch):
+    """It may be padded beyond the vocabulary of the configuration."""
+    def argmax(x, w, workspace=None, out=None, status=None, logits=None):
+        assert logits.shape == (x.shape[0], w.shape[0]) and logits.dtype == torch.bfloat16
+        return logits.zero_().argmax(1)
+
+    monkeypatch.setattr(pkg("ops"), "lm_head_argmax", argmax)
+    e = HostEngine()
+    e.lm_head, e.vocab_size, e.argmax_ws, e.gemm_status = torch.zeros(80, HIDDEN), 64, None, None
+    tokens, logits = e._pick_with_logits(torch.zeros(3, HIDDEN))
+    assert tokens.shape == (3,) and logits.shape == (3, 80)
