@@ -390,6 +390,7 @@ class PagedEngine:
         decode kernel for the rest.
         Returns (next tokens of the B decode rows (device), token after the chunk's last position, its logits);
         the last two are None unless `want_first` (the logits also unless the engine was built with keep_logits).
+        With keep_logits `last_logits` holds the decode rows' logits, as after a step.
         Advances ctx_lens of the decode rows by one."""
         n = len(chunk_token_ids)
         if self.ep_state is not None:
@@ -408,15 +409,16 @@ class PagedEngine:
         table = torch.cat([row.unsqueeze(0).expand(n, -1), self.block_table[:B]])
         h = self._mixed_hidden(tokens, pos, table, first_pos, n, B, slot)
         first = logits = None
-        if want_first:
-            # the chunk's last row and the decode rows are neighbours: lm_head is streamed once for both
-            nxt = self._pick(h[n - 1:])
-            self.next_tokens[:B].copy_(nxt[1:])
-            first = int(nxt[0])
+        # the chunk's last row and the decode rows are neighbours: lm_head is streamed once for both
+        lo, out = (n - 1, None) if want_first else (n, self.next_tokens[:B])
+        if self.keep_logits:
+            nxt, kept = self._pick_with_logits(h[lo:], out)
+            self.last_logits = kept[n - lo:]
         else:
-            self._pick(h[n:], self.next_tokens[:B])
-        if want_first and self.keep_logits:
-            logits = self._logits(h[n - 1:n])[0]
+            nxt, kept = self._pick(h[lo:], out), None
+        if want_first:
+            self.next_tokens[:B].copy_(nxt[1:])
+            first, logits = int(nxt[0]), None if kept is None else kept[0]
         self.ctx_lens[:B] += 1
         return self.next_tokens[:B], first, logits
 

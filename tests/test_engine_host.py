@@ -115,3 +115,22 @@ def test_kept_logits_have_the_rows_of_the_output_matrix(monkeypatch):
     e.lm_head, e.vocab_size, e.argmax_ws, e.gemm_status = torch.zeros(80, HIDDEN), 64, None, None
     tokens, logits = e._pick_with_logits(torch.zeros(3, HIDDEN))
     assert tokens.shape == (3,) and logits.shape == (3, 80)
+
+
+@pytest.mark.parametrize("want_first", [True, False])
+def test_a_mixed_pass_leaves_the_logits_of_its_decode_rows(want_first):
+    """Row i of the pass has logits of i: two rows of a chunk, three of a decode step."""
+    n, B = 2, 3
+    e = HostEngine()
+    e.keep_logits, e.max_batch, e.last_logits = True, B, "an earlier step's"
+    e.tokens, e.ctx_lens, e.next_tokens = (torch.zeros(B, dtype=t) for t in (torch.int64, torch.int32, torch.int64))
+    e.block_table = torch.zeros(B, e.max_pages, dtype=torch.int32)
+    rows = torch.arange(n + B).float().view(-1, 1)
+    e._mixed_hidden = lambda *a: rows
+    e._pick = lambda h, out=None: h[:, 0].long() if out is None else out.copy_(h[:, 0].long())
+    e._logits = lambda h: h.expand(-1, 4)
+    e._pick_with_logits = lambda h, out=None: (e._pick(h, out), e._logits(h))
+    tokens, first, logits = e.mixed_step(B, [5, 6], [0], 0, want_first=want_first)
+    assert tokens.tolist() == [2, 3, 4] and e.ctx_lens.tolist() == [1, 1, 1]
+    assert torch.equal(e.last_logits, rows[n:].expand(-1, 4))
+    assert first == (1 if want_first else None) and (logits.tolist() == [1.0] * 4 if want_first else logits is None)
