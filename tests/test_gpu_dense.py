@@ -135,6 +135,20 @@ def test_lm_head_argmax_writes_the_logits_of_the_plain_product(ops, M, V, K, dty
     assert torch.equal(tok, ops.lm_head_argmax(xd, wd))
 
 
+@pytest.mark.parametrize("M,V,K", [(256, 151936, 128), (33, 60001, 64), (1, 151936, 64)])
+def test_lm_head_logits_of_several_weight_tiles_per_cta(ops, M, V, K):
+    """Three tiles a CTA and more: accumulators are used again and a tile's logits are stored while the next one's products run.
+    The token is the arg-max of the fp32 logits as far as their keys go, which drop 5 of 24 bits."""
+    x, w, _ = make(M, V, K, seed=V + M, wstd=1.0)
+    xd, wd = x.to(DEV), w.to(DEV)
+    for dtype, want in ((torch.bfloat16, ops.dense_gemm(xd, wd, k_split=1)), (torch.float32, ops.dense_gemm_f32_out(xd, wd))):
+        logits = torch.full((M, V), float("nan"), dtype=dtype, device=DEV)
+        tok = ops.lm_head_argmax(xd, wd, logits=logits)
+        assert torch.equal(logits, want)
+    best = logits.max(dim=1).values
+    assert bool((best - logits[torch.arange(M, device=DEV), tok] <= 2.0 ** -18 * best.abs()).all())
+
+
 @pytest.mark.parametrize("R,hq,hkv,K", [(256, 32, 4, 2048), (1, 32, 4, 2048), (37, 64, 4, 4096), (300, 8, 2, 512)])
 def test_qkv_projection_with_norm_rope_and_page_write_equals_the_two_kernels(ops, R, hq, hkv, K):
     """b200_qkv_rope_append_gemm against b200_dense_gemm_bf16 (no K split) + b200_qk_norm_rope_append: the query
