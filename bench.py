@@ -319,7 +319,7 @@ def prefill_phase(args, cfg, dev, rank, world):
     torch.cuda.synchronize()
     e2e_s = time.perf_counter() - t0
     # the attention kernel alone: one chunk-sized launch per layer on that layer's own pages
-    chunk = min(n, 1024)
+    chunk = min(n, engine._default_chunk(n))
     q = torch.randn(chunk, cfg.q_heads, cfg.head_dim, device=dev, dtype=torch.bfloat16)
     row = torch.zeros(engine.max_pages, dtype=torch.int32, device=dev)
     row[:pages] = torch.arange(3 * pages, 4 * pages, dtype=torch.int32, device=dev)
@@ -355,12 +355,12 @@ def prefill_phase(args, cfg, dev, rank, world):
     line = {"metric": "prefill tok/s", "value": args.steps * n / (ms / 1e3), "unit": "tok/s", "n_gpus": 1, "steps": args.steps,
             "warmup": max(3, args.warmup), "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "fp8 experts (e4m3, fp32 accumulate) + bf16 attention/dense", "data": "synthetic",
-            "config": {"workload": f"{args.model} prompt pass, one sequence of {n} random token ids per step, chunks of 1024, "
+            "config": {"workload": f"{args.model} prompt pass, one sequence of {n} random token ids per step, chunks of {chunk}, "
                                    f"page {PAGE}, cold prefix cache (outside the headline decode metric)",
                        "l2": "every step runs all layers: 32 GB of weights between two uses of any page"},
             "e2e": {"value": args.steps * n / e2e_s, "unit": "tok/s", "h2d_bytes_per_step": n * 8, "d2h_bytes_per_step": 8,
                     "api": "B200Backend.prefill"},
-            "gpu_launches": engine.kernel_launches_per_step * args.steps * ((n + 1023) // 1024),
+            "gpu_launches": engine.kernel_launches_per_step * args.steps * -(-n // chunk),
             "clocks": clocks.summary(), "roofline": roof}
     print(json.dumps(line))
 
