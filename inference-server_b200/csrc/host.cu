@@ -118,18 +118,36 @@ struct MapKey {
   uint32_t box[4];
   uint64_t stride[3];  // bytes, of dim[1..]
   bool operator==(const MapKey& o) const {
+    if (base != o.base || device != o.device || elem_bytes != o.elem_bytes) return false;
     for (int i = 0; i < 4; ++i)
       if (dim[i] != o.dim[i] || box[i] != o.box[i] || (i < 3 && stride[i] != o.stride[i])) return false;
-    return device == o.device && base == o.base && elem_bytes == o.elem_bytes;
+    return true;
   }
+  size_t set() const {  // FNV-1a over the words, folded
+    uint64_t h = 14695981039346656037ull;
+    auto mix = [&h](uint64_t v) { h = (h ^ v) * 1099511628211ull; };
+    mix(reinterpret_cast<uintptr_t>(base));
+    mix(static_cast<uint64_t>(device) << 32 | static_cast<uint32_t>(elem_bytes));
+    for (int i = 0; i < 4; ++i) mix(dim[i] << 9 ^ box[i]);
+    for (int i = 0; i < 3; ++i) mix(stride[i]);
+    return static_cast<size_t>((h ^ h >> 29 ^ h >> 47) % kMapSets);
+  }
+  static constexpr size_t kMapSets = 1024;
 };
 struct MapEntry {
   MapKey key;
   CUtensorMap map;
 };
+// Encoded maps in sets of eight, the oldest of a full set making room.  Every launch looks up a few, so a lookup must not depend
+// on how many there are: a list that was searched from its start took 5 us a lookup with 4000 maps in it, and passes of
+// few rows, whose launches the host issues one by one, are bound by that.
+struct MapSet {
+  MapEntry entry[8];
+  uint32_t used = 0;  // entries ever put here
+};
 
 static std::mutex g_map_mu;
-static std::vector<MapEntry> g_maps;
+static MapSet* g_maps = nullptr;
 static EncodeTiledFn g_encode = nullptr;
 
 // Tensor of `rank` 2 to 4 dimensions.
@@ -137,9 +155,11 @@ static int get_tensor_map(int rank, MapKey key, CUtensorMap* out) {
   cudaError_t ce = cudaGetDevice(&key.device);
   if (ce != cudaSuccess) return cuda_fail(ce, "cudaGetDevice");
   std::lock_guard<std::mutex> lock(g_map_mu);
-  for (const MapEntry& e : g_maps) {
-    if (e.key == key) {
-      *out = e.map;
+  if (g_maps == nullptr) g_maps = new MapSet[MapKey::kMapSets];
+  MapSet& set = g_maps[key.set()];
+  for (uint32_t i = 0; i < 8 && i < set.used; ++i) {
+    if (set.entry[i].key == key) {
+      *out = set.entry[i].map;
       return 0;
     }
   }
@@ -175,8 +195,8 @@ static int get_tensor_map(int rank, MapKey key, CUtensorMap* out) {
     set_detail("cuTensorMapEncodeTiled failed with CUresult %d (base %p rows %llu cols %llu)", (int)r, key.base, rows, cols);
     return -kErrTensorMap;
   }
-  if (g_maps.size() >= 4096) g_maps.erase(g_maps.begin(), g_maps.begin() + 2048);
-  g_maps.push_back(entry);
+  set.entry[set.used % 8] = entry;
+  if (++set.used == 16) set.used = 8;
   *out = entry.map;
   return 0;
 }

@@ -213,3 +213,32 @@ def test_qkv_projection_epilogue_reports_bad_positions_and_pages(ops):
     ops.qkv_rope_append_gemm(x, w, one, one, cs, cs, pos, table, pool, pool.clone(), hq, 1e-6, status)
     with pytest.raises(Exception, match="block table entry"):
         ops.read_status(status, "qkv_rope_append_gemm")
+
+
+def test_launches_do_not_slow_down_with_the_number_of_operands_seen(ops):
+    """Every launch looks up the tensor maps of its operands.  After 10000 other operands, more than are kept, results are right, for
+    operands first seen long ago too, and a call takes the host no longer (best of many; a search through 4000 maps took
+    a second 9 us)."""
+    import time
+
+    w, n = make(1, 128, 64, seed=0)[1].to(DEV), 10000
+    many = torch.randn(n, 256, generator=torch.Generator().manual_seed(1)).bfloat16().to(DEV)
+    out = torch.empty(4, 128, dtype=torch.bfloat16, device=DEV)
+
+    def host_us(a):
+        best = float("inf")
+        for _ in range(30):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            for _ in range(50):
+                ops.dense_gemm(a, w, out=out, k_split=1)
+            best = min(best, (time.perf_counter() - t) / 50 * 1e6)
+        return best
+
+    before = host_us(many[0].view(4, 64))
+    for i in range(n):
+        ops.dense_gemm(many[i].view(4, 64), w, out=out, k_split=1)
+    for i in (0, 1, 4999, n - 1):
+        got = ops.dense_gemm(many[i].view(4, 64), w, k_split=1)
+        assert rel_err(got, many[i].view(4, 64).float().cpu() @ w.float().cpu().t()) < TOL
+    assert host_us(many[n - 1].view(4, 64)) < 1.5 * before
