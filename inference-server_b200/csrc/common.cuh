@@ -237,7 +237,7 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
                    bar)
                : "memory");
 }
-// The same from a converged warp, by its elected lane.
+// The same from a converged warp, by its elected lane (mixed_prefill_tc.cu, whose issue loops are a whole warp's).
 __device__ __forceinline__ void tc_commit_elected(uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred e;\n\t"

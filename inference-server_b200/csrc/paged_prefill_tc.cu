@@ -11,9 +11,8 @@
 //            head into a two-stage ring; warp 11 does the same with V.  A page (16 tokens) is one box of 8-row
 //            swizzled atoms.  A TMA copy costs about 100 cycles to issue whatever its size, and 32 copies of
 //            2 KB per key tile from one warp were what the kernel waited for: 3300 cycles per key tile, with or
-//            without its exponentials, its products or its P stores. With a box per page and two warps
-//            1024 tokens behind 14 k, 32 / 4 heads: 400 -> 330 us, 2048 tokens in two chunks 47 -> 39 us each, 91
-//            tokens 12.9 -> 11.6 us.
+//            without its exponentials, its products or its P stores. With a box per page and two warps, 32 / 4 heads: 1024 tokens
+//            behind 14336 398 -> 325 us, from nothing 32.8 -> 27.6 us, 91 tokens behind 1000 21.5 -> 18.1 us.
 //   warp 1   score issuer (one thread): S = Q K^T as 8 x tcgen05.mma M128 N128 K16 (kind::f16, bf16, both
 //            operands K-major) into one of two S accumulators in TMEM, as far ahead as those allow.
 //   warp 2   P V issuer (one thread): O += P V as 2 x 4 tcgen05.mma M128 N128 K16, P (bf16, written by the
