@@ -669,11 +669,13 @@ class DecodeEngine(PagedEngine):
         split partials would double as well: 1024.
         A row's bits may depend on the length: the o projection of at most about 256 rows is cut along K, so the last 91 rows
         of 1115 have their sums in another order as a pass of their own (2047 and 1500 tokens give the same bits)."""
-        cfg = self.cfg
+        cfg, short = self.cfg, min(self.short_prompt_chunk, self.prompt_chunk)
+        if "prompt_chunk" in vars(self):  # set for this engine
+            return self.prompt_chunk
         if not ops.paged_attn_prefill_supported(cfg.q_heads, cfg.kv_heads, cfg.head_dim, PAGE, torch.bfloat16):
-            return self.short_prompt_chunk
+            return short
         grown = getattr(self, "_prefill_chunk", 0) == self.prompt_chunk
-        return self.prompt_chunk if grown or tokens > self.short_prompt_chunk else self.short_prompt_chunk
+        return self.prompt_chunk if grown or tokens > short else short
 
     def _begin_prompt(self, chunk: int) -> int:
         ep = self.ep_state is not None

@@ -73,6 +73,14 @@ def test_prompt_buffers_are_sized_by_the_prompts(host_ops):
         run(e, 100, chunk=-1)
 
 
+@pytest.mark.parametrize("chunk,kv_heads", [(512, 4), (3000, 4), (3000, 8)])
+def test_a_pass_length_set_for_the_engine_is_kept(host_ops, chunk, kv_heads):
+    e = HostEngine(kv_heads=kv_heads)
+    e.prompt_chunk = chunk
+    assert run(e, 700) == [(lo, min(chunk, 700 - lo)) for lo in range(0, 700, chunk)]
+    assert run(e, 2500) == [(lo, min(chunk, 2500 - lo)) for lo in range(0, 2500, chunk)] and host_ops.moe == [chunk]
+
+
 def test_shapes_without_the_tiled_kernel_keep_short_passes(host_ops):
     """Their split partials grow with the pass (32 / 8 heads of 128)."""
     e = HostEngine(kv_heads=8)
