@@ -4,7 +4,10 @@
 // reference is described there (src/inference_server/kv_cache/hf_format.py:21-45 gather +
 // src/inference_server/backends/torch_backend.py:107-147 chunk forward).
 //
-//   grid     (query tiles, kv heads).  A CTA owns 128 rows of the score matrix: 128 / G consecutive prompt
+// This form has one tile of rows per CTA and short chains; it serves calls whose tiles all have an SM of their own and whose
+// walks are short (paged_prefill_pairs.cu has the rule and the other form).
+//
+//   grid     query tiles x kv heads.  A CTA owns 128 rows of the score matrix: 128 / G consecutive prompt
 //            positions x the G query heads of its kv head, and walks the key tiles (128 keys = 8 pages) of
 //            the context up to its last position.  Heavy tiles (late positions) are issued first.
 //   warp 0   TMA producer: the Q tile once, then per key tile the 8 K pages of the kv
@@ -47,16 +50,11 @@
 // kErrDevWaitTimeout and the thread stops waiting but keeps the loop structure (the named barriers between
 // partner warps are still met), so the kernel ends.
 
-#include "common.cuh"
 #include "host.h"
+#include "prefill_tc.cuh"
 
 namespace b200 {
 
-constexpr int kTcPage = 16;
-constexpr int kTcRows = 128;                 // score rows per CTA = M of the MMAs
-constexpr int kTcKeys = 128;                 // keys per tile = N of S, K of P V
-constexpr int kTcPages = kTcKeys / kTcPage;
-constexpr int kTcHalfBytes = 128 * 128;      // 128 rows x 64 bf16: one swizzled column half of a tile
 constexpr int kTcPBytes = 2 * kTcHalfBytes;  // P: 128 rows x 128 keys
 constexpr int kTcSoftmaxWarps = 8;
 constexpr int kTcThreads = (4 + kTcSoftmaxWarps) * 32;
@@ -68,53 +66,6 @@ struct TcCfg {
   static constexpr int kRingBytes = 5 * kTileBytes + kTcPBytes;            // Q, P, K0, K1, V0, V1
   static constexpr int kSmemBytes = kRingBytes + 1024 + kTcExtraBytes;
 };
-constexpr float kTcRescaleLog2 = 8.f;        // rescale O when the max grew by more than this (log2 domain)
-
-// bf16 x bf16 -> f32; A K-major; B K-major or (b_mn) MN-major.
-__host__ __device__ constexpr uint32_t tc_idesc_bf16(uint32_t m, uint32_t n, uint32_t b_mn) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
-}
-// Descriptor of an MN-major operand tile with 128-byte swizzle: 64 elements of the M/N dimension are contiguous
-// (128 B), consecutive K rows are 128 B apart, groups of 8 K rows `sbo` bytes apart, and the next 64 elements of
-// the M/N dimension start `lbo` bytes further.
-__device__ __forceinline__ uint64_t umma_desc_mn128(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>(lbo >> 4) << 16;
-  d |= static_cast<uint64_t>(sbo >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;  // descriptor version (sm_100)
-  d |= static_cast<uint64_t>(2) << 61;  // 128-byte swizzle
-  return d;
-}
-// Descriptor of a K-major operand tile of 8 x 128 B swizzled atoms; groups of 8 rows `sbo` bytes apart.
-__device__ __forceinline__ uint64_t tc_desc_k_atoms(uint32_t smem_addr, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>(1) << 16;  // leading byte offset (unused)
-  d |= static_cast<uint64_t>(sbo >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;  // descriptor version (sm_100)
-  d |= static_cast<uint64_t>(2) << 61;  // 128-byte swizzle
-  return d;
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]),
-        "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]),
-        "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() {
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 
 // The two warps that own the same 32 score rows (warp w and w + 4 of the softmax warps) meet here.
 __device__ __forceinline__ void pair_barrier(int quarter) {
@@ -190,18 +141,19 @@ paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_sm;
-  // Set-up done; Q and this chunk's K/V rows come from the kernel before this one.
-  grid_dep_wait();
-  grid_dep_launch();
-
-  const int qt = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);  // late positions first
-  const int h = blockIdx.y;
+  // late positions first, all kv heads of them side by side
+  const int qt = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) / num_kv_heads;
+  const int h = static_cast<int>(blockIdx.x) % num_kv_heads;
   const int t0 = qt * QT;
   const int t_end = min(t0 + QT, num_tokens);       // one past the tile's last real prompt token
   const int last_pos = first_pos + t_end - 1;       // last position any row of this CTA sees
   const int kt0 = first_visible(first_pos + t0 + 1, chunk) / kTcKeys;  // key tile of the first key any row sees
   const int n_tiles = last_pos / kTcKeys - kt0 + 1;
   const int last_page = last_pos / kTcPage;
+
+  // Set-up done; Q and this chunk's K/V rows come from the kernel before this one.
+  grid_dep_wait();
+  grid_dep_launch();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA ------
@@ -452,7 +404,7 @@ static int launch_prefill_tc_g(const CUtensorMap& qmap, const CUtensorMap& kmap,
                                const int* table_row, void* out, int* err, int num_tokens, int first_pos, int hq, int hkv,
                                int num_blocks, float scale, int chunk, const float* gate, cudaStream_t st) {
   const int group = hq / hkv, qt = kTcRows / group;
-  const dim3 grid((num_tokens + qt - 1) / qt, hkv);
+  const dim3 grid((num_tokens + qt - 1) / qt * hkv);
   int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&paged_attn_prefill_tc_kernel<D, G>), TcCfg<D>::kSmemBytes);
   if (rc) return rc;
   B200_CUDA(launch_overlapped(paged_attn_prefill_tc_kernel<D, G>, grid, dim3(kTcThreads), TcCfg<D>::kSmemBytes, st, qmap,
@@ -462,30 +414,12 @@ static int launch_prefill_tc_g(const CUtensorMap& qmap, const CUtensorMap& kmap,
   return 0;
 }
 
-// The tcgen05 form of the prompt attention: head_dim 64 or 128, 1 to 128 query heads per kv head, at most 65535 kv
-// heads, q and out 16-byte aligned.  Arguments as launch_prefill in paged_prefill.cu, which has checked them.
-int launch_prefill_tc(const void* q, const void* k_pool, const void* v_pool, const int* table_row, void* out, int* err,
-                      int num_tokens, int first_pos, int hq, int hkv, int head_dim, int num_blocks, float scale,
-                      int chunk, const float* gate, cudaStream_t st) {
-  const int group = hq / hkv;
-  CUtensorMap qmap, kmap, vmap;
-  const uint64_t rows = static_cast<uint64_t>(num_blocks) * hkv * kTcPage;
-  int rc = get_tensor_map_atoms(k_pool, rows, head_dim, kTcPage, &kmap);
-  if (rc) return rc;
-  rc = get_tensor_map_atoms(v_pool, rows, head_dim, kTcPage, &vmap);
-  if (rc) return rc;
-  const bool q_tma = head_dim == 128 && (group == 8 || group == 16);
-  if (q_tma) {
-    // 8 query heads per kv head: the CTA's positions in one box; 16: a box per position
-    rc = group == 8 ? get_tensor_map_atoms_of(q, num_tokens, hq, head_dim, kTcRows / 8, &qmap)
-                    : get_tensor_map_atoms(q, static_cast<uint64_t>(num_tokens) * hq, head_dim, 16, &qmap);
-    if (rc) return rc;
-  } else {
-    qmap = kmap;  // not read
-  }
-#define B200_TC_ARGS qmap, kmap, vmap, q, table_row, out, err, num_tokens, first_pos, hq, hkv, num_blocks, scale, chunk, \
-                     gate, st
-  if (q_tma && group == 8) return launch_prefill_tc_g<128, 8>(B200_TC_ARGS);
+// Arguments as launch_prefill_pairs, which calls this form where it is the better one.
+int launch_prefill_single(const CUtensorMap& qmap, const CUtensorMap& kmap, const CUtensorMap& vmap, bool q_tma, int head_dim, const void* q,
+                          const int* table_row, void* out, int* err, int num_tokens, int first_pos, int hq, int hkv, int num_blocks,
+                          float scale, int chunk, const float* gate, cudaStream_t st) {
+#define B200_TC_ARGS qmap, kmap, vmap, q, table_row, out, err, num_tokens, first_pos, hq, hkv, num_blocks, scale, chunk, gate, st
+  if (q_tma && hq / hkv == 8) return launch_prefill_tc_g<128, 8>(B200_TC_ARGS);
   if (q_tma) return launch_prefill_tc_g<128, 16>(B200_TC_ARGS);
   if (head_dim == 128) return launch_prefill_tc_g<128, 0>(B200_TC_ARGS);
   return launch_prefill_tc_g<64, 0>(B200_TC_ARGS);

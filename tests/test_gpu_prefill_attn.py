@@ -75,3 +75,37 @@ def test_positions_past_the_table_and_bad_pages_are_reported_not_read(ops):
     ops.paged_attn_prefill(q.to(DEV), kp.to(DEV), vp.to(DEV), bad.to(DEV), 0, 0.1, status)
     with pytest.raises(Exception, match="block table entry"):
         ops.read_status(status, "paged_attn_prefill")
+
+
+@pytest.mark.parametrize("hq,hkv,d,first,rows,chunk", [
+    (32, 4, 128, 0, 1280, 0),       # TMA queries, 8 heads per kv head, several waves
+    (32, 4, 128, 5000, 1008, 0),    # an odd number of tiles: the last CTA has one
+    (64, 4, 128, 123, 661, 0),      # 16 heads per kv head, a last tile of five positions
+    (24, 8, 128, 300, 977, 0),      # 42 positions per tile, copied queries
+    (64, 4, 128, 121, 700, 128),    # chunk edges between and inside the tiles of a CTA
+    (40, 8, 64, 77, 1900, 512),     # head_dim 64; tiles that see different numbers of key tiles
+])
+def test_two_tiles_per_cta_give_the_bits_of_one(ops, hq, hkv, d, first, rows, chunk):
+    """More tiles of rows than SMs: two per CTA.  The same rows in calls of a few whole tiles each, one per CTA: the same bits."""
+    q, kp, vp, row = (t.to(DEV) for t in case(hq, hkv, d, first, rows, seed=rows))
+    gate = torch.randn(rows, hq, generator=torch.Generator().manual_seed(1)).to(DEV)
+    status = torch.zeros(64, dtype=torch.int32, device=DEV)
+
+    def run(lo, hi):
+        return ops.paged_attn_prefill_chunked(q[lo:hi], kp, vp, row, first + lo, d ** -0.5, status, chunk, gate[lo:hi])
+
+    tile = 128 // (hq // hkv)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert -(-rows // tile) * hkv > sms
+    step = sms // hkv // 2 * tile
+    whole = run(0, rows)
+    pieces = torch.cat([run(lo, min(rows, lo + step)) for lo in range(0, rows, step)])
+    ops.read_status(status, "paged_attn_prefill_chunked")
+    assert torch.equal(whole, pieces)
+    # and a few rows against decode attention, which sees a row's own chunk likewise: two results that round P and the output to bf16
+    # (2^-9 each) differ by at most 4 * 2^-9 = 7.8e-3
+    for p in (0, rows // 2, rows - 1):
+        ws = ops.paged_attn_workspace(1, hq, d, row.numel(), 16, 1024, DEV)
+        lens = torch.tensor([first + p + 1], dtype=torch.int32, device=DEV)
+        dec = ops.paged_attn_decode_chunked(q[p:p + 1], kp, vp, row[None], lens, d ** -0.5, 1024, ws, chunk, gate[p:p + 1])
+        assert rel_err(whole[p:p + 1], dec) < TOL
