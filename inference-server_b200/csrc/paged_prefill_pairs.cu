@@ -88,19 +88,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return d;
 }
 
-// Whether a phase is over, asked without waiting: the answer can be on its way while other work runs.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // G: query heads per kv head (8 or 16, Q tiles by TMA); 0 = `group` of them.
 template <int D, int G>
 __global__ void __launch_bounds__(kPairThreads, 1)
