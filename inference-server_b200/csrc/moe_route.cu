@@ -31,10 +31,12 @@ constexpr int kRouteMaxPerLane = 8;  // num_experts <= 256
 __device__ __forceinline__ float logit_f32(const float* p, size_t i) { return p[i]; }
 __device__ __forceinline__ float logit_f32(const __nv_bfloat16* p, size_t i) { return __bfloat162float(p[i]); }
 
-template <typename LT>
+template <typename LT, int PER>
 __global__ void __launch_bounds__(kRouteWarps * 32)
 moe_route_kernel(const LT* __restrict__ logits, int T, int E, int K, int renorm,
                  const int* __restrict__ num_valid, int* __restrict__ topk_ids, float* __restrict__ topk_w) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * kRouteWarps + warp;
   if (t >= T) return;
@@ -45,56 +47,29 @@ moe_route_kernel(const LT* __restrict__ logits, int T, int E, int K, int renorm,
     }
     return;
   }
-  float v[kRouteMaxPerLane];
-  float mx = -INFINITY;
+  float v[PER];
 #pragma unroll
-  for (int j = 0; j < kRouteMaxPerLane; ++j) {
+  for (int j = 0; j < PER; ++j) {
     const int e = lane + 32 * j;
     v[j] = e < E ? logit_f32(logits, static_cast<size_t>(t) * E + e) : -INFINITY;
-    mx = fmaxf(mx, v[j]);
   }
-  mx = warp_max(mx);
+  float mine;
+  int my_id;
+  warp_topk<PER>(v, E, K, lane, &mine, &my_id);
+  const float mx = __shfl_sync(0xffffffffu, mine, 0);
+  const float my_p = expf(mine - mx);
   float den = 0.f;
+  if (renorm) {
+    den = lane_sum_in_order(my_p, K);
+  } else {
 #pragma unroll
-  for (int j = 0; j < kRouteMaxPerLane; ++j)
-    if (lane + 32 * j < E) den += expf(v[j] - mx);
-  den = warp_sum(den);
-
-  unsigned taken = 0;  // bit j: this lane's candidate j has been selected
-  float sel_sum = 0.f, my_p = 0.f;
-  int my_id = 0;
-  for (int k = 0; k < K; ++k) {
-    float bv = -INFINITY;
-    int be = 0x7fffffff;
-#pragma unroll
-    for (int j = 0; j < kRouteMaxPerLane; ++j) {
-      const int e = lane + 32 * j;
-      if (e < E && !((taken >> j) & 1u) && (be == 0x7fffffff || v[j] > bv)) {
-        bv = v[j];
-        be = e;
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int oe = __shfl_xor_sync(0xffffffffu, be, o);
-      const bool better = oe != 0x7fffffff && (be == 0x7fffffff || ov > bv || (ov == bv && oe < be));
-      if (better) {
-        bv = ov;
-        be = oe;
-      }
-    }
-    if ((be & 31) == lane) taken |= 1u << (be >> 5);
-    const float p = expf(bv - mx);
-    sel_sum += p;
-    if (lane == k) {
-      my_p = p;
-      my_id = be;
-    }
+    for (int j = 0; j < PER; ++j)
+      if (lane + 32 * j < E) den += expf(v[j] - mx);
+    den = warp_sum(den);
   }
   if (lane < K) {
     topk_ids[static_cast<size_t>(t) * K + lane] = my_id;
-    topk_w[static_cast<size_t>(t) * K + lane] = my_p / (renorm ? sel_sum : den);
+    topk_w[static_cast<size_t>(t) * K + lane] = my_p / den;
   }
 }
 
@@ -115,37 +90,11 @@ moe_route_sigmoid_kernel(const LT* __restrict__ logits, int T, int E, int K, int
     const int e = lane + 32 * j;
     v[j] = e < E ? logit_f32(logits, static_cast<size_t>(t) * E + e) : -INFINITY;
   }
-  unsigned taken = 0;
-  float sum = 0.f, my_s = 0.f;
-  int my_id = 0;
-  for (int k = 0; k < K; ++k) {
-    float bv = -INFINITY;
-    int be = 0x7fffffff;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      const int e = lane + 32 * j;
-      if (e < E && !((taken >> j) & 1u) && (be == 0x7fffffff || v[j] > bv)) {
-        bv = v[j];
-        be = e;
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int oe = __shfl_xor_sync(0xffffffffu, be, o);
-      if (oe != 0x7fffffff && (be == 0x7fffffff || ov > bv || (ov == bv && oe < be))) {
-        bv = ov;
-        be = oe;
-      }
-    }
-    if ((be & 31) == lane) taken |= 1u << (be >> 5);
-    const float s = 1.f / (1.f + expf(-bv));
-    sum += s;
-    if (lane == k) {
-      my_s = s;
-      my_id = be;
-    }
-  }
+  float mine;
+  int my_id;
+  warp_topk<PER>(v, E, K, lane, &mine, &my_id);
+  const float my_s = 1.f / (1.f + expf(-mine));
+  const float sum = lane_sum_in_order(my_s, K);
   if (lane < K) {
     topk_ids[static_cast<size_t>(t) * K + lane] = my_id;
     topk_w[static_cast<size_t>(t) * K + lane] = (renorm ? my_s / (sum + 1e-20f) : my_s) * scale;
@@ -748,14 +697,18 @@ extern "C" int b200_moe_route(const void* logits, int logits_dtype, int num_toke
   if (rc) return rc;
   if (num_tokens == 0) return 0;
   const int blocks = (num_tokens + kRouteWarps - 1) / kRouteWarps;
-  if (logits_dtype == 1)
-    moe_route_kernel<float><<<blocks, kRouteWarps * 32, 0, as_stream(stream)>>>(
-        static_cast<const float*>(logits), num_tokens, num_experts, top_k, renormalize, num_valid_rows, topk_ids,
-        topk_weights);
-  else
-    moe_route_kernel<__nv_bfloat16><<<blocks, kRouteWarps * 32, 0, as_stream(stream)>>>(
-        static_cast<const __nv_bfloat16*>(logits), num_tokens, num_experts, top_k, renormalize, num_valid_rows,
-        topk_ids, topk_weights);
+#define B200_ROUTE(LT, PER)                                                                                                       \
+  B200_CUDA(launch_overlapped(moe_route_kernel<LT, PER>, dim3(blocks), dim3(kRouteWarps * 32), 0, as_stream(stream),               \
+                              static_cast<const LT*>(logits), num_tokens, num_experts, top_k, renormalize, num_valid_rows, topk_ids, \
+                              topk_weights))
+  if (logits_dtype == 1) {
+    if (num_experts <= 128) B200_ROUTE(float, 4);
+    else B200_ROUTE(float, kRouteMaxPerLane);
+  } else {
+    if (num_experts <= 128) B200_ROUTE(__nv_bfloat16, 4);
+    else B200_ROUTE(__nv_bfloat16, kRouteMaxPerLane);
+  }
+#undef B200_ROUTE
   B200_CUDA(cudaGetLastError());
   return 0;
 }

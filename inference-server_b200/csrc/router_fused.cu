@@ -20,6 +20,10 @@
 //            shared memory: CTA r sums rows ROWS/8 * r ... in rank order.
 //   route  = those rows are routed by a warp each exactly as moe_route_kernel does (selection on
 //            the logits, ties to the lower expert id), on fp32 logits that never leave the chip.
+// What bounds it is a chain of dependent waits, so each step asks for all it needs at once: the rows a warp adds, the fragments of
+// several MMA steps, and the top-k is two warp reductions per round (warp_topk, common.cuh).  128 experts of width 2048, us before and
+// now: 1 row 8.0, 5.0   256: 10.1, 6.9   1024: 14.6, 11.1   2048: 28.6, 21.6.  (A form without clusters, the router matrix streamed
+// through each CTA for 16 rows, took 22.4 at 2048 rows and 18.8 at one.)
 // Everything is deterministic (fixed summation orders, no atomics).
 
 #include <mutex>
@@ -67,8 +71,46 @@ struct RouterFusedParams {
   int T, H, E, K, renorm;
 };
 
+// Top-k of a row by a warp (the arithmetic of moe_route_kernel) from its fp32 logits in shared memory.
+__device__ __forceinline__ void rf_route_row(const RouterFusedParams& p, int row, const float* lg, int lane) {
+  const int E = p.E, K = p.K;
+  if (p.num_valid != nullptr && row >= *p.num_valid) {
+    if (lane < K) {
+      p.topk_ids[static_cast<size_t>(row) * K + lane] = -1;
+      p.topk_w[static_cast<size_t>(row) * K + lane] = 0.f;
+    }
+    return;
+  }
+  constexpr int kPer = kRfMaxExperts / 32;
+  float v[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int e = lane + 32 * j;
+    v[j] = e < E ? lg[e] : -INFINITY;
+  }
+  float mine;
+  int my_id;
+  warp_topk<kPer>(v, E, K, lane, &mine, &my_id);
+  const float mx = __shfl_sync(0xffffffffu, mine, 0);
+  const float my_p = expf(mine - mx);
+  float den = 0.f;
+  if (p.renorm) {
+    den = lane_sum_in_order(my_p, K);
+  } else {
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      if (lane + 32 * j < E) den += expf(v[j] - mx);
+    den = warp_sum(den);
+  }
+  if (lane < K) {
+    p.topk_ids[static_cast<size_t>(row) * K + lane] = my_id;
+    p.topk_w[static_cast<size_t>(row) * K + lane] = my_p / den;
+  }
+}
+
+// (four CTAs of the 16-row form per SM, three of the 32-row form: where shared memory allows so many, registers must not forbid them)
 template <int ROWS>
-__global__ void __launch_bounds__(kRfThreads, 1)
+__global__ void __launch_bounds__(kRfThreads, ROWS == 16 ? 4 : 3)
 add_rmsnorm_route_kernel(const RouterFusedParams p) {
 #ifdef B200_DEVICE_OK
   extern __shared__ __align__(16) uint8_t rf_smem[];
@@ -98,38 +140,54 @@ add_rmsnorm_route_kernel(const RouterFusedParams p) {
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  // The router matrix is a weight; the rows come from the kernels before this one.
+  // (a lane's first piece of the norm weights too)
+  uint4 wfirst = make_uint4(0u, 0u, 0u, 0u);
+  if (lane < cols / 8) wfirst = *reinterpret_cast<const uint4*>(p.norm_w + col0 + lane * 8);
+  // The router matrix and the norm's weights are weights; the rows come from the kernels before this one.
   grid_dep_wait();
   grid_dep_launch();
 
-  // ---- residual add, partial sums of squares: warp w owns rows kOwn * w ...
+  // ---- residual add, partial sums of squares: warp w owns rows kOwn * w ..., whose loads are in flight together
+  float ss[kOwn];
 #pragma unroll
-  for (int rr = 0; rr < kOwn; ++rr) {
-    const int r = kOwn * warp + rr, row = row0 + r;
-    float ss = 0.f;
-    for (int c = lane; c < cols / 8; c += 32) {
-      uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+  for (int rr = 0; rr < kOwn; ++rr) ss[rr] = 0.f;
+  for (int c = lane; c < cols / 8; c += 32) {
+    uint4 xv[kOwn], dv[kOwn];
+#pragma unroll
+    for (int rr = 0; rr < kOwn; ++rr) {
+      const int row = row0 + kOwn * warp + rr;
+      const size_t off = static_cast<size_t>(row) * p.H + col0 + c * 8;
+      xv[rr] = dv[rr] = make_uint4(0u, 0u, 0u, 0u);
       if (row < p.T) {
-        const size_t off = static_cast<size_t>(row) * p.H + col0 + c * 8;
-        raw = *reinterpret_cast<const uint4*>(p.x + off);
+        xv[rr] = *reinterpret_cast<const uint4*>(p.x + off);
+        if (p.delta != nullptr) dv[rr] = *reinterpret_cast<const uint4*>(p.delta + off);
+      }
+    }
+#pragma unroll
+    for (int rr = 0; rr < kOwn; ++rr) {
+      const int r = kOwn * warp + rr, row = row0 + r;
+      uint4 raw = xv[rr];
+      if (row < p.T) {
         __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&raw);
         if (p.delta != nullptr) {
-          const uint4 draw = *reinterpret_cast<const uint4*>(p.delta + off);
-          const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&draw);
+          const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&dv[rr]);
 #pragma unroll
           for (int j = 0; j < 4; ++j) h2[j] = __hadd2(h2[j], d2[j]);  // the residual add happens in bf16, as in the model
-          *reinterpret_cast<uint4*>(p.x + off) = raw;
+          *reinterpret_cast<uint4*>(p.x + static_cast<size_t>(row) * p.H + col0 + c * 8) = raw;
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float2 f = __bfloat1622float2(h2[j]);
-          ss += f.x * f.x + f.y * f.y;
+          ss[rr] += f.x * f.x + f.y * f.y;
         }
       }
       *reinterpret_cast<uint4*>(a_tile + r * pitch + c * 8) = raw;
     }
-    ss = warp_sum(ss);
-    if (lane == 0) ss_part[r] = ss;
+  }
+#pragma unroll
+  for (int rr = 0; rr < kOwn; ++rr) {
+    const float sum = warp_sum(ss[rr]);
+    if (lane == 0) ss_part[kOwn * warp + rr] = sum;
   }
   __syncwarp();
   rf_cluster_sync();  // #1: every slice's partial sums are written
@@ -145,15 +203,15 @@ add_rmsnorm_route_kernel(const RouterFusedParams p) {
   __syncthreads();
 
   // ---- normalise: out = weight * bf16(x * inv); kept in shared memory as the A operand, written out as h
+  for (int c = lane; c < cols / 8; c += 32) {
+    const uint4 wraw = c == lane ? wfirst : *reinterpret_cast<const uint4*>(p.norm_w + col0 + c * 8);
+    const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(&wraw);
 #pragma unroll
-  for (int rr = 0; rr < kOwn; ++rr) {
-    const int r = kOwn * warp + rr, row = row0 + r;
-    const float inv = inv_sm[r];
-    for (int c = lane; c < cols / 8; c += 32) {
+    for (int rr = 0; rr < kOwn; ++rr) {
+      const int r = kOwn * warp + rr, row = row0 + r;
+      const float inv = inv_sm[r];
       uint4 raw = *reinterpret_cast<const uint4*>(a_tile + r * pitch + c * 8);
       const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-      const uint4 wraw = *reinterpret_cast<const uint4*>(p.norm_w + col0 + c * 8);
-      const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(&wraw);
       uint4 o;
       __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
@@ -180,16 +238,24 @@ add_rmsnorm_route_kernel(const RouterFusedParams p) {
     const uint32_t a_addr = smem_u32(a_tile) + static_cast<uint32_t>(((mat & 1) * 8 + lr) * pitch * 2 + (mat >> 1) * 16);
     const uint32_t b_addr =
         smem_u32(w_tile) + static_cast<uint32_t>((warp * 16 + (mat >> 1) * 8 + lr) * pitch * 2 + (mat & 1) * 16);
-    for (int ks = 0; ks < cols / 16; ++ks) {
-      uint32_t b0, b1, b2, b3;
-      ldmatrix_x4(b_addr + ks * 32, b0, b1, b2, b3);
+    // the fragments of kStep steps are in flight together (a slice is a multiple of 64 columns)
+    constexpr int kStep = ROWS == 16 ? 4 : 2;
+    for (int k0 = 0; k0 < cols / 16; k0 += kStep) {
+      uint32_t b[kStep][4], a[kStep][kMt][4];
 #pragma unroll
-      for (int mt = 0; mt < kMt; ++mt) {
-        uint32_t a[4];
-        ldmatrix_x4(a_addr + mt * 16 * pitch * 2 + ks * 32, a[0], a[1], a[2], a[3]);
-        mma_bf16_16816(acc[mt][0], a, b0, b1);
-        mma_bf16_16816(acc[mt][1], a, b2, b3);
+      for (int k = 0; k < kStep; ++k) {
+        ldmatrix_x4(b_addr + (k0 + k) * 32, b[k][0], b[k][1], b[k][2], b[k][3]);
+#pragma unroll
+        for (int mt = 0; mt < kMt; ++mt)
+          ldmatrix_x4(a_addr + mt * 16 * pitch * 2 + (k0 + k) * 32, a[k][mt][0], a[k][mt][1], a[k][mt][2], a[k][mt][3]);
       }
+#pragma unroll
+      for (int k = 0; k < kStep; ++k)
+#pragma unroll
+        for (int mt = 0; mt < kMt; ++mt) {
+          mma_bf16_16816(acc[mt][0], a[k][mt], b[k][0], b[k][1]);
+          mma_bf16_16816(acc[mt][1], a[k][mt], b[k][2], b[k][3]);
+        }
     }
     const int gq = lane >> 2, tq = lane & 3;
 #pragma unroll
@@ -228,68 +294,7 @@ add_rmsnorm_route_kernel(const RouterFusedParams p) {
   // ---- top-k of these rows (the arithmetic of moe_route_kernel)
   if (warp < kOwn) {
     const int row = row0 + kOwn * static_cast<int>(rank) + warp;
-    if (row < p.T) {
-      const int E = p.E, K = p.K;
-      if (p.num_valid != nullptr && row >= *p.num_valid) {
-        if (lane < K) {
-          p.topk_ids[static_cast<size_t>(row) * K + lane] = -1;
-          p.topk_w[static_cast<size_t>(row) * K + lane] = 0.f;
-        }
-      } else {
-        constexpr int kPer = kRfMaxExperts / 32;
-        const float* lg = lg_fin + warp * E;
-        float v[kPer];
-        float mx = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-          const int e = lane + 32 * j;
-          v[j] = e < E ? lg[e] : -INFINITY;
-          mx = fmaxf(mx, v[j]);
-        }
-        mx = warp_max(mx);
-        float den = 0.f;
-#pragma unroll
-        for (int j = 0; j < kPer; ++j)
-          if (lane + 32 * j < E) den += expf(v[j] - mx);
-        den = warp_sum(den);
-        unsigned taken = 0;
-        float sel_sum = 0.f, my_p = 0.f;
-        int my_id = 0;
-        for (int k = 0; k < K; ++k) {
-          float bv = -INFINITY;
-          int be = 0x7fffffff;
-#pragma unroll
-          for (int j = 0; j < kPer; ++j) {
-            const int e = lane + 32 * j;
-            if (e < E && !((taken >> j) & 1u) && (be == 0x7fffffff || v[j] > bv)) {
-              bv = v[j];
-              be = e;
-            }
-          }
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oe = __shfl_xor_sync(0xffffffffu, be, o);
-            const bool better = oe != 0x7fffffff && (be == 0x7fffffff || ov > bv || (ov == bv && oe < be));
-            if (better) {
-              bv = ov;
-              be = oe;
-            }
-          }
-          if ((be & 31) == lane) taken |= 1u << (be >> 5);
-          const float pr = expf(bv - mx);
-          sel_sum += pr;
-          if (lane == k) {
-            my_p = pr;
-            my_id = be;
-          }
-        }
-        if (lane < K) {
-          p.topk_ids[static_cast<size_t>(row) * K + lane] = my_id;
-          p.topk_w[static_cast<size_t>(row) * K + lane] = my_p / (p.renorm ? sel_sum : den);
-        }
-      }
-    }
+    if (row < p.T) rf_route_row(p, row, lg_fin + warp * p.E, lane);
   }
   __syncwarp();
   rf_cluster_sync();  // #3: nobody leaves while a peer may still read its shared memory
@@ -367,11 +372,11 @@ static int resident_route_clusters(int H, int E, int* out) {
 }
 
 // Rows per cluster: 16, or 32 where that leaves at most three waves of clusters in place of four.  A wave of 32-row clusters takes
-// 1.15-1.3 times one of 16-row clusters (128 experts: width 512 14.2 and 12.1 us, 2048 14.6 and 11.4, 4096 13.9 and 10.6), and how many of either
+// 1.0-1.15 times one of 16-row clusters (128 experts: width 512 10.2 and 9.2 us, 2048 9.5 and 8.8), and how many of either
 // the GPU holds depends on their shared memory, so on width and experts.  us with 16 and with 32, 128 experts:
-//   width 2048   513 rows 11.4, 13.2   576: 19.4, 13.6   1024: 22.3, 14.6   2048: 43.7, 28.6
-//   width  512  1024 rows 12.1, 14.2  1500: 21.0, 14.7   2048: 22.9, 25.3   4096: 43.5, 40.6
-//   width 4096   128 rows 10.6, 13.6   256: 20.6, 13.9    512: 31.6, 27.0   1024: 54.2, 41.6
+//   width 2048   513 rows 8.8, 9.8   576: 12.9, 10.1   1024: 16.8, 11.3   2048: 32.1, 21.7
+//   width  512  1024 rows 9.2, 10.2  1500: 14.9, 10.9   2048: 17.1, 17.7   4096: 31.5, 28.3
+//   width 4096   256 rows 14.7, 9.5   512: 22.8, 18.6   1024: 39.6, 29.0
 static int route_rows(int T, int H, int E, int* out) {
   *out = 16;
   const int c16 = (T + 15) / 16, c32 = (T + 31) / 32;

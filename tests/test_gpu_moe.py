@@ -298,3 +298,36 @@ def test_down_product_with_a_row_map_and_many_rows_per_expert(ops, T):
     want, got = ops.moe_fp8_gemm_down(hq, hs, w2, s2, p), torch.zeros(T * K, H, dtype=torch.bfloat16, device=DEV)
     ops.moe_fp8_gemm_down(hq, hs, w2, s2, p, out=got, out_row_map=to)
     assert torch.equal(got[to.long()], want) and bool(want.any())
+
+
+@pytest.mark.parametrize("E,K", [(16, 16), (33, 8), (128, 8), (129, 1), (200, 32), (256, 8)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_top_k_of_ties_infinities_and_zeros(ops, E, K, dtype):
+    """Few distinct values, both zeros and both infinities among them: largest first, equal ones by lower id, in both routers."""
+    g = torch.Generator().manual_seed(E + K)
+    values = torch.tensor([0.0, -0.0, 1.5, -1.5, 3e-39, -3e-39, float("-inf"), 60.0])
+    logits = values[torch.randint(0, len(values), (41, E), generator=g)]
+    logits[0] = float("-inf")
+    logits[1] = -0.0
+    logits[2, E // 2] = float("inf")
+    logits = logits.to(dtype)
+    want = torch.argsort(logits.float(), dim=1, descending=True, stable=True)[:, :K].to(torch.int32)
+    ids, w = ops.moe_route(logits.to(DEV), K, True)
+    assert torch.equal(ids.cpu(), want)
+    finite = torch.isfinite(logits.float().max(dim=1).values)
+    p = torch.softmax(logits.double(), -1).gather(1, want.long())
+    p = p / p.sum(-1, keepdim=True)
+    torch.testing.assert_close(w.cpu().double()[finite], p[finite], rtol=3e-6, atol=1e-9)
+    ids, w = ops.moe_route_sigmoid(logits.to(DEV), K, 1.0)
+    assert torch.equal(ids.cpu(), want)
+
+
+def test_top_k_of_rows_with_a_nan_names_different_existing_experts(ops):
+    logits = torch.randn(64, 128, generator=torch.Generator().manual_seed(3))
+    logits[torch.arange(64), torch.arange(64) * 2] = float("nan")
+    logits[7] = float("nan")
+    for ids, _ in (ops.moe_route(logits.to(DEV), 8, True), ops.moe_route_sigmoid(logits.to(DEV), 8, 1.0)):
+        ids = ids.cpu()
+        assert int(ids.min()) >= 0 and int(ids.max()) < 128
+        assert all(len(set(r.tolist())) == 8 for r in ids)
+        assert not bool((ids[:7] == torch.arange(7)[:, None] * 2).any())  # a NaN comes after every number
