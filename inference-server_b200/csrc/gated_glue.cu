@@ -48,7 +48,7 @@ residual_norm_kernel(float* __restrict__ x, const Pending<T> p, const float* __r
   for (int j = 0; j < 8; ++j) f[j] = w[j] = 0.f;
   if (in) {
     load8<float>(x + at, f);
-    load8<float>(weight + col, w);
+    if (MAXT <= 512) load8<float>(weight + col, w);
     const bool any = p.dense != nullptr || p.expert_rows != nullptr;
     if (any) {
       Raw8<T> g;
@@ -60,25 +60,30 @@ residual_norm_kernel(float* __restrict__ x, const Pending<T> p, const float* __r
         load8<T>(p.dense + at, d);
       } else {
         for (int k0 = 0; k0 < p.top_k; k0 += 8) {  // eight pairs at a time: their rows are in flight together
-          int rows[8];
-          float pw[8];
+          const int n = min(8, p.top_k - k0);
+          const int* rows = p.row_of_pair + static_cast<size_t>(m) * p.top_k + k0;
+          const float* pw = p.pair_weight + static_cast<size_t>(m) * p.top_k + k0;
           Raw8<T> raw[8];
+          unsigned have = 0u;
+          {
+            int row[8];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const bool have = k0 + u < p.top_k;
-            rows[u] = have ? p.row_of_pair[static_cast<size_t>(m) * p.top_k + k0 + u] : -1;
-            pw[u] = have ? p.pair_weight[static_cast<size_t>(m) * p.top_k + k0 + u] : 0.f;
+            for (int u = 0; u < 8; ++u) row[u] = u < n ? __ldg(rows + u) : -1;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (row[u] >= 0) {
+                have |= 1u << u;
+                raw[u].load(p.expert_rows + static_cast<size_t>(row[u]) * ld + col);
+              }
           }
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (rows[u] >= 0) raw[u].load(p.expert_rows + static_cast<size_t>(rows[u]) * ld + col);
-#pragma unroll
           for (int u = 0; u < 8; ++u) {
-            if (rows[u] < 0) continue;
+            if (!((have >> u) & 1u)) continue;
+            const float weight_of = __ldg(pw + u);
             float y[8];
             raw[u].get(y);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) d[j] = fmaf(pw[u], y[j], d[j]);
+            for (int j = 0; j < 8; ++j) d[j] = fmaf(weight_of, y[j], d[j]);
           }
         }
       }
@@ -98,6 +103,7 @@ residual_norm_kernel(float* __restrict__ x, const Pending<T> p, const float* __r
       for (int j = 0; j < 8; ++j) f[j] = col + j < width ? f[j] + d[j] : 0.f;
       store8<float>(x + at, f);
     }
+    if (MAXT > 512) load8<float>(weight + col, w);
   }
   const int warps = blockDim.x >> 5;
   float mean = 0.f;
@@ -364,10 +370,15 @@ static int launch_residual_norm(float* x, const void* dense, const void* expert_
   const Pending<T> p{static_cast<const T*>(dense), static_cast<const T*>(expert_rows), row_of_pair, pair_weight, top_k, bias,
                      static_cast<const T*>(gate)};
   const int threads = (ld / 8 + 31) / 32 * 32;
+  int sms = 0;
+  const int rc = device_sm_count(&sms);
+  if (rc) return rc;
 #define B200_RNORM(CENTER, MAXT)                                                                                     \
   B200_CUDA(launch_overlapped(residual_norm_kernel<T, CENTER, MAXT>, dim3(rows), dim3(threads), 0, st, x, p, weight, eps, \
                               width, ld, static_cast<T*>(out)))
-  if (threads <= 512) {
+  // More rows than two CTAs per SM take at once: the form with at most 64 registers, of which four fit (rows of width 2048 with eight
+  // experts' rows each, us: 512 rows 6.3, 5.7   1777: 20.2, 15.5   4096: 53.1, 41.1; without a sublayer 17.7, 12.5).
+  if (threads <= 512 && (sizeof(T) == 4 || rows <= 2 * sms)) {
     if (center) B200_RNORM(true, 512);
     else B200_RNORM(false, 512);
   } else {

@@ -456,10 +456,15 @@ static int launch_group_rmsnorm(float* x, const void* delta, const void* weight,
   const int threads = (ld / 8 + 31) / 32 * 32;
   const bool wide = (width / groups) % 256 == 0;
   const size_t smem = wide ? 32 * 4 : static_cast<size_t>(ld + groups) * 4;
+  int sms = 0;
+  const int rc = device_sm_count(&sms);
+  if (rc) return rc;
 #define B200_NORM_ARGS                                                                                              \
   x, static_cast<const T*>(delta), static_cast<const T*>(weight), eps, width, ld, groups, static_cast<T*>(out),      \
       static_cast<const T*>(conv_w), taps, static_cast<T*>(hist), positions, block_table, pm
-  if (threads <= 512) {
+  // More rows than three CTAs per SM take at once: the form with at most 64 registers, of which four fit (width 2048, us: 512 rows 4.2,
+  // 3.3   1024: 5.9, 5.1   2048: 9.3, 8.6   4096: 16.6, 14.7).
+  if (threads <= 512 && (sizeof(T) == 4 || rows <= 3 * sms)) {
     if (wide)
       B200_CUDA(launch_overlapped(group_rmsnorm_kernel<T, true, 512>, dim3(rows), dim3(threads), smem, st, B200_NORM_ARGS));
     else

@@ -102,10 +102,12 @@ moe_route_sigmoid_kernel(const LT* __restrict__ logits, int T, int E, int K, int
 }
 
 // ---------------------------------------------------------------- permute ---
-constexpr int kRankThreads = 256;
+constexpr int kRankThreads = 256, kRankManyThreads = 1024;
+constexpr int kRankMany = 8192;  // pairs
 
 // moe_rank_kernel for more than 16 pairs per thread: a thread's `chunk` ids (a multiple of 4) are read in 16-byte pieces, eight of
 // them in flight, once to count and once to place.
+template <int THREADS>
 __device__ __forceinline__ void rank_long(const int* __restrict__ ids, int n_pairs, int chunk, int e, int* __restrict__ rank,
                                           int* __restrict__ counts, int* warp_tot) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -141,7 +143,7 @@ __device__ __forceinline__ void rank_long(const int* __restrict__ ids, int n_pai
   __syncthreads();
   int before = 0, total = 0;
 #pragma unroll
-  for (int w = 0; w < kRankThreads / 32; ++w) {
+  for (int w = 0; w < THREADS / 32; ++w) {
     const int t = warp_tot[w];
     if (w < warp) before += t;
     total += t;
@@ -158,16 +160,17 @@ __device__ __forceinline__ void rank_long(const int* __restrict__ ids, int n_pai
 }
 
 // One CTA per expert: stable rank of every pair routed to this expert.
-__global__ void __launch_bounds__(kRankThreads)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : 8)
 moe_rank_kernel(const int* __restrict__ topk_ids, int n_pairs, int* __restrict__ rank,
                 int* __restrict__ counts) {
-  __shared__ int warp_tot[kRankThreads / 32];
+  __shared__ int warp_tot[THREADS / 32];
   grid_dep_wait();
   grid_dep_launch();
   const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int chunk = (n_pairs + kRankThreads - 1) / kRankThreads;
-  if (chunk > 16) {  // many pairs: whole 16-byte pieces per thread
-    rank_long(topk_ids, n_pairs, (chunk + 3) & ~3, e, rank, counts, warp_tot);
+  const int chunk = (n_pairs + THREADS - 1) / THREADS;
+  if (chunk > (THREADS > 256 ? 4 : 16)) {  // many pairs: whole 16-byte pieces per thread
+    rank_long<THREADS>(topk_ids, n_pairs, (chunk + 3) & ~3, e, rank, counts, warp_tot);
     return;
   }
   const int lo = min(n_pairs, tid * chunk), hi = min(n_pairs, lo + chunk);
@@ -191,7 +194,7 @@ moe_rank_kernel(const int* __restrict__ topk_ids, int n_pairs, int* __restrict__
   __syncthreads();
   int before = 0, total = 0;
 #pragma unroll
-  for (int w = 0; w < kRankThreads / 32; ++w) {
+  for (int w = 0; w < THREADS / 32; ++w) {
     const int t = warp_tot[w];
     if (w < warp) before += t;
     total += t;
@@ -201,6 +204,16 @@ moe_rank_kernel(const int* __restrict__ topk_ids, int n_pairs, int* __restrict__
   for (int u = 0; u < kHold; ++u)
     if (held[u] == e) rank[lo + u] = run++;
   if (tid == 0) counts[e] = total;
+}
+
+// A CTA reads all pairs' experts, so with many pairs its time is a thread's chain of loads and compares: 1024 threads then (us of the rank
+// and scatter kernels with 256 and 1024 threads: 4096 pairs 10.6, 11.6   16384: 20.4, 19.7   32768: 43.9, 34.3).
+static int launch_rank(const int* ids, int n_pairs, int num_experts, int* rank, int* counts, cudaStream_t st) {
+  if (n_pairs > kRankMany)
+    B200_CUDA(launch_overlapped(moe_rank_kernel<kRankManyThreads>, dim3(num_experts), dim3(kRankManyThreads), 0, st, ids, n_pairs, rank, counts));
+  else
+    B200_CUDA(launch_overlapped(moe_rank_kernel<kRankThreads>, dim3(num_experts), dim3(kRankThreads), 0, st, ids, n_pairs, rank, counts));
+  return 0;
 }
 
 constexpr int kScatterThreads = 256;
@@ -584,6 +597,8 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y,
                                    const int* __restrict__ row_of_pair,
                                    const float* __restrict__ topk_w, int H, int K,
                                    __nv_bfloat16* __restrict__ out) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int t = blockIdx.x, tid = threadIdx.x;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int k = 0; k < K; ++k) {
@@ -652,6 +667,75 @@ __global__ void moe_combine_add_rmsnorm_kernel(const __nv_bfloat16* __restrict__
       }
     }
   }
+  __nv_bfloat162* x2 = reinterpret_cast<__nv_bfloat162*>(&xr);
+  float f[8], ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    x2[j] = __hadd2(x2[j], __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]));
+    const float2 p = __bfloat1622float2(x2[j]);
+    f[2 * j] = p.x;
+    f[2 * j + 1] = p.y;
+    ss += p.x * p.x + p.y * p.y;
+  }
+  *reinterpret_cast<uint4*>(x + base) = xr;
+  ss = warp_sum(ss);
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  __syncthreads();
+  float tot = (tid & 31) < (blockDim.x + 31) / 32 ? red[tid & 31] : 0.f;
+  tot = warp_sum(tot);
+  const float inv = rsqrtf(tot / static_cast<float>(H) + eps);
+  const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(&wraw);
+  uint4 o;
+  __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    o2[j] = __hmul2(w2[j], __floats2bfloat162_rn(f[2 * j] * inv, f[2 * j + 1] * inv));
+  *reinterpret_cast<uint4*>(out + base) = o;
+}
+
+// The same for many tokens: at most 64 registers, so that four CTAs of 256 threads fit on an SM where two of the form above do; the loads
+// that are not asked for up front then are those of the weights.  us, width 2048, 8 rows each, that form and this one: 37 tokens 2.4,
+// 2.5   512: 4.7, 4.1   2048: 15.6, 11.5   4096: 41.1, 34.
+__global__ void __maxnreg__(64)
+moe_combine_add_rmsnorm_many_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_pair,
+                                    const float* __restrict__ topk_w, int H, int K, __nv_bfloat16* __restrict__ x,
+                                    const __nv_bfloat16* __restrict__ weight, float eps, __nv_bfloat16* __restrict__ out) {
+  __shared__ float red[32];
+  grid_dep_wait();
+  grid_dep_launch();
+  const int t = blockIdx.x, tid = threadIdx.x;
+  const size_t base = static_cast<size_t>(t) * H + tid * 8;
+  uint4 xr = *reinterpret_cast<const uint4*>(x + base);
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int k0 = 0; k0 < K; k0 += 8) {
+    const int* rows = row_of_pair + static_cast<size_t>(t) * K + k0;
+    uint4 raws[8];
+    unsigned have = 0u;
+    {
+      int row[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) row[u] = k0 + u < K ? __ldg(rows + u) : -1;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (row[u] >= 0) {
+          have |= 1u << u;
+          raws[u] = *reinterpret_cast<const uint4*>(y + static_cast<size_t>(row[u]) * H + tid * 8);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (!((have >> u) & 1u)) continue;
+      const float w = __ldg(topk_w + static_cast<size_t>(t) * K + k0 + u);
+      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raws[u]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 p = __bfloat1622float2(h2[j]);
+        acc[2 * j] += w * p.x;
+        acc[2 * j + 1] += w * p.y;
+      }
+    }
+  }
+  const uint4 wraw = *reinterpret_cast<const uint4*>(weight + tid * 8);
   __nv_bfloat162* x2 = reinterpret_cast<__nv_bfloat162*>(&xr);
   float f[8], ss = 0.f;
 #pragma unroll
@@ -753,8 +837,8 @@ extern "C" int b200_moe_permute(const int32_t* topk_ids, int num_tokens, int num
   int* counts = reinterpret_cast<int*>(p + 256);
   int* rank = reinterpret_cast<int*>(p + 256 + ((static_cast<size_t>(num_experts) * 4 + 255) & ~size_t(255)));
   const int n_pairs = num_tokens * top_k;
-  moe_rank_kernel<<<num_experts, kRankThreads, 0, st>>>(topk_ids, n_pairs, rank, counts);
-  B200_CUDA(cudaGetLastError());
+  rc = launch_rank(topk_ids, n_pairs, num_experts, rank, counts, st);
+  if (rc) return rc;
   const int blocks = n_pairs > 0 ? (n_pairs + kScatterThreads - 1) / kScatterThreads : 1;
   moe_scatter_kernel<<<blocks, kScatterThreads, (2 * num_experts + 1) * sizeof(int), st>>>(
       topk_ids, rank, counts, n_pairs, num_experts, tile_experts, 128, sorted_pair_ids, row_of_pair,
@@ -796,8 +880,8 @@ static int permute_quant_impl(const int32_t* topk_ids, const void* x, int num_to
   int* err = reinterpret_cast<int*>(p);
   int* counts = reinterpret_cast<int*>(p + 256);
   int* rank = reinterpret_cast<int*>(p + 256 + ((static_cast<size_t>(num_experts) * 4 + 255) & ~size_t(255)));
-  B200_CUDA(launch_overlapped(moe_rank_kernel, dim3(num_experts), dim3(kRankThreads), 0, st, topk_ids,
-                              num_tokens * top_k, rank, counts));
+  rc = launch_rank(topk_ids, num_tokens * top_k, num_experts, rank, counts, st);
+  if (rc) return rc;
   const size_t smem = (4 * static_cast<size_t>(num_experts) + 2 + 32 + top_k) * sizeof(int);
   B200_CUDA(launch_overlapped(moe_scatter_quant_kernel, dim3(num_tokens), dim3(hidden / 8), smem, st,
                               static_cast<const __nv_bfloat16*>(x), topk_ids, rank, counts, num_experts, top_k, hidden,
@@ -858,8 +942,8 @@ extern "C" int b200_moe_permute_copy(const int32_t* topk_ids, const void* x, int
   uint8_t* p = static_cast<uint8_t*>(workspace);
   int* counts = reinterpret_cast<int*>(p + 256);
   int* rank = reinterpret_cast<int*>(p + 256 + ((static_cast<size_t>(num_experts) * 4 + 255) & ~size_t(255)));
-  B200_CUDA(launch_overlapped(moe_rank_kernel, dim3(num_experts), dim3(kRankThreads), 0, st, topk_ids, num_tokens * top_k, rank,
-                              counts));
+  rc = launch_rank(topk_ids, num_tokens * top_k, num_experts, rank, counts, st);
+  if (rc) return rc;
   const int vec = row_bytes / 16;
   const int threads = vec >= 256 ? 256 : (vec + 31) / 32 * 32;
   const size_t smem = (4 * static_cast<size_t>(num_experts) + 2 + 32 + top_k) * sizeof(int);
@@ -964,10 +1048,20 @@ extern "C" int b200_moe_combine_add_rmsnorm(const void* y_sorted, const int32_t*
   int rc = check_device(nullptr);
   if (rc) return rc;
   if (num_tokens == 0) return 0;
-  B200_CUDA(launch_overlapped(moe_combine_add_rmsnorm_kernel, dim3(num_tokens), dim3(hidden / 8), 0, as_stream(stream),
+  int sms = 0;
+  rc = device_sm_count(&sms);
+  if (rc) return rc;
+  if (num_tokens > 2 * sms || hidden > 4096) {
+    B200_CUDA(launch_overlapped(moe_combine_add_rmsnorm_many_kernel, dim3(num_tokens), dim3(hidden / 8), 0, as_stream(stream),
                               static_cast<const __nv_bfloat16*>(y_sorted), row_of_pair, topk_weights, hidden, top_k,
                               static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(weight), eps,
                               static_cast<__nv_bfloat16*>(out)));
+  } else {
+    B200_CUDA(launch_overlapped(moe_combine_add_rmsnorm_kernel, dim3(num_tokens), dim3(hidden / 8), 0, as_stream(stream),
+                              static_cast<const __nv_bfloat16*>(y_sorted), row_of_pair, topk_weights, hidden, top_k,
+                              static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(weight), eps,
+                              static_cast<__nv_bfloat16*>(out)));
+  }
   return 0;
 }
 
@@ -1000,6 +1094,17 @@ extern "C" int b200_moe_combine(const void* y_sorted, const int32_t* row_of_pair
   int rc = check_device(nullptr);
   if (rc) return rc;
   if (num_tokens == 0) return 0;
+  int sms = 0;
+  rc = device_sm_count(&sms);
+  if (rc) return rc;
+  // Few tokens: the launch overlaps the end of the kernel before (64 tokens 3.3 -> 3.0 us); with many, CTAs that arrive early only take room
+  // (1024 tokens of width 4096 8.7 us, 9.6 overlapped).
+  if (num_tokens <= 2 * sms) {
+    B200_CUDA(launch_overlapped(moe_combine_kernel, dim3(num_tokens), dim3(hidden / 8), 0, as_stream(stream),
+                                static_cast<const __nv_bfloat16*>(y_sorted), row_of_pair, topk_weights, hidden, top_k,
+                                static_cast<__nv_bfloat16*>(out)));
+    return 0;
+  }
   moe_combine_kernel<<<num_tokens, hidden / 8, 0, as_stream(stream)>>>(
       static_cast<const __nv_bfloat16*>(y_sorted), row_of_pair, topk_weights, hidden, top_k,
       static_cast<__nv_bfloat16*>(out));
@@ -1040,8 +1145,8 @@ extern "C" int b200_moe_permute_gather_fp8(const int32_t* ids, int num_rows, int
   int* err = reinterpret_cast<int*>(p);
   int* counts = reinterpret_cast<int*>(p + 256);
   int* rank = reinterpret_cast<int*>(p + 256 + ((static_cast<size_t>(num_experts) * 4 + 255) & ~size_t(255)));
-  moe_rank_kernel<<<num_experts, kRankThreads, 0, st>>>(ids, num_rows, rank, counts);
-  B200_CUDA(cudaGetLastError());
+  rc = launch_rank(ids, num_rows, num_experts, rank, counts, st);
+  if (rc) return rc;
   const int threads = hidden / 16 < 256 ? (hidden / 16 < 32 ? 32 : hidden / 16) : 256;
   const size_t smem = (2 * static_cast<size_t>(num_experts) + 1) * sizeof(int);
   moe_scatter_rows_kernel<<<num_rows, threads, smem, st>>>(

@@ -429,3 +429,29 @@ def test_projection_with_biases_and_activations(ops, dtype):
     pages = torch.stack([pool.cpu()[int(table[0, t // 16]), :, t % 16].reshape(-1) for t in range(M)])
     for got, want in ((q, y[:, :64]), (pages, y[:, 64:128]), (a, ref.silu(y[:, 128:176])), (g, torch.sigmoid(y[:, 176:272])), (f, y[:, 272:])):
         assert rel_err(got, want) < TOL[dtype]
+
+
+@pytest.mark.parametrize("width,ld,center", [(2048, 2048, True), (204, 256, False), (4000, 4096, True)])
+def test_norms_of_many_rows_give_the_bits_of_few(ops, width, ld, center):
+    """More rows than fit the SMs at once go to forms with fewer registers: the same rows a few at a time, the same bits."""
+    P = pkg("gated").Pending
+    M, top = 3 * torch.cuda.get_device_properties(0).multi_processor_count + 5, 9
+    cut = (torch.arange(ld) < width).to(DEV)
+    x, w = randn(M, ld, seed=1).to(DEV) * cut, (1 + randn(ld, seed=2)).to(DEV) * cut
+    d, g, e = (randn(M, ld, seed=s, dtype=BF).to(DEV) * cut for s in (3, 4, 5))
+    bias, pairs = randn(ld, seed=6).to(DEV) * cut, torch.randint(-1, M, (M, top), generator=torch.Generator().manual_seed(7)).to(torch.int32).to(DEV)
+    pw = torch.rand(M, top, generator=torch.Generator().manual_seed(8)).to(DEV)
+
+    def check(f):
+        def of(lo, hi):
+            xs = x[lo:hi].clone()
+            return f(xs, lo, hi), xs
+        whole, parts = of(0, M), [of(lo, min(M, lo + 100)) for lo in range(0, M, 100)]
+        for i in range(2):
+            assert torch.equal(whole[i], torch.cat([p[i] for p in parts]))
+
+    check(lambda xs, lo, hi: ops.residual_norm(xs, P(dense=d[lo:hi], gate=g[lo:hi], bias=bias), w, 1e-3, width, center))
+    check(lambda xs, lo, hi: ops.residual_norm(xs, P(expert_rows=e, row_of_pair=pairs[lo:hi].contiguous(), pair_weight=pw[lo:hi].contiguous(),
+                                                     gate=g[lo:hi]), w, 1e-3, width, center))
+    check(lambda xs, lo, hi: ops.residual_norm(xs, None, w, 1e-3, width, center))
+    check(lambda xs, lo, hi: ops.group_rmsnorm(xs, d[lo:hi], w.to(BF), 1e-3, width, 4))

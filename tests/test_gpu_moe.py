@@ -331,3 +331,42 @@ def test_top_k_of_rows_with_a_nan_names_different_existing_experts(ops):
         assert int(ids.min()) >= 0 and int(ids.max()) < 128
         assert all(len(set(r.tolist())) == 8 for r in ids)
         assert not bool((ids[:7] == torch.arange(7)[:, None] * 2).any())  # a NaN comes after every number
+
+
+@pytest.mark.parametrize("T,H,K", [(300, 2048, 8), (331, 256, 1), (299, 4096, 9), (3, 4352, 8)])
+def test_combine_of_many_tokens_gives_the_bits_of_few(ops, T, H, K):
+    """The form for many tokens (and for widths beyond 4096) against the plain combine and a torch norm; rows that are dropped (-1)
+    add nothing."""
+    g = torch.Generator().manual_seed(T + H + K)
+    y = torch.randn(T * K, H, generator=g).bfloat16().to(DEV)
+    rows = torch.randperm(T * K, generator=g).view(T, K).to(torch.int32)
+    rows[torch.rand(T, K, generator=g) < 0.1] = -1
+    rows, w = rows.to(DEV), torch.rand(T, K, generator=g).to(DEV)
+    x0 = torch.randn(T, H, generator=g).bfloat16().to(DEV)
+    nw = (1 + 0.1 * torch.randn(H, generator=g)).bfloat16().to(DEV)
+    x = x0.clone()
+    out = ops.moe_combine_add_rmsnorm(y, rows, w, x, nw, 1e-6)
+    want = (x0 + ops.moe_combine(y, rows, w))  # both sums in pair order, fp32, rounded once
+    assert torch.equal(x, want)
+    f = want.float()
+    ref = nw.float() * (f * torch.rsqrt((f * f).mean(-1, keepdim=True) + 1e-6)).bfloat16().float()
+    assert rel_err(out, ref) < 8e-3  # two bf16 roundings
+    if H <= 4096:
+        xs = x0.clone()
+        few = torch.cat([ops.moe_combine_add_rmsnorm(y, rows[i:i + 64].contiguous(), w[i:i + 64].contiguous(), xs[i:i + 64], nw, 1e-6)
+                         for i in range(0, T, 64)])
+        assert torch.equal(out, few) and torch.equal(x, xs)
+
+
+@pytest.mark.parametrize("T,E,K", [(1024, 128, 8), (1025, 128, 8), (4099, 16, 5), (700, 200, 32)])
+def test_ranks_of_many_pairs(ops, T, E, K):
+    """More pairs than the 256-thread rank kernel takes: pairs of an expert in their order, experts one after the other."""
+    g = torch.Generator().manual_seed(T)
+    ids = torch.stack([torch.randperm(E, generator=g)[:K] for _ in range(T)]).to(torch.int32)
+    ids[5, 0] = -1
+    p = ops.moe_permute(ids.to(DEV), E)
+    flat = ids.flatten()
+    order = torch.argsort(torch.where(flat < 0, E, flat), stable=True)[: int((flat >= 0).sum())]
+    want = torch.full((T * K,), -1, dtype=torch.int32)
+    want[order] = torch.arange(len(order), dtype=torch.int32)
+    assert torch.equal(p.row_of_pair.cpu().flatten(), want)
