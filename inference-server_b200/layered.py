@@ -34,7 +34,7 @@ from dataclasses import dataclass
 import torch
 
 from . import gated, ops
-from .engine import PAGE, PagedEngine
+from .engine import PAGE, PagedEngine, token_tensor
 
 GLU_ALPHA = 1.702          # of the design's gated unit
 SINUSOID_BASE = 10000.0
@@ -571,7 +571,7 @@ class LayeredEngine(gated.GatedMechanisms, PagedEngine):
 
     def _prompt_hidden(self, token_ids: list[int], row: torch.Tensor, lo: int, chunk: int, slot: int) -> torch.Tensor:
         n = len(token_ids)
-        tokens = torch.tensor(token_ids, device=self.device)
+        tokens = token_tensor(token_ids, self.device)
         pos = torch.arange(lo, lo + n, device=self.device, dtype=torch.int32)
         return self._forward(tokens, pos, row.unsqueeze(0).expand(n, -1).contiguous(), (lo, n), slots=self._slots_of(slot, n))
 

@@ -142,3 +142,14 @@ def test_a_mixed_pass_leaves_the_logits_of_its_decode_rows(want_first):
     assert tokens.tolist() == [2, 3, 4] and e.ctx_lens.tolist() == [1, 1, 1]
     assert torch.equal(e.last_logits, rows[n:].expand(-1, 4))
     assert first == (1 if want_first else None) and (logits.tolist() == [1.0] * 4 if want_first else logits is None)
+
+
+def test_token_ids_of_any_kind_give_what_torch_makes_of_them():
+    import numpy as np
+    f = pkg("engine").token_tensor
+    ids = [3, 0, 151935, 7]
+    for given in (ids, tuple(ids), [np.int64(v) for v in ids], [np.int32(v) for v in ids], np.array(ids, dtype=np.int32), torch.tensor(ids)):
+        got = f(given, "cpu")
+        assert got.tolist() == ids and not got.is_floating_point()
+    assert f([2 ** 40], "cpu").tolist() == [2 ** 40] and f([], "cpu").numel() == 0
+    assert f([1.5], "cpu").is_floating_point()  # and what is no token id stays what it was
