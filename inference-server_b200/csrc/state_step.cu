@@ -55,10 +55,15 @@ __device__ __forceinline__ float cta_sum(float v, float* red) {
   return s;
 }
 
-template <typename T, int RPT, bool DELTA>
-__global__ void __launch_bounds__(kStepThreads)
+// HELD: the state waits in shared memory (a thread's own pieces, fetched by cp.async) and not in registers.  64 KB of state per CTA take 64
+// registers a thread, which with all else leaves room for two CTAs on an SM; three fit this way, and what a CTA does beside
+// moving its state (window, norms, sums) is hidden better.  us in registers and held, 16 heads of 128 x 128: delta rule 37 rows 15.8, 14.3
+// 256: 112, 85 (its bytes: 83); lightning 256 rows 82, 79.  With no more CTAs than two per SM, and for states of other sizes than 9 to 16
+// rows per thread, registers (100 x 120, 64 rows of 4 heads: 7.2, 9.1; 128 x 64 has room for its CTAs as it is).
+template <typename T, int RPT, bool DELTA, bool HELD>
+__global__ void __launch_bounds__(kStepThreads, HELD ? 3 : 0)
 state_step_kernel(const StepParams p) {
-  extern __shared__ float st_sm[];  // k[dim], q[dim], v[vdim], part[2][row groups][vdim], u[vdim]
+  extern __shared__ __align__(16) float st_sm[];  // k[dim], q[dim], v[vdim], part[2][row groups][vdim], u[vdim]
   __shared__ float red[kStepThreads / 32], sums[kStepThreads / 32][3];
   grid_dep_wait();
   grid_dep_launch();
@@ -79,6 +84,7 @@ state_step_kernel(const StepParams p) {
   float* vs = qs + p.dim;
   float* part = vs + p.vdim;
   float* us = part + 2 * rgs * p.vdim;
+  float4* held = reinterpret_cast<float4*>(us + p.vdim) + tid;  // HELD: piece i of this thread at held[i * kStepThreads]
   const int per = p.heads / p.qk_heads, qh = h / per;
   const T* act = static_cast<const T*>(p.act) + static_cast<size_t>(row) * p.ld;
   // q, k, v of this head, one value per thread and turn
@@ -124,10 +130,17 @@ state_step_kernel(const StepParams p) {
     norm_w = p.norm[tid];
     gate_v = to_f32<T>(static_cast<const T*>(p.gate)[(static_cast<size_t>(row) * p.heads + h) * p.vdim + tid]);
   }
-  float4 S[RPT];
+  float4 S[HELD ? 1 : RPT];
 #pragma unroll
   for (int i = 0; i < RPT; ++i) {
     const int r = rg + i * rgs;
+    if (HELD) {  // nothing is read, and zeros written, where there is no state
+      const bool have = in && pos > 0 && r < p.dim;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(held + i * kStepThreads)),
+                   "l"(have ? src + static_cast<size_t>(r) * p.vdim : p.state), "r"(have ? 16 : 0)
+                   : "memory");
+      continue;
+    }
     S[i] = in && pos > 0 && r < p.dim ? __ldcs(reinterpret_cast<const float4*>(src + static_cast<size_t>(r) * p.vdim))
                                       : make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -192,6 +205,7 @@ state_step_kernel(const StepParams p) {
   } else {
     g = p.decay[h];
   }
+  if (HELD) asm volatile("cp.async.wait_all;" ::: "memory");  // a thread reads its own pieces only
   if (in) {
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
 #pragma unroll
@@ -199,16 +213,17 @@ state_step_kernel(const StepParams p) {
       const int r = rg + i * rgs;
       if (r >= p.dim) break;
       const float kv = ks[r], qv = qs[r];
+      const float4 s = HELD ? held[i * kStepThreads] : S[HELD ? 0 : i];
       if (DELTA) {
-        a.x = fmaf(kv, S[i].x, a.x);
-        a.y = fmaf(kv, S[i].y, a.y);
-        a.z = fmaf(kv, S[i].z, a.z);
-        a.w = fmaf(kv, S[i].w, a.w);
+        a.x = fmaf(kv, s.x, a.x);
+        a.y = fmaf(kv, s.y, a.y);
+        a.z = fmaf(kv, s.z, a.z);
+        a.w = fmaf(kv, s.w, a.w);
       }
-      b.x = fmaf(qv, S[i].x, b.x);
-      b.y = fmaf(qv, S[i].y, b.y);
-      b.z = fmaf(qv, S[i].z, b.z);
-      b.w = fmaf(qv, S[i].w, b.w);
+      b.x = fmaf(qv, s.x, b.x);
+      b.y = fmaf(qv, s.y, b.y);
+      b.z = fmaf(qv, s.z, b.z);
+      b.w = fmaf(qv, s.w, b.w);
     }
     if (DELTA) *reinterpret_cast<float4*>(part + rg * p.vdim + c) = a;
     *reinterpret_cast<float4*>(part + (rgs + rg) * p.vdim + c) = b;
@@ -244,11 +259,12 @@ state_step_kernel(const StepParams p) {
       const int r = rg + i * rgs;
       if (r >= p.dim) break;
       const float kv = ks[r];
+      const float4 s = HELD ? held[i * kStepThreads] : S[HELD ? 0 : i];
       float4 v;
-      v.x = fmaf(kv, u.x, g * S[i].x);
-      v.y = fmaf(kv, u.y, g * S[i].y);
-      v.z = fmaf(kv, u.z, g * S[i].z);
-      v.w = fmaf(kv, u.w, g * S[i].w);
+      v.x = fmaf(kv, u.x, g * s.x);
+      v.y = fmaf(kv, u.y, g * s.y);
+      v.z = fmaf(kv, u.z, g * s.z);
+      v.w = fmaf(kv, u.w, g * s.w);
       __stcs(reinterpret_cast<float4*>(dst + static_cast<size_t>(r) * p.vdim), v);
     }
   }
@@ -274,12 +290,24 @@ template <typename T, bool DELTA>
 static int launch_step(const StepParams& p, cudaStream_t st) {
   const int rpt = step_rows_per_thread(p.dim, p.vdim), rgs = kStepThreads / (p.vdim / 4);
   const size_t smem = (2 * static_cast<size_t>(p.dim) + 2 * p.vdim + 2 * static_cast<size_t>(rgs) * p.vdim) * 4;
+  int sms = 0;
+  int rc = device_sm_count(&sms);
+  if (rc) return rc;
 #define B200_STEP(RPT)                                                                                                   \
-  B200_CUDA(launch_overlapped(state_step_kernel<T, RPT, DELTA>, dim3(p.heads, p.rows), dim3(kStepThreads), smem, st, p))
+  B200_CUDA(launch_overlapped(state_step_kernel<T, RPT, DELTA, false>, dim3(p.heads, p.rows), dim3(kStepThreads), smem, st, p))
+#define B200_STEP_HELD(RPT)                                                                                              \
+  {                                                                                                                      \
+    const size_t with = smem + static_cast<size_t>(RPT) * kStepThreads * 16;                                             \
+    rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&state_step_kernel<T, RPT, DELTA, true>), static_cast<int>(with)); \
+    if (rc) return rc;                                                                                                   \
+    B200_CUDA(launch_overlapped(state_step_kernel<T, RPT, DELTA, true>, dim3(p.heads, p.rows), dim3(kStepThreads), with, st, p)); \
+  }
   if (rpt <= 4) B200_STEP(4);
   else if (rpt <= 8) B200_STEP(8);
+  else if (rpt <= 16 && p.heads * p.rows > 2 * sms) B200_STEP_HELD(16)
   else if (rpt <= 16) B200_STEP(16);
   else B200_STEP(32);
+#undef B200_STEP_HELD
 #undef B200_STEP
   return 0;
 }

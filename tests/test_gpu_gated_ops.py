@@ -455,3 +455,35 @@ def test_norms_of_many_rows_give_the_bits_of_few(ops, width, ld, center):
                                                      gate=g[lo:hi]), w, 1e-3, width, center))
     check(lambda xs, lo, hi: ops.residual_norm(xs, None, w, 1e-3, width, center))
     check(lambda xs, lo, hi: ops.group_rmsnorm(xs, d[lo:hi], w.to(BF), 1e-3, width, 4))
+
+
+@pytest.mark.parametrize("H,d,dv", [(8, 128, 128), (9, 100, 120), (6, 72, 124)])
+def test_state_steps_of_many_rows_give_the_bits_of_few(ops, H, d, dv):
+    """More (row, head) pairs than two per SM keep the state in shared memory: the same rows a few at a time, the same bits; first
+    positions, whose state is not read, among them."""
+    R = 2 * torch.cuda.get_device_properties(0).multi_processor_count // H + 9
+    C = 2 * H * d + H * dv
+    w = SimpleNamespace(heads=H, qk_heads=H, d=d, dv=dv, conv=randn(4, C, seed=1, dtype=BF, scale=0.3).to(DEV), a_log=randn(H, seed=2).to(DEV),
+                        dt_bias=randn(H, seed=3).to(DEV), decay=torch.rand(H, generator=torch.Generator().manual_seed(4)).to(DEV),
+                        head_norm=(1 + randn(dv, seed=5)).to(DEV))
+    act, ba = randn(R, C, seed=6, dtype=BF).to(DEV), randn(R, 2 * H, seed=7).to(DEV)
+    gate, ring = randn(R, H * dv, seed=8, dtype=BF).to(DEV), randn(R, 4, C, seed=9, dtype=BF).to(DEV)
+    state = randn(R, 2, H, d, dv, seed=10).to(DEV)
+    state[torch.arange(R) % 5 == 0] = float("nan")  # rows at position 0 must not look at it
+    slots, pos = torch.randperm(R, generator=torch.Generator().manual_seed(11)).to(torch.int32).to(DEV), torch.empty(R, dtype=torch.int32)
+    pos[:] = torch.where(slots.cpu() % 5 == 0, 0, 1 + torch.arange(R, dtype=torch.int32) % 9)
+    pos, st = pos.to(DEV), status()
+
+    def step(cuts):
+        S, L, rg = state.clone(), state.clone(), ring.clone()
+        out, o = torch.empty(R, H * dv, dtype=BF, device=DEV), torch.empty(R, H, dv, device=DEV)
+        for lo, hi in cuts:
+            at = (slots[lo:hi], pos[lo:hi])
+            ops.state_step(act[lo:hi], w, S, *at, None, st, ba=ba[lo:hi], q_scale=d ** -0.5, ring=rg, gate=gate[lo:hi], eps=1e-6, size=dv,
+                           out=out[lo:hi])
+            ops.state_step(act[lo:hi], w, L, *at, o[lo:hi], st)
+        return out, o, S, L, rg
+
+    for a, b in zip(step([(0, R)]), step([(lo, min(R, lo + 16)) for lo in range(0, R, 16)])):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    ops.read_status(st, "state step")
