@@ -58,6 +58,8 @@
 // kErrDevWaitTimeout and the thread stops waiting but keeps the loop structure, so the kernel ends.
 
 #include <algorithm>
+#include <functional>
+#include <utility>
 
 #include "host.h"
 #include "prefill_tc.cuh"
@@ -420,33 +422,44 @@ paged_attn_prefill_pairs_kernel(const __grid_constant__ CUtensorMap q_map, const
 #endif
 }
 
-// Key tiles until the last CTA is done, if each takes `per` tiles of rows and the longest are taken first: no
-// less than the longest, the mean, and k times the k-th that an SM takes.
-static float walk_length(int row_tiles, int per, int hkv, int qt, int first_pos, int num_tokens, int chunk, int sms) {
-  const int ctas = (row_tiles + per - 1) / per;
-  auto length = [&](int c) {  // of the c-th CTA of a kv head, late positions first, with three key tiles for its beginning and end
-    const int t0 = (ctas - 1 - c) * per * qt, last = first_pos + std::min(t0 + per * qt, num_tokens) - 1;
+// When the last CTA is done, in thirds of a single tile's key tile, if the first `pairs` CTAs of a kv head take two tiles of rows: every SM
+// takes the next CTA in the order of the grid.  A key tile of two tiles of rows counts 4/3 of one of a single tile, and what a CTA
+// does before and after its walk four key tiles.
+static int last_walk_end(int row_tiles, int pairs, int hkv, int qt, int first_pos, int num_tokens, int chunk, int sms) {
+  using Free = std::pair<int, int>;  // a time, and how many SMs are free at it
+  constexpr int kMost = 256;
+  Free heap[kMost] = {{0, std::min(sms, kMost)}};
+  int used = 1, end = 0;
+  for (int c = 0, t = row_tiles; c < row_tiles - pairs; ++c) {
+    const int tiles = c < pairs ? 2 : 1;
+    t -= tiles;
+    const int t0 = t * qt, last = first_pos + std::min(t0 + tiles * qt, num_tokens) - 1;
     const int first = chunk > 0 ? (first_pos + t0) / chunk * chunk : 0;
-    return last / kTcKeys - first / kTcKeys + 4;
-  };
-  float sum = 0.f, most = 0.f;
-  const int step = std::max(1, ctas / 64);
-  int seen = 0;
-  for (int c = 0; c < ctas; c += step, ++seen) sum += length(c), most = std::max(most, static_cast<float>(length(c)));
-  const float total = sum / seen * ctas * hkv;
-  float longest = std::max(most, total / sms);
-  for (int k = 2; (k - 1) * sms < ctas * hkv; ++k) longest = std::max(longest, static_cast<float>(k) * length((k - 1) * sms / hkv));
-  return longest;
+    const int length = (last / kTcKeys - first / kTcKeys + 1) * (tiles + 2) + 12;
+    for (int left = hkv; left > 0;) {
+      Free& next = heap[0];
+      const int time = next.first, taken = std::min(next.second, left);
+      next.second -= taken;
+      if (next.second == 0) std::pop_heap(heap, heap + used--, std::greater<Free>());
+      heap[used++] = {time + length, taken};
+      std::push_heap(heap, heap + used, std::greater<Free>());
+      end = std::max(end, time + length);
+      left -= taken;
+    }
+  }
+  return end;
 }
 // Single tiles that see at most this many keys go to the other form (paged_prefill_tc.cu).  Its loop is the slower one by 0.14 us per key
 // tile of 128, but two threads share a row and its straight-line code is half as long, which a kernel that runs once per layer fetches anew
 // each time: back to back both take 7.2 us for 91 tokens from nothing, and a whole pass over such a prompt (12 layers) 2211 us with
 // the other form, 2255 with this one; 17 tokens behind 14000 150 and 133 us.
 constexpr int kSingleKeys = 3072;
-// How many CTAs of a kv head take two tiles of rows.  A key tile of two takes 1.5 times as long as one of a single tile; what a CTA does
-// before and after its walk is worth about three key tiles.  None while every tile has an SM of its own (us, single tiles and pairs,
-// 32 / 4 heads, 500 tokens behind 333, 128 tiles: 16.3, 18.6; 8 / 8 heads, 2048 behind 8192, 128 tiles: 121, 138); all where pairs
-// end earlier (1024 from nothing 22.5, 21.8; 1024 behind 14336 290, 217).
+// How many CTAs of a kv head take two tiles of rows.  None while every tile has an SM of its own (us, single tiles and pairs,
+// 32 / 4 heads, 500 tokens behind 333, 128 tiles: 16.3, 18.6; 8 / 8 heads, 2048 behind 8192, 128 tiles: 121, 138).  With up to three
+// tiles per SM the better of none and all by last_walk_end: over 678 calls of 600 to 4096 tokens, nine head counts, with and without
+// chunks, the rule's choice is 0.3 percent behind the better form of each in the mean and 15 at worst, none 28 percent and all 0.8 (32 / 4
+// heads from nothing: 600 tokens 13.9, 15.3; 1024 22.7, 21.3; 64 / 4 in chunks of 512, 1024 tokens 35.6, 24.9; 8 / 8, 3000 tokens 41.9, 46.7).
+// Beyond that all (32 / 4, 2048 tokens 64, 42).
 static int prefill_pairs(int row_tiles, int hkv, int qt, int first_pos, int num_tokens, int chunk, int sms) {
   if (row_tiles * hkv <= sms) return 0;
   const int all = row_tiles / 2;
@@ -456,8 +469,9 @@ static int prefill_pairs(int row_tiles, int hkv, int qt, int first_pos, int num_
     const int pairs = std::min(all, row_tiles * hkv / (2 * sms) * sms / hkv);
     return (row_tiles - 2 * pairs) * hkv <= sms ? pairs : all;
   }
-  const float two = 1.5f * walk_length(row_tiles, 2, hkv, qt, first_pos, num_tokens, chunk, sms);
-  return two < walk_length(row_tiles, 1, hkv, qt, first_pos, num_tokens, chunk, sms) ? all : 0;
+  if (row_tiles * hkv > 3 * sms) return all;
+  const int two = last_walk_end(row_tiles, all, hkv, qt, first_pos, num_tokens, chunk, sms);
+  return two < last_walk_end(row_tiles, 0, hkv, qt, first_pos, num_tokens, chunk, sms) ? all : 0;
 }
 
 template <int D, int G>
