@@ -433,8 +433,10 @@ int b200_argmax_rows(const float* logits, int64_t* out, int num_rows, int n, voi
  * first `width` columns (center), or x / sqrt(mean square + eps) * weight.  The sublayer's rows are delta [num_rows, ld], or
  * the pair_weight-weighted sum of expert_rows[row_of_pair[m, k]], k < top_k (-1: no row), or absent (both NULL: x unchanged).
  * bias [ld] fp32, gate [num_rows, ld] may be NULL; weight [ld] fp32.  ld a multiple of 8, at most 8192; columns from width on
- * stay zero.
+ * stay zero.  There are two forms of the kernel with the same results; b200_residual_norm_form says which one a call takes (1: the
+ * one of fewer registers, < 0 on error).
  */
+int b200_residual_norm_form(int num_rows, int ld, int center, int dtype);
 int b200_residual_norm(float* x, const void* delta, const void* expert_rows, const int32_t* row_of_pair,
                        const float* pair_weight, int top_k, const float* bias, const void* gate, const float* weight,
                        float eps, int num_rows, int width, int ld, int center, void* out, int dtype, void* stream);

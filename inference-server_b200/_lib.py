@@ -56,6 +56,7 @@ SIGNATURES = {
     "b200_moe_bf16_down": (c_int, [c_void_p] * 6 + [c_int] * 6 + [c_void_p]),
     "b200_moe_route_sigmoid": (c_int, [c_void_p] + [c_int] * 5 + [c_float] + [c_void_p] * 3),
     "b200_moe_permute_copy": (c_int, [c_void_p] * 2 + [c_int] * 5 + [c_void_p] * 5 + [c_size_t, c_void_p]),
+    "b200_residual_norm_form": (c_int, [c_int] * 4),
     "b200_residual_norm": (c_int, [c_void_p] * 5 + [c_int] + [c_void_p] * 3 + [c_float] + [c_int] * 4 + [c_void_p, c_int, c_void_p]),
     "b200_mix_heads": (c_int, [c_void_p] * 3 + [c_int] * 5 + [c_void_p]),
     "b200_conv_silu": (c_int, [c_void_p] * 2 + [c_int] + [c_void_p] * 3 + [c_int] * 4 + [c_void_p] * 2 + [c_int, c_void_p]),

@@ -62,13 +62,17 @@ residual_norm_kernel(float* __restrict__ x, const Pending<T> p, const float* __r
         for (int k0 = 0; k0 < p.top_k; k0 += 8) {  // eight pairs at a time: their rows are in flight together
           const int n = min(8, p.top_k - k0);
           const int* rows = p.row_of_pair + static_cast<size_t>(m) * p.top_k + k0;
-          const float* pw = p.pair_weight + static_cast<size_t>(m) * p.top_k + k0;
+          const float* weights = p.pair_weight + static_cast<size_t>(m) * p.top_k + k0;
           Raw8<T> raw[8];
+          float pw[8];  // with registers to spare the weights are asked for with the row numbers
           unsigned have = 0u;
           {
             int row[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) row[u] = u < n ? __ldg(rows + u) : -1;
+            for (int u = 0; u < 8; ++u) {
+              row[u] = u < n ? __ldg(rows + u) : -1;
+              if (MAXT <= 512) pw[u] = u < n ? __ldg(weights + u) : 0.f;
+            }
 #pragma unroll
             for (int u = 0; u < 8; ++u)
               if (row[u] >= 0) {
@@ -79,7 +83,7 @@ residual_norm_kernel(float* __restrict__ x, const Pending<T> p, const float* __r
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             if (!((have >> u) & 1u)) continue;
-            const float weight_of = __ldg(pw + u);
+            const float weight_of = MAXT <= 512 ? pw[u] : __ldg(weights + u);
             float y[8];
             raw[u].get(y);
 #pragma unroll
@@ -362,6 +366,22 @@ group_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ w,
   }
 }
 
+// Which form a call takes: the one of at most 512 threads asks for all loads of a row at once (102 to 108 registers), the other has 64
+// registers and so more CTAs on an SM.  Rows longer than 512 threads have the second only, fp32 rows of up to 512 threads the first.  The
+// line is where the first form's CTAs no longer fit the GPU at once.  us with each form, the norm together with a product of 512 features
+// ahead of it and one behind, eight experts' rows per row; without a sublayer the lines lie a little lower, with one a little higher:
+//   width  512  1024 rows 12.7, 14.8   2048: 15.5, 15.4     width 2048  200 rows 14.1, 16.1   512: 18.1, 18.3   2048: 45.5, 42.1
+//   width 1024   512 rows 13.8, 15.9   4096: 42.9, 39.8     width 4096  100 rows 15.4, 17.7   200: 18.5, 18.6   2048: 86.2, 76.1
+template <typename T>
+static int residual_norm_many(int rows, int ld, int center, bool* out) {
+  const int threads = (ld / 8 + 31) / 32 * 32;
+  *out = threads > 512;
+  if (threads > 512 || sizeof(T) == 4) return 0;
+  const void* few = reinterpret_cast<const void*>(center ? &residual_norm_kernel<T, true, 512> : &residual_norm_kernel<T, false, 512>);
+  const void* many = reinterpret_cast<const void*>(center ? &residual_norm_kernel<T, true, 1024> : &residual_norm_kernel<T, false, 1024>);
+  return many_form_pays(few, many, threads, 0, 0, rows, out);
+}
+
 template <typename T>
 static int launch_residual_norm(float* x, const void* dense, const void* expert_rows, const int* row_of_pair,
                                 const float* pair_weight, int top_k, const float* bias, const void* gate,
@@ -370,15 +390,13 @@ static int launch_residual_norm(float* x, const void* dense, const void* expert_
   const Pending<T> p{static_cast<const T*>(dense), static_cast<const T*>(expert_rows), row_of_pair, pair_weight, top_k, bias,
                      static_cast<const T*>(gate)};
   const int threads = (ld / 8 + 31) / 32 * 32;
-  int sms = 0;
-  const int rc = device_sm_count(&sms);
+  bool many = false;
+  const int rc = residual_norm_many<T>(rows, ld, center, &many);
   if (rc) return rc;
 #define B200_RNORM(CENTER, MAXT)                                                                                     \
   B200_CUDA(launch_overlapped(residual_norm_kernel<T, CENTER, MAXT>, dim3(rows), dim3(threads), 0, st, x, p, weight, eps, \
                               width, ld, static_cast<T*>(out)))
-  // More rows than two CTAs per SM take at once: the form with at most 64 registers, of which four fit (rows of width 2048 with eight
-  // experts' rows each, us: 512 rows 6.3, 5.7   1777: 20.2, 15.5   4096: 53.1, 41.1; without a sublayer 17.7, 12.5).
-  if (threads <= 512 && (sizeof(T) == 4 || rows <= 2 * sms)) {
+  if (!many) {
     if (center) B200_RNORM(true, 512);
     else B200_RNORM(false, 512);
   } else {
@@ -392,6 +410,14 @@ static int launch_residual_norm(float* x, const void* dense, const void* expert_
 }  // namespace b200
 
 using namespace b200;
+
+extern "C" int b200_residual_norm_form(int num_rows, int ld, int center, int dtype) {
+  B200_REQUIRE(num_rows >= 0 && ld > 0 && ld % 8 == 0 && ld <= 8192, "residual_norm_form: %d rows of %d", num_rows, ld);
+  B200_GLUE_DTYPE("residual_norm_form");
+  bool many = false;
+  const int rc = dtype == 0 ? residual_norm_many<__nv_bfloat16>(num_rows, ld, center, &many) : residual_norm_many<float>(num_rows, ld, center, &many);
+  return rc ? rc : many;
+}
 
 extern "C" int b200_residual_norm(float* x, const void* delta, const void* expert_rows, const int32_t* row_of_pair,
                                   const float* pair_weight, int top_k, const float* bias, const void* gate,

@@ -104,6 +104,43 @@ int ensure_dynamic_smem(const void* kernel, int bytes) {
   return 0;
 }
 
+struct KernelResidency {
+  const void* kernel;
+  int device, threads;
+  size_t smem;
+  int ctas;
+};
+static std::vector<KernelResidency> g_residency;
+
+int resident_ctas(const void* kernel, int threads, size_t smem, int* out) {
+  int dev = 0;
+  B200_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(g_dev_mu);
+  for (const KernelResidency& r : g_residency)
+    if (r.kernel == kernel && r.device == dev && r.threads == threads && r.smem == smem) {
+      *out = r.ctas;
+      return 0;
+    }
+  cudaFuncAttributes attr;
+  B200_CUDA(cudaFuncGetAttributes(&attr, kernel));
+  int ctas = 0;
+  if (threads <= attr.maxThreadsPerBlock)
+    B200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kernel, threads, smem));
+  if (g_residency.size() < 256) g_residency.push_back(KernelResidency{kernel, dev, threads, smem, ctas});
+  *out = ctas;
+  return 0;
+}
+
+int many_form_pays(const void* few, const void* many, int threads, size_t few_smem, size_t many_smem, long long ctas, bool* out) {
+  int held_few = 0, held_many = 0, sms = 0;
+  int rc = resident_ctas(few, threads, few_smem, &held_few);
+  if (!rc) rc = resident_ctas(many, threads, many_smem, &held_many);
+  if (!rc) rc = device_sm_count(&sms);
+  if (rc) return rc;
+  *out = held_few == 0 || (held_many > held_few && ctas > static_cast<long long>(held_few) * sms);
+  return 0;
+}
+
 // ------------------------------------------------------- tensor-map cache --
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,

@@ -21,6 +21,15 @@ int ensure_dynamic_smem(const void* kernel, int bytes);
 // Multiprocessor count of the current device (cached per device, thread-safe).
 int device_sm_count(int* out);
 
+// CTAs of `threads` threads and `smem` bytes of dynamic shared memory of a kernel that an SM of the current device holds at once, 0
+// where it cannot be launched so.  Asked of the runtime once per kernel, device and shape; thread-safe.
+int resident_ctas(const void* kernel, int threads, size_t smem, int* out);
+
+// A kernel in two forms, `few` whose threads ask for all their loads at once and `many` with fewer registers, so that an SM may hold
+// more of its CTAs: *out says whether a grid of `ctas` goes to `many`.  That is so where `few` cannot be launched, or holds less than
+// the grid at once while `many` holds more than `few`.  How many that are depends on the threads per CTA, so on the width of a row.
+int many_form_pays(const void* few, const void* many, int threads, size_t few_smem, size_t many_smem, long long ctas, bool* out);
+
 // Looks up (or encodes and caches) a 2-D row-major tensor map:
 //   rows x cols elements of `elem_bytes` (1 = uint8, 2 = bf16), row pitch =
 //   cols * elem_bytes, box = box_rows x box_cols, 128-byte swizzle.

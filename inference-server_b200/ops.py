@@ -723,6 +723,18 @@ def argmax_rows(logits, out=None):
 # --------------------------------------- gated layer-list decoders (gated.py)
 
 
+def _form(name: str, *args) -> int:
+    form = getattr(_lib.load(), name)(*(int(a) for a in args))
+    if form < 0:
+        check(form, name)
+    return form
+
+
+def residual_norm_form(num_rows: int, ld: int, center: bool = True, dtype=torch.bfloat16) -> int:
+    """The form of its kernel that residual_norm takes on the current device; 1: the one of fewer registers.  Same results."""
+    return _form("b200_residual_norm_form", num_rows, ld, center, DTYPE_CODE[dtype])
+
+
 def residual_norm(x, pending, weight, eps: float, width: int, center: bool = True, out=None, dtype=torch.bfloat16):
     """x (fp32) += (sublayer + bias) * gate in place (`pending`: gated.Pending or None); returns layer norm (center) or RMS norm
     of x over its first `width` columns times weight (fp32)."""

@@ -1,0 +1,59 @@
+"""Kernels that come in two forms: which call goes to which, and that both give the same bits."""
+import pytest
+import torch
+
+from conftest import pkg
+
+pytestmark = pytest.mark.gpu
+DEV, BF = "cuda", torch.bfloat16
+
+
+def randn(*shape, seed, dtype=torch.float32):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(dtype).to(DEV)
+
+
+def line(form, lo=1, hi=1 << 17):
+    """The smallest count from `lo` on that goes to form 1, where there is one."""
+    if not form(hi):
+        return None
+    while lo < hi:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if form(mid) else (mid + 1, hi)
+    return lo
+
+
+def same_bits(call, rows, step):
+    """All rows in one call, and a few at a time: `call(lo, hi)` gives tensors by row."""
+    whole, parts = call(0, rows), [call(lo, min(rows, lo + step)) for lo in range(0, rows, step)]
+    for i, t in enumerate(whole):
+        assert torch.equal(t, torch.cat([p[i] for p in parts]))
+
+
+@pytest.mark.parametrize("center", [True, False])
+def test_residual_norm_goes_by_what_an_sm_holds(ops, center):
+    """A CTA has a thread for eight columns, so that rows of half the width have twice as many CTAs on an SM: the form that has more
+    of them has nothing to offer before they are used up."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    lines = [line(lambda n: ops.residual_norm_form(n, ld, center)) for ld in (256, 512, 1024, 2048, 4096)]
+    assert all(b < a for a, b in zip(lines, lines[1:]))
+    assert all((n - 1) % sms == 0 for n in lines) and lines[-1] == sms + 1  # 512 threads: one CTA per SM, and two
+    assert ops.residual_norm_form(1, 4104, center) == 1  # more than 512 threads: the only form
+    assert ops.residual_norm_form(1 << 17, 512, center, torch.float32) == 0
+
+
+@pytest.mark.parametrize("width,ld", [(250, 256), (1024, 1024), (4090, 4096)])
+def test_residual_norm_forms_give_the_same_bits(ops, width, ld):
+    P = pkg("gated").Pending
+    M, top = line(lambda n: ops.residual_norm_form(n, ld)) + 7, 9
+    cut = (torch.arange(ld) < width).to(DEV)
+    x, w, bias = randn(M, ld, seed=1) * cut, (1 + randn(ld, seed=2)) * cut, randn(ld, seed=6) * cut
+    d, gate, e = (randn(M, ld, seed=s, dtype=BF) * cut for s in (3, 4, 5))
+    pairs = torch.randint(-1, M, (M, top), generator=torch.Generator().manual_seed(7)).to(torch.int32).to(DEV)
+    pw = torch.rand(M, top, generator=torch.Generator().manual_seed(8)).to(DEV)
+    for pending in (lambda a, b: None, lambda a, b: P(dense=d[a:b], gate=gate[a:b], bias=bias),
+                    lambda a, b: P(expert_rows=e, row_of_pair=pairs[a:b].contiguous(), pair_weight=pw[a:b].contiguous(), gate=gate[a:b])):
+        def call(a, b):
+            xs = x[a:b].clone()
+            return ops.residual_norm(xs, pending(a, b), w, 1e-3, width), xs
+        assert ops.residual_norm_form(M, ld) == 1 and ops.residual_norm_form(100, ld) == 0
+        same_bits(call, M, 100)
