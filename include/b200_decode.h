@@ -699,8 +699,10 @@ int b200_moe_combine(const void* y_sorted, const int32_t* row_of_pair, const flo
 /*
  * b200_moe_combine followed by b200_add_rmsnorm in one kernel: the combined
  * expert output is rounded to bf16, added to the residual stream x (in place)
- * and the result is normalised with `weight` into `out`.
+ * and the result is normalised with `weight` into `out`.  There are two forms of the kernel with the same
+ * results; the _form call says which one a call takes (1: the one of fewer registers, < 0 on error).
  */
+int b200_moe_combine_add_rmsnorm_form(int num_tokens, int hidden);
 int b200_moe_combine_add_rmsnorm(const void* y_sorted, const int32_t* row_of_pair,
                                  const float* topk_weights, void* x, const void* weight, float eps,
                                  int num_tokens, int hidden, int top_k, void* out, void* stream);

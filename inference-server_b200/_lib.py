@@ -99,6 +99,7 @@ SIGNATURES = {
     "b200_moe_fp8_gemm_down_staged": (c_int, [c_int] * 3),
     "b200_moe_fp8_gemm_down": (c_int, [c_void_p] * 9 + [c_int] * 5 + [c_void_p]),
     "b200_moe_combine": (c_int, [c_void_p] * 3 + [c_int] * 3 + [c_void_p, c_void_p]),
+    "b200_moe_combine_add_rmsnorm_form": (c_int, [c_int] * 2),
     "b200_moe_combine_add_rmsnorm": (c_int, [c_void_p] * 5 + [c_float] + [c_int] * 3 + [c_void_p, c_void_p]),
     "b200_moe_fp8_workspace_bytes": (c_size_t, [c_int] * 5),
     "b200_moe_fp8_forward": (c_int, [c_void_p, c_void_p, c_int] + [c_void_p] * 6 + [c_size_t] + [c_int] * 7 + [c_void_p]),

@@ -693,9 +693,8 @@ __global__ void moe_combine_add_rmsnorm_kernel(const __nv_bfloat16* __restrict__
   *reinterpret_cast<uint4*>(out + base) = o;
 }
 
-// The same for many tokens: at most 64 registers, so that four CTAs of 256 threads fit on an SM where two of the form above do; the loads
-// that are not asked for up front then are those of the weights.  us, width 2048, 8 rows each, that form and this one: 37 tokens 2.4,
-// 2.5   512: 4.7, 4.1   2048: 15.6, 11.5   4096: 41.1, 34.
+// The same with at most 64 registers in place of 92, so that more CTAs of a row may fit on an SM; the loads that are not asked for up front
+// then are those of the weights.  (Both as one template, with these lines switched: the form above 10 percent slower.)
 __global__ void __maxnreg__(64)
 moe_combine_add_rmsnorm_many_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of_pair,
                                     const float* __restrict__ topk_w, int H, int K, __nv_bfloat16* __restrict__ x,
@@ -760,6 +759,17 @@ moe_combine_add_rmsnorm_many_kernel(const __nv_bfloat16* __restrict__ y, const i
   for (int j = 0; j < 4; ++j)
     o2[j] = __hmul2(w2[j], __floats2bfloat162_rn(f[2 * j] * inv, f[2 * j + 1] * inv));
   *reinterpret_cast<uint4*>(out + base) = o;
+}
+
+// Which form a call of moe_combine_add_rmsnorm takes: the second where CTAs of the first no longer fit the GPU at once and more of the second
+// do (not at 4352 to 5376 columns, where both have one CTA per SM), and beyond 5376 columns, for which the first has no registers.  us of
+// the first and of the second between two products of 512 features, 8 rows each:
+//   width  512  1024 tokens 12.0, 12.8   2048: 14.1, 13.3     width 2048  200 tokens 13.3, 14.2   512: 16.8, 16.1   2048: 39.0, 32.7
+//   width 1024   512 tokens 13.1, 13.8   2048: 18.7, 17.7     width 4096  100 tokens 14.4, 15.1   200: 16.8, 15.9   2048: 74.4, 62.2
+//   width 5120   512 tokens 26.8, 27.6
+static int combine_many(int tokens, int hidden, bool* out) {
+  return many_form_pays(reinterpret_cast<const void*>(&moe_combine_add_rmsnorm_kernel),
+                        reinterpret_cast<const void*>(&moe_combine_add_rmsnorm_many_kernel), hidden / 8, 0, 0, tokens, out);
 }
 
 }  // namespace b200
@@ -1034,6 +1044,16 @@ extern "C" int b200_gather_rows_fp8(const void* src_q, const float* src_scale, c
   return 0;
 }
 
+extern "C" int b200_moe_combine_add_rmsnorm_form(int num_tokens, int hidden) {
+  B200_REQUIRE(num_tokens >= 0 && hidden > 0 && hidden % 256 == 0 && hidden <= 8192, "moe_combine_add_rmsnorm_form: %d rows of %d",
+               num_tokens, hidden);
+  int rc = check_device(nullptr);
+  if (rc) return rc;
+  bool many = false;
+  rc = combine_many(num_tokens, hidden, &many);
+  return rc ? rc : many;
+}
+
 extern "C" int b200_moe_combine_add_rmsnorm(const void* y_sorted, const int32_t* row_of_pair,
                                             const float* topk_weights, void* x, const void* weight,
                                             float eps, int num_tokens, int hidden, int top_k, void* out,
@@ -1048,20 +1068,13 @@ extern "C" int b200_moe_combine_add_rmsnorm(const void* y_sorted, const int32_t*
   int rc = check_device(nullptr);
   if (rc) return rc;
   if (num_tokens == 0) return 0;
-  int sms = 0;
-  rc = device_sm_count(&sms);
+  bool many = false;
+  rc = combine_many(num_tokens, hidden, &many);
   if (rc) return rc;
-  if (num_tokens > 2 * sms || hidden > 4096) {
-    B200_CUDA(launch_overlapped(moe_combine_add_rmsnorm_many_kernel, dim3(num_tokens), dim3(hidden / 8), 0, as_stream(stream),
-                              static_cast<const __nv_bfloat16*>(y_sorted), row_of_pair, topk_weights, hidden, top_k,
-                              static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(weight), eps,
+  B200_CUDA(launch_overlapped(many ? moe_combine_add_rmsnorm_many_kernel : moe_combine_add_rmsnorm_kernel, dim3(num_tokens),
+                              dim3(hidden / 8), 0, as_stream(stream), static_cast<const __nv_bfloat16*>(y_sorted), row_of_pair,
+                              topk_weights, hidden, top_k, static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(weight), eps,
                               static_cast<__nv_bfloat16*>(out)));
-  } else {
-    B200_CUDA(launch_overlapped(moe_combine_add_rmsnorm_kernel, dim3(num_tokens), dim3(hidden / 8), 0, as_stream(stream),
-                              static_cast<const __nv_bfloat16*>(y_sorted), row_of_pair, topk_weights, hidden, top_k,
-                              static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(weight), eps,
-                              static_cast<__nv_bfloat16*>(out)));
-  }
   return 0;
 }
 

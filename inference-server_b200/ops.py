@@ -1408,6 +1408,11 @@ def moe_combine(y_sorted, row_of_pair, topk_weights):
     return out
 
 
+def moe_combine_add_rmsnorm_form(num_tokens: int, hidden: int) -> int:
+    """The form of its kernel that moe_combine_add_rmsnorm takes on the current device; 1: the one of fewer registers.  Same results."""
+    return _form("b200_moe_combine_add_rmsnorm_form", num_tokens, hidden)
+
+
 def moe_combine_add_rmsnorm(y_sorted, row_of_pair, topk_weights, x, weight, eps: float, out=None):
     """x += bf16(sum_k w * y) in place; returns weight * rmsnorm(x)."""
     _need(y_sorted, "y_sorted", torch.bfloat16)

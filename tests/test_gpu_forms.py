@@ -57,3 +57,27 @@ def test_residual_norm_forms_give_the_same_bits(ops, width, ld):
             return ops.residual_norm(xs, pending(a, b), w, 1e-3, width), xs
         assert ops.residual_norm_form(M, ld) == 1 and ops.residual_norm_form(100, ld) == 0
         same_bits(call, M, 100)
+
+
+def test_combine_goes_by_what_an_sm_holds(ops):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    lines = [line(lambda n: ops.moe_combine_add_rmsnorm_form(n, h)) for h in (256, 512, 1024, 2048, 4096)]
+    assert all(b < a for a, b in zip(lines, lines[1:]))
+    assert all((n - 1) % sms == 0 for n in lines) and lines[-1] == sms + 1  # 512 threads: one CTA per SM, and two
+    assert ops.moe_combine_add_rmsnorm_form(1 << 17, 5120) == 0  # 640 threads: one CTA per SM of either form
+    assert ops.moe_combine_add_rmsnorm_form(1, 8192) == 1        # 1024 threads, for which the other form has no registers
+
+
+@pytest.mark.parametrize("H,K", [(256, 8), (1024, 9), (4096, 2)])
+def test_combine_forms_give_the_same_bits(ops, H, K):
+    T = line(lambda n: ops.moe_combine_add_rmsnorm_form(n, H)) + 7
+    y, x, nw = randn(T * K, H, seed=1, dtype=BF), randn(T, H, seed=2, dtype=BF), (1 + 0.1 * randn(H, seed=3)).to(BF)
+    rows = torch.randperm(T * K, generator=torch.Generator().manual_seed(4)).view(T, K).to(torch.int32)
+    rows[torch.rand(T, K, generator=torch.Generator().manual_seed(5)) < 0.1] = -1
+    rows, w = rows.to(DEV), torch.rand(T, K, generator=torch.Generator().manual_seed(6)).to(DEV)
+
+    def call(a, b):
+        xs = x[a:b].clone()
+        return ops.moe_combine_add_rmsnorm(y, rows[a:b].contiguous(), w[a:b].contiguous(), xs, nw, 1e-6), xs
+    assert ops.moe_combine_add_rmsnorm_form(T, H) == 1 and ops.moe_combine_add_rmsnorm_form(100, H) == 0
+    same_bits(call, T, 100)
