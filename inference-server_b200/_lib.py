@@ -42,6 +42,7 @@ SIGNATURES = {
     "b200_dense_glu_gemm": (c_int, [c_void_p] * 4 + [c_int] * 3 + [c_float] * 2 + [c_void_p]),
     "b200_gemm_f32": (c_int, [c_void_p] * 3 + [c_int] * 9 + [c_void_p]),
     "b200_embed_sinusoid": (c_int, [c_void_p] * 7 + [c_int] * 6 + [c_void_p]),
+    "b200_group_rmsnorm_form": (c_int, [c_int] * 5),
     "b200_group_rmsnorm": (c_int, [c_void_p] * 3 + [c_float] + [c_int] * 4 + [c_void_p] * 2 + [c_int] + [c_void_p] * 3
                            + [c_int] * 3 + [c_void_p, c_int, c_void_p]),
     "b200_short_conv": (c_int, [c_void_p] * 2 + [c_int] + [c_void_p] * 2 + [c_int] * 3 + [c_void_p] + [c_int] * 3

@@ -449,22 +449,43 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
   }
 }
 
+// The groups of a row are whole warps' columns: their sums meet in 32 words, and not in a row of shared memory.
+static bool group_norm_wide(int width, int groups) { return (width / groups) % 256 == 0; }
+static size_t group_norm_smem(int width, int ld, int groups) {
+  return group_norm_wide(width, groups) ? 32 * 4 : static_cast<size_t>(ld + groups) * 4;
+}
+
+// Which form a call takes: the one of at most 512 threads has 78 registers, the other 64 and so, at most widths, more CTAs on an SM (not at
+// 3072).  Rows longer than 512 threads have the second only, fp32 activations of up to 512 threads the first.  The line is where the first
+// form's CTAs no longer fit the GPU at once.  us with each form, the norm of 16 groups between two products of 512 features:
+//   width  512  1500 rows 17.1, 18.1   2048: 21.6, 18.3     width 2048  297 rows 16.8, 17.5   512: 19.6, 18.1   2048: 35.3, 33.0
+//   width 1024   700 rows 16.4, 17.3   1024: 19.5, 17.3     width 4096  100 rows 14.2, 14.7   200: 16.3, 15.3   2048: 53.0, 44.5
+template <typename T>
+static int group_rmsnorm_many(int rows, int width, int ld, int groups, bool* out) {
+  const int threads = (ld / 8 + 31) / 32 * 32;
+  *out = threads > 512;
+  if (threads > 512 || sizeof(T) == 4) return 0;
+  const bool wide = group_norm_wide(width, groups);
+  const void* few = reinterpret_cast<const void*>(wide ? &group_rmsnorm_kernel<T, true, 512> : &group_rmsnorm_kernel<T, false, 512>);
+  const void* many = reinterpret_cast<const void*>(wide ? &group_rmsnorm_kernel<T, true, 1024> : &group_rmsnorm_kernel<T, false, 1024>);
+  const size_t smem = group_norm_smem(width, ld, groups);
+  return many_form_pays(few, many, threads, smem, smem, rows, out);
+}
+
 template <typename T>
 static int launch_group_rmsnorm(float* x, const void* delta, const void* weight, float eps, int rows, int width, int ld,
                                 int groups, void* out, const void* conv_w, int taps, void* hist, const int* positions,
                                 const int* block_table, const PageMap& pm, cudaStream_t st) {
   const int threads = (ld / 8 + 31) / 32 * 32;
-  const bool wide = (width / groups) % 256 == 0;
-  const size_t smem = wide ? 32 * 4 : static_cast<size_t>(ld + groups) * 4;
-  int sms = 0;
-  const int rc = device_sm_count(&sms);
+  const bool wide = group_norm_wide(width, groups);
+  const size_t smem = group_norm_smem(width, ld, groups);
+  bool many = false;
+  const int rc = group_rmsnorm_many<T>(rows, width, ld, groups, &many);
   if (rc) return rc;
 #define B200_NORM_ARGS                                                                                              \
   x, static_cast<const T*>(delta), static_cast<const T*>(weight), eps, width, ld, groups, static_cast<T*>(out),      \
       static_cast<const T*>(conv_w), taps, static_cast<T*>(hist), positions, block_table, pm
-  // More rows than three CTAs per SM take at once: the form with at most 64 registers, of which four fit (width 2048, us: 512 rows 4.2,
-  // 3.3   1024: 5.9, 5.1   2048: 9.3, 8.6   4096: 16.6, 14.7).
-  if (threads <= 512 && (sizeof(T) == 4 || rows <= 3 * sms)) {
+  if (!many) {
     if (wide)
       B200_CUDA(launch_overlapped(group_rmsnorm_kernel<T, true, 512>, dim3(rows), dim3(threads), smem, st, B200_NORM_ARGS));
     else
@@ -519,6 +540,16 @@ extern "C" int b200_embed_sinusoid(const int64_t* tokens, const int32_t* positio
     B200_CUDA(launch_overlapped(embed_sinusoid_kernel<float>, dim3(num_rows), dim3(threads), 0, as_stream(stream), tk,
                                 positions, static_cast<const float*>(embed), lo, hi, x, err, width, ld, vocab, n_hi));
   return 0;
+}
+
+extern "C" int b200_group_rmsnorm_form(int num_rows, int width, int ld, int groups, int dtype) {
+  B200_REQUIRE(num_rows >= 0 && width > 0 && ld >= width && ld % 8 == 0 && ld <= 8192 && groups > 0 && width % groups == 0,
+               "group_rmsnorm_form: %d rows of %d (pitch %d) in %d groups", num_rows, width, ld, groups);
+  B200_GLUE_DTYPE("group_rmsnorm_form");
+  bool many = false;
+  const int rc = dtype == 0 ? group_rmsnorm_many<__nv_bfloat16>(num_rows, width, ld, groups, &many)
+                            : group_rmsnorm_many<float>(num_rows, width, ld, groups, &many);
+  return rc ? rc : many;
 }
 
 extern "C" int b200_group_rmsnorm(float* x, const void* delta, const void* weight, float eps, int num_rows, int width,

@@ -32,6 +32,13 @@ def _need(t: torch.Tensor, name: str, dtype=None):
         raise ValueError(f"{name} must be {dtype}, got {t.dtype}")
 
 
+def _form(name: str, *args) -> int:
+    form = getattr(_lib.load(), name)(*(int(a) for a in args))
+    if form < 0:
+        check(form, name)
+    return form
+
+
 def read_status(status: torch.Tensor, where: str = "device status") -> None:
     """Synchronise and raise if the device status word at the start of `status` is set."""
     rc = _lib.load().b200_read_status(status.data_ptr(), _stream())
@@ -647,6 +654,11 @@ def embed_sinusoid(tokens, positions, embed, tables, width: int, status=None):
     return x
 
 
+def group_rmsnorm_form(num_rows: int, width: int, ld: int, groups: int, dtype=torch.bfloat16) -> int:
+    """The form of its kernel that group_rmsnorm takes on the current device; 1: the one of fewer registers.  Same results."""
+    return _form("b200_group_rmsnorm_form", num_rows, width, ld, groups, DTYPE_CODE[dtype])
+
+
 def group_rmsnorm(x, delta, weight, eps: float, width: int, groups: int, conv_w=None, hist=None, positions=None,
                   block_table=None, page: int = 16, status=None, out=None):
     """x (fp32) += delta in place; returns weight * x / rms per group of columns, in weight's dtype.  With conv_w [taps, ld]
@@ -721,13 +733,6 @@ def argmax_rows(logits, out=None):
 
 
 # --------------------------------------- gated layer-list decoders (gated.py)
-
-
-def _form(name: str, *args) -> int:
-    form = getattr(_lib.load(), name)(*(int(a) for a in args))
-    if form < 0:
-        check(form, name)
-    return form
 
 
 def residual_norm_form(num_rows: int, ld: int, center: bool = True, dtype=torch.bfloat16) -> int:

@@ -81,3 +81,27 @@ def test_combine_forms_give_the_same_bits(ops, H, K):
         return ops.moe_combine_add_rmsnorm(y, rows[a:b].contiguous(), w[a:b].contiguous(), xs, nw, 1e-6), xs
     assert ops.moe_combine_add_rmsnorm_form(T, H) == 1 and ops.moe_combine_add_rmsnorm_form(100, H) == 0
     same_bits(call, T, 100)
+
+
+@pytest.mark.parametrize("parts", [1, 16])
+def test_grouped_norm_goes_by_what_an_sm_holds(ops, parts):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    lines = [line(lambda n: ops.group_rmsnorm_form(n, w, w, parts)) for w in (512, 1024, 2048, 4096)]
+    assert all(b < a for a, b in zip(lines, lines[1:]))
+    assert all((n - 1) % sms == 0 for n in lines) and lines[-1] == sms + 1  # 512 threads: one CTA per SM, and two
+    assert ops.group_rmsnorm_form(1 << 17, 3072, 3072, parts) == 0  # 384 threads: two CTAs per SM of either form
+    assert ops.group_rmsnorm_form(1, 4104, 4104, 1) == 1            # more than 512 threads: the only form
+    assert ops.group_rmsnorm_form(1 << 17, 512, 512, parts, torch.float32) == 0
+
+
+@pytest.mark.parametrize("width,ld,groups", [(510, 512, 6), (1024, 1024, 4), (4096, 4096, 1)])
+def test_grouped_norm_forms_give_the_same_bits(ops, width, ld, groups):
+    M = line(lambda n: ops.group_rmsnorm_form(n, width, ld, groups)) + 7
+    cut = (torch.arange(ld) < width).to(DEV)
+    x, d, w = randn(M, ld, seed=1) * cut, randn(M, ld, seed=2, dtype=BF) * cut, ((1 + randn(ld, seed=3)) * cut).to(BF)
+
+    def call(a, b):
+        xs = x[a:b].clone()
+        return ops.group_rmsnorm(xs, d[a:b], w, 1e-3, width, groups), xs
+    assert ops.group_rmsnorm_form(M, width, ld, groups) == 1 and ops.group_rmsnorm_form(100, width, ld, groups) == 0
+    same_bits(call, M, 100)
