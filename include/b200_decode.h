@@ -518,9 +518,11 @@ int b200_state_chunk(const void* act, int ld, int q_off, int k_off, int v_off, c
  * One decode step: every row is a sequence of its own.  decay given: act is activated, o [num_rows, heads, vdim] gets the
  * result.  Otherwise act holds the inputs of the convolution (conv_w, taps and ring as in b200_conv_silu over the rows' ld
  * channels), and out[m, h] = o / sqrt(mean square over norm_size + eps) * norm * gate[m, h] * out_scale, rows out_ld apart.
- * _supported: dim and vdim multiples of 4 that fit a CTA's registers.
+ * _supported: dim and vdim multiples of 4 that fit a CTA's registers.  _held: whether the states of a call wait in shared memory (1)
+ * or in registers (0; < 0 on error), with the same results; `delta`: the gated delta rule.
  */
 int b200_state_step_supported(int dim, int vdim);
+int b200_state_step_held(int num_rows, int heads, int dim, int vdim, int delta, int dtype);
 int b200_state_step(const void* act, int ld, int q_off, int k_off, int v_off, const void* conv_w, void* ring, int taps,
                     const float* ba, const float* a_log, const float* dt_bias, const float* decay, float* state,
                     const int32_t* slots, const int32_t* positions, float* o, const void* gate, const float* norm, void* out,

@@ -57,9 +57,11 @@ __device__ __forceinline__ float cta_sum(float v, float* red) {
 
 // HELD: the state waits in shared memory (a thread's own pieces, fetched by cp.async) and not in registers.  64 KB of state per CTA take 64
 // registers a thread, which with all else leaves room for two CTAs on an SM; three fit this way, and what a CTA does beside
-// moving its state (window, norms, sums) is hidden better.  us in registers and held, 16 heads of 128 x 128: delta rule 37 rows 15.8, 14.3
-// 256: 112, 85 (its bytes: 83); lightning 256 rows 82, 79.  With no more CTAs than two per SM, and for states of other sizes than 9 to 16
-// rows per thread, registers (100 x 120, 64 rows of 4 heads: 7.2, 9.1; 128 x 64 has room for its CTAs as it is).
+// moving its state (window, norms, sums) is hidden better.  us in registers and held, 16 heads of 128 x 128: delta rule 37 rows 17.1, 14.2
+// 256: 118, 90 (its bytes: 83); lightning 256 rows 88, 84.  Registers stay (step_held below) where the CTAs fit two per SM (100 x 120, 64 rows of
+// 4 heads: 7.2, 9.1), where the vectors of a long head leave shared memory for two CTAs only (64 rows of 16 heads, delta rule and
+// lightning, 32 x 512: 36, 40 and 25.8, 27.3; 1024 x 16: 51, 55 and 31.8, 37.0), and for states of other sizes than 9 to 16 rows per thread
+// (128 x 64 has room for its CTAs as it is).
 template <typename T, int RPT, bool DELTA, bool HELD>
 __global__ void __launch_bounds__(kStepThreads, HELD ? 3 : 0)
 state_step_kernel(const StepParams p) {
@@ -286,28 +288,40 @@ static int step_rows_per_thread(int dim, int vdim) {
   return rgs > 0 ? (dim + rgs - 1) / rgs : 1 << 30;
 }
 
+// Shared memory of a CTA without and with its state, which takes 16 pieces of 16 bytes per thread.
+static size_t step_smem(int dim, int vdim) {
+  return (2 * static_cast<size_t>(dim) + 2 * vdim + 2 * static_cast<size_t>(kStepThreads / (vdim / 4)) * vdim) * 4;
+}
+static size_t step_held_smem(int dim, int vdim) { return step_smem(dim, vdim) + static_cast<size_t>(16) * kStepThreads * 16; }
+
+// Whether the states of a call wait in shared memory: more CTAs of that form fit on an SM, and there are more than the other's hold.
+template <typename T, bool DELTA>
+static int step_held(int rows, int heads, int dim, int vdim, bool* out) {
+  const int rpt = step_rows_per_thread(dim, vdim);
+  *out = false;
+  if (rpt <= 8 || rpt > 16) return 0;
+  const void* held = reinterpret_cast<const void*>(&state_step_kernel<T, 16, DELTA, true>);
+  int rc = ensure_dynamic_smem(held, static_cast<int>(step_held_smem(dim, vdim)));
+  if (rc) return rc;
+  return many_form_pays(reinterpret_cast<const void*>(&state_step_kernel<T, 16, DELTA, false>), held, kStepThreads, step_smem(dim, vdim),
+                        step_held_smem(dim, vdim), static_cast<long long>(rows) * heads, out);
+}
+
 template <typename T, bool DELTA>
 static int launch_step(const StepParams& p, cudaStream_t st) {
-  const int rpt = step_rows_per_thread(p.dim, p.vdim), rgs = kStepThreads / (p.vdim / 4);
-  const size_t smem = (2 * static_cast<size_t>(p.dim) + 2 * p.vdim + 2 * static_cast<size_t>(rgs) * p.vdim) * 4;
-  int sms = 0;
-  int rc = device_sm_count(&sms);
+  const int rpt = step_rows_per_thread(p.dim, p.vdim);
+  const size_t smem = step_smem(p.dim, p.vdim), with = step_held_smem(p.dim, p.vdim);
+  bool held = false;
+  const int rc = step_held<T, DELTA>(p.rows, p.heads, p.dim, p.vdim, &held);
   if (rc) return rc;
 #define B200_STEP(RPT)                                                                                                   \
   B200_CUDA(launch_overlapped(state_step_kernel<T, RPT, DELTA, false>, dim3(p.heads, p.rows), dim3(kStepThreads), smem, st, p))
-#define B200_STEP_HELD(RPT)                                                                                              \
-  {                                                                                                                      \
-    const size_t with = smem + static_cast<size_t>(RPT) * kStepThreads * 16;                                             \
-    rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&state_step_kernel<T, RPT, DELTA, true>), static_cast<int>(with)); \
-    if (rc) return rc;                                                                                                   \
-    B200_CUDA(launch_overlapped(state_step_kernel<T, RPT, DELTA, true>, dim3(p.heads, p.rows), dim3(kStepThreads), with, st, p)); \
-  }
   if (rpt <= 4) B200_STEP(4);
   else if (rpt <= 8) B200_STEP(8);
-  else if (rpt <= 16 && p.heads * p.rows > 2 * sms) B200_STEP_HELD(16)
+  else if (held)
+    B200_CUDA(launch_overlapped(state_step_kernel<T, 16, DELTA, true>, dim3(p.heads, p.rows), dim3(kStepThreads), with, st, p));
   else if (rpt <= 16) B200_STEP(16);
   else B200_STEP(32);
-#undef B200_STEP_HELD
 #undef B200_STEP
   return 0;
 }
@@ -320,6 +334,19 @@ extern "C" int b200_state_step_supported(int dim, int vdim) {
   // the head's vectors and partial sums stay below the 48 KiB of shared memory a kernel has without asking for more
   return dim > 0 && vdim > 0 && dim % 4 == 0 && vdim % 4 == 0 && vdim <= 1024 && step_rows_per_thread(dim, vdim) <= 32 &&
          (2 * dim + 2 * vdim + 2 * 4 * kStepThreads) * 4 <= 46 * 1024;
+}
+
+extern "C" int b200_state_step_held(int num_rows, int heads, int dim, int vdim, int delta, int dtype) {
+  B200_REQUIRE(num_rows >= 0 && heads > 0 && b200_state_step_supported(dim, vdim), "state_step_held: %d rows, %d heads, state %d x %d",
+               num_rows, heads, dim, vdim);
+  B200_GLUE_DTYPE("state_step_held");
+  bool held = false;
+  int rc = 0;
+  if (dtype == 0)
+    rc = delta ? step_held<__nv_bfloat16, true>(num_rows, heads, dim, vdim, &held) : step_held<__nv_bfloat16, false>(num_rows, heads, dim, vdim, &held);
+  else
+    rc = delta ? step_held<float, true>(num_rows, heads, dim, vdim, &held) : step_held<float, false>(num_rows, heads, dim, vdim, &held);
+  return rc ? rc : held;
 }
 
 extern "C" int b200_state_step(const void* act, int ld, int q_off, int k_off, int v_off, const void* conv_w, void* ring, int taps,

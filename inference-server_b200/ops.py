@@ -955,6 +955,11 @@ def state_step_supported(dim: int, vdim: int) -> bool:
     return bool(_lib.load().b200_state_step_supported(int(dim), int(vdim)))
 
 
+def state_step_held(num_rows: int, heads: int, dim: int, vdim: int, delta: bool, dtype=torch.bfloat16) -> bool:
+    """Whether the states of a call wait in shared memory and not in registers (the results are the same)."""
+    return bool(_form("b200_state_step_held", num_rows, heads, dim, vdim, delta, DTYPE_CODE[dtype]))
+
+
 def state_step(act, w, state, slots, positions, o, status=None, ba=None, q_scale: float = 1.0, ring=None, gate=None, eps: float = 0.0,
                size: int = 0, scale: float = 1.0, out=None):
     """One decode step of the recurrence per row.  Without `ba`: `act` is activated, o [M, H, dv] fp32 gets the result.  With it

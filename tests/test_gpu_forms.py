@@ -105,3 +105,14 @@ def test_grouped_norm_forms_give_the_same_bits(ops, width, ld, groups):
         return ops.group_rmsnorm(xs, d[a:b], w, 1e-3, width, groups), xs
     assert ops.group_rmsnorm_form(M, width, ld, groups) == 1 and ops.group_rmsnorm_form(100, width, ld, groups) == 0
     same_bits(call, M, 100)
+
+
+@pytest.mark.parametrize("delta", [True, False])
+@pytest.mark.parametrize("dtype", [BF, torch.float32])
+def test_states_wait_in_shared_memory_where_more_of_them_fit(ops, delta, dtype):
+    """In registers two CTAs fit on an SM; with 64 KB of state and the vectors of the head in shared memory three or two."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for dim, vdim in ((128, 128), (100, 120), (64, 256), (256, 64)):
+        assert not ops.state_step_held(2 * sms, 1, dim, vdim, delta, dtype) and ops.state_step_held(2 * sms + 1, 1, dim, vdim, delta, dtype)
+    for dim, vdim in ((32, 512), (16, 1024), (12, 1024), (512, 32), (1024, 16), (128, 64), (144, 144)):
+        assert not ops.state_step_held(4096, 16, dim, vdim, delta, dtype)
