@@ -599,8 +599,11 @@ int b200_moe_route(const void* logits, int logits_dtype, int num_tokens, int num
  *   num_tiles       1 int32
  *   workspace       b200_moe_permute_workspace_bytes(...); starts with the
  *                   status word
+ * b200_moe_rank_threads: threads of a CTA of the kernel that ranks an expert's
+ * pairs, 256 or 1024, on a GPU of num_sms SMs (here and in the calls below).
  */
 size_t b200_moe_permute_workspace_bytes(int num_tokens, int num_experts, int top_k);
+int b200_moe_rank_threads(int num_pairs, int num_experts, int num_sms);
 int b200_moe_max_tiles(int num_tokens, int num_experts, int top_k);
 int b200_moe_permute(const int32_t* topk_ids, int num_tokens, int num_experts, int top_k,
                      int32_t* sorted_pair_ids, int32_t* row_of_pair, int32_t* expert_offsets,

@@ -89,6 +89,7 @@ SIGNATURES = {
     "b200_moe_route": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "b200_moe_permute_workspace_bytes": (c_size_t, [c_int] * 3),
     "b200_moe_max_tiles": (c_int, [c_int] * 3),
+    "b200_moe_rank_threads": (c_int, [c_int] * 3),
     "b200_moe_permute": (
         c_int,
         [c_void_p, c_int, c_int, c_int] + [c_void_p] * 5 + [c_int, c_void_p, c_size_t, c_void_p],

@@ -103,10 +103,9 @@ moe_route_sigmoid_kernel(const LT* __restrict__ logits, int T, int E, int K, int
 
 // ---------------------------------------------------------------- permute ---
 constexpr int kRankThreads = 256, kRankManyThreads = 1024;
-constexpr int kRankMany = 8192;  // pairs
 
-// moe_rank_kernel for more than 16 pairs per thread: a thread's `chunk` ids (a multiple of 4) are read in 16-byte pieces, eight of
-// them in flight, once to count and once to place.
+// moe_rank_kernel with 1024 threads, and with 256 for more than 16 pairs per thread: a thread's `chunk` ids (a multiple of 4) are read in
+// 16-byte pieces, eight of them in flight; places are kept of the first 64, and of more the ids are read again.
 template <int THREADS>
 __device__ __forceinline__ void rank_long(const int* __restrict__ ids, int n_pairs, int chunk, int e, int* __restrict__ rank,
                                           int* __restrict__ counts, int* warp_tot) {
@@ -169,7 +168,7 @@ moe_rank_kernel(const int* __restrict__ topk_ids, int n_pairs, int* __restrict__
   grid_dep_launch();
   const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int chunk = (n_pairs + THREADS - 1) / THREADS;
-  if (chunk > (THREADS > 256 ? 4 : 16)) {  // many pairs: whole 16-byte pieces per thread
+  if (THREADS > kRankThreads || chunk > 16) {  // many pairs: whole 16-byte pieces per thread
     rank_long<THREADS>(topk_ids, n_pairs, (chunk + 3) & ~3, e, rank, counts, warp_tot);
     return;
   }
@@ -206,10 +205,21 @@ moe_rank_kernel(const int* __restrict__ topk_ids, int n_pairs, int* __restrict__
   if (tid == 0) counts[e] = total;
 }
 
-// A CTA reads all pairs' experts, so with many pairs its time is a thread's chain of loads and compares: 1024 threads then (us of the rank
-// and scatter kernels with 256 and 1024 threads: 4096 pairs 10.6, 11.6   16384: 20.4, 19.7   32768: 43.9, 34.3).
+// A CTA reads all pairs' experts, so with many pairs its time is a thread's chain of loads and compares: 1024 threads then, from 8192 pairs
+// on.  An SM holds one such CTA (and eight of 256 threads), so more experts than SMs take a second wave, which pays from 16384 pairs on,
+// where 256 threads begin to read ids again.  us of the rank and scatter kernels with 256 and 1024 threads, rows of 256 bytes:
+//    16 experts  4096 pairs 4.9, 5.3    8192: 8.3, 7.9     16384: 14.8, 13.1
+//   128 experts  4096 pairs 8.5, 9.0    8192: 9.8, 8.5     16384: 14.3, 9.4     32768: 94, 14
+//   256 experts  8192 pairs 14.1, 13.9  9000: 12.1, 15.1   14500: 15.8, 16.9    16384: 19.3, 17.0   20000: 23.6, 17.9
+//  1024 experts  8192 pairs 43, 48     16384: 54, 57       24576: 127, 76
+static int rank_threads(int n_pairs, int num_experts, int sms) {
+  return n_pairs >= (num_experts <= sms ? 8192 : 16384) ? kRankManyThreads : kRankThreads;
+}
 static int launch_rank(const int* ids, int n_pairs, int num_experts, int* rank, int* counts, cudaStream_t st) {
-  if (n_pairs > kRankMany)
+  int sms = 0;
+  const int rc = device_sm_count(&sms);
+  if (rc) return rc;
+  if (rank_threads(n_pairs, num_experts, sms) == kRankManyThreads)
     B200_CUDA(launch_overlapped(moe_rank_kernel<kRankManyThreads>, dim3(num_experts), dim3(kRankManyThreads), 0, st, ids, n_pairs, rank, counts));
   else
     B200_CUDA(launch_overlapped(moe_rank_kernel<kRankThreads>, dim3(num_experts), dim3(kRankThreads), 0, st, ids, n_pairs, rank, counts));
@@ -819,6 +829,12 @@ extern "C" size_t b200_moe_permute_workspace_bytes(int num_tokens, int num_exper
 extern "C" int b200_moe_max_tiles(int num_tokens, int num_experts, int top_k) {
   if (num_tokens < 0 || num_experts <= 0 || top_k <= 0) return 0;
   return (num_tokens * top_k + 127) / 128 + num_experts;
+}
+
+extern "C" int b200_moe_rank_threads(int num_pairs, int num_experts, int num_sms) {
+  B200_REQUIRE(num_pairs >= 0 && num_experts > 0 && num_sms > 0, "moe_rank_threads: %d pairs, %d experts, %d SMs", num_pairs, num_experts,
+               num_sms);
+  return rank_threads(num_pairs, num_experts, num_sms);
 }
 
 extern "C" int b200_moe_permute(const int32_t* topk_ids, int num_tokens, int num_experts, int top_k,

@@ -116,3 +116,17 @@ def test_states_wait_in_shared_memory_where_more_of_them_fit(ops, delta, dtype):
         assert not ops.state_step_held(2 * sms, 1, dim, vdim, delta, dtype) and ops.state_step_held(2 * sms + 1, 1, dim, vdim, delta, dtype)
     for dim, vdim in ((32, 512), (16, 1024), (12, 1024), (512, 32), (1024, 16), (128, 64), (144, 144)):
         assert not ops.state_step_held(4096, 16, dim, vdim, delta, dtype)
+
+
+@pytest.mark.parametrize("T,E,K", [(1023, 128, 8), (1024, 128, 8), (1100, 256, 8), (2047, 256, 8), (2048, 256, 8), (5462, 160, 3), (16400, 1024, 1)])
+def test_ranks_on_both_sides_of_the_line(ops, T, E, K):
+    """Pairs of an expert in their order, experts one after the other, dropped pairs nowhere."""
+    ids = torch.rand(T, E, generator=torch.Generator().manual_seed(T)).topk(K, dim=1).indices.to(torch.int32)
+    ids[T // 2, 0] = -1
+    p = ops.moe_permute(ids.to(DEV), E)
+    flat = ids.flatten()
+    order = torch.argsort(torch.where(flat < 0, E, flat), stable=True)[: int((flat >= 0).sum())]
+    want = torch.full((T * K,), -1, dtype=torch.int32)
+    want[order] = torch.arange(len(order), dtype=torch.int32)
+    assert torch.equal(p.row_of_pair.cpu().flatten(), want)
+    assert torch.equal(p.expert_offsets.cpu().diff(), torch.bincount(flat[flat >= 0], minlength=E).to(torch.int32))
