@@ -228,8 +228,10 @@ int b200_kv_append(const void* k_new, const void* v_new, void* k_pool, void* v_p
  *              product is then computed without a K split (slower when there are few weight tiles)
  *   k_split    0 = chosen by the library; 1, 2, 4 or 8 = CTAs that share one weight tile
  *   status_word  optional device int32 for a bounded wait that ran out
+ * b200_dense_gemm_row_tile: rows of x per work item of a product of more than 256 rows without a K split, on a GPU of num_sms SMs.
  */
 size_t b200_dense_gemm_workspace_bytes(int num_rows, int out_features);
+int b200_dense_gemm_row_tile(int num_rows, int out_features, int num_sms);
 int b200_dense_gemm_bf16(const void* x, const void* w, void* y, void* workspace, size_t workspace_bytes,
                          void* status_word, int num_rows, int out_features, int in_features, int k_split,
                          void* stream);

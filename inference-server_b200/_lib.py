@@ -35,6 +35,7 @@ SIGNATURES = {
     "b200_paged_attn_decode_static": (c_int, [c_void_p] * 7 + [c_int] * 7 + [c_float, c_int, c_void_p]),
     "b200_kv_append": (c_int, [c_void_p] * 7 + [c_int] * 7 + [c_void_p]),
     "b200_dense_gemm_workspace_bytes": (c_size_t, [c_int, c_int]),
+    "b200_dense_gemm_row_tile": (c_int, [c_int] * 3),
     "b200_dense_gemm_bf16": (c_int, [c_void_p] * 4 + [c_size_t, c_void_p] + [c_int] * 4 + [c_void_p]),
     "b200_dense_gemm_bf16_f32": (c_int, [c_void_p] * 4 + [c_size_t, c_void_p] + [c_int] * 4 + [c_void_p]),
     "b200_dense_gemm_grouped": (c_int, [c_void_p] * 4 + [c_int] * 9 + [c_void_p]),

@@ -355,8 +355,9 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
             slot = 0;
             phase ^= 1;
           }
-          // The next stage is asked for ahead of this one's MMAs: a question behind them waits until they have been taken in (gated unit of
-          // 768, width 2048, 64 rows: 12.3 -> 11.2 us; 5120 features, 64 rows 9.2 -> 8.8).
+          // Whether the next stage is there is asked without waiting, and a wait follows only if it is not: a wait takes its time also where the
+          // phase is over (gated unit of 768, width 2048, 64 rows: 12.0 -> 11.5 us; 5120 features, 100 rows 8.7 -> 8.4; 143 products 3 percent in
+          // the mean).  Ahead of this stage's MMAs, between or behind them makes no difference.
           ready = mbar_test(bar_full + 8 * slot, phase);
           const uint64_t b_desc = umma_desc_k128(sx);
 #pragma unroll
@@ -951,19 +952,27 @@ static int max_resident_clusters(int ks, int* out) {
   return 0;
 }
 
-// Rows per work item without a K split: the width that needs the fewest waves of CTAs, then the least data per CTA.
-static int pick_xbox_waves(int num_rows, int tiles, int w_rows, int sms) {
+// Rows per work item without a K split: the width that needs the fewest waves of CTAs, then the least data per CTA.  A narrower item is
+// taken where its estimate is below `share` of the wider one's.
+static int pick_xbox_waves(int num_rows, int tiles, int w_rows, int sms, double share = 1.0) {
   int pick = pick_xbox(num_rows);
   double best = 1e30;
   for (int xbox = pick; xbox >= 32; xbox -= 32) {
     const int items = tiles * ((num_rows + xbox - 1) / xbox);
     const double cost = static_cast<double>((items + sms - 1) / sms) * (static_cast<double>(w_rows) + xbox) + xbox * 0.25;
-    if (cost < best) {
+    if (cost < share * best) {
       best = cost;
       pick = xbox;
     }
   }
   return pick;
+}
+
+// The same for plain products of more than 256 rows: six waves of 192 rows against five of 256 are estimated 0.8 percent cheaper and are 1 to
+// 3 percent slower (us of 192 and 256: 5120 <- 2048, 4096 rows 69.9, 68.2; 9216 <- 2048, 2246 rows 69.4, 68.4; 5632 <- 2048, 3700 rows 69.8,
+// 68.5).  Not so with the q/k/v epilogue, which takes the longer the more rows an item has (64 + 2 x 4 heads, 2246 rows: 72, 77).
+static int plain_row_tile(int num_rows, int out_features, int sms) {
+  return pick_xbox_waves(num_rows, (out_features + 127) / 128, 128, sms, 0.99);
 }
 
 // Shape of the launch: rows of X per work item and CTAs that share a weight tile along K.
@@ -1086,9 +1095,9 @@ static int dense_gemm_any(const void* x, const void* w, void* y, bool y_is_f32, 
     if (rc) return rc;
     p.xbox = plan.xbox;
     p.ksplit = plan.ksplit;
-    // Without a split any multiple of 32 rows will do (2048 <- 4096: 1300 rows as 128 items of 192 rows in place of 96 of 256 26.7 -> 20.1 us;
-    // 5120 <- 2048: 1000 rows 24.5 -> 20.6).
-    if (p.ksplit == 1 && num_rows > kDenseMaxRows) p.xbox = pick_xbox_waves(num_rows, p.n_tiles, 128, sms);
+    // Without a split any multiple of 32 rows will do (2048 <- 4096: 1300 rows as 144 items of 160 rows in place of 96 of 256 26.1 -> 19.3 us,
+    // 1500 as 128 of 192 26.0 -> 22.2; 5120 <- 2048: 1000 rows 23.6 -> 19.8).
+    if (p.ksplit == 1 && num_rows > kDenseMaxRows) p.xbox = plain_row_tile(num_rows, out_features, sms);
   }
   p.m_tiles = (num_rows + p.xbox - 1) / p.xbox;
   B200_REQUIRE((p.ksplit == 1 || p.ksplit == 2 || p.ksplit == 4 || p.ksplit == 8) &&
@@ -1114,6 +1123,12 @@ static int dense_gemm_any(const void* x, const void* w, void* y, bool y_is_f32, 
   // with a cluster every CTA has exactly one work item; without, a CTA walks items persistently
   const int grid = p.ksplit > 1 ? items : (items < sms ? items : sms);
   return launch_dense<1, kEpiStore>(w_map, x_map, p, grid, as_stream(stream));
+}
+
+extern "C" int b200_dense_gemm_row_tile(int num_rows, int out_features, int num_sms) {
+  B200_REQUIRE(num_rows > 0 && out_features > 0 && num_sms > 0, "dense_gemm_row_tile: %d rows, %d features, %d SMs", num_rows, out_features,
+               num_sms);
+  return plain_row_tile(num_rows, out_features, num_sms);
 }
 
 extern "C" int b200_dense_gemm_bf16(const void* x, const void* w, void* y, void* workspace, size_t workspace_bytes,
