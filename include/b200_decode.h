@@ -135,7 +135,11 @@ int b200_paged_attn_decode_chunked(const void* q, const void* k_pool, const void
 /*
  * b200_paged_attn_prefill with the same two options (gate: [num_tokens, num_q_heads]), always on the tcgen05 kernel:
  * head_dim 64 or 128, any number of query heads per kv head up to 128; q, out and pools 16-byte aligned.
+ * b200_paged_attn_prefill_pairs: how many CTAs of a kv head take two tiles of 128 score rows each on a GPU of num_sms SMs, the others one
+ * (< 0 on error); *short_form (may be NULL): whether the call goes to the kernel for single tiles that see few keys.
  */
+int b200_paged_attn_prefill_pairs(int num_tokens, int first_position, int num_q_heads, int num_kv_heads, int chunk, int num_sms,
+                                  int* short_form);
 int b200_paged_attn_prefill_chunked(const void* q, const void* k_pool, const void* v_pool,
                                     const int32_t* block_table_row, void* out, void* status_word, int num_tokens,
                                     int first_position, int num_q_heads, int num_kv_heads, int head_dim,

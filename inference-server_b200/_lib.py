@@ -28,6 +28,7 @@ SIGNATURES = {
     "b200_paged_attn_decode_pairs": (c_int, [c_void_p] * 7 + [c_size_t] + [c_int] * 7 + [c_float, c_int, c_void_p]),
     "b200_paged_attn_decode_chunked": (
         c_int, [c_void_p] * 7 + [c_size_t] + [c_int] * 7 + [c_float] + [c_int] * 3 + [c_void_p] * 2),
+    "b200_paged_attn_prefill_pairs": (c_int, [c_int] * 6 + [c_void_p]),
     "b200_paged_attn_prefill_chunked": (c_int, [c_void_p] * 6 + [c_int] * 8 + [c_float, c_int] + [c_void_p] * 2),
     "b200_latent_attn_supported": (c_int, [c_int, c_int]),
     "b200_latent_attn_decode": (c_int, [c_void_p] * 6 + [c_size_t] + [c_int] * 6 + [c_float, c_int] + [c_void_p] * 2),

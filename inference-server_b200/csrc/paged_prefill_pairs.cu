@@ -53,6 +53,8 @@
 // In this form a row may find its first key tiles fully masked: its running maximum stays -inf, its exponentials are taken
 // against 0 (and are all 0), and the first key tile it does see rescales by 0 what is an exact 0.
 //
+// Registers: 168 per thread at launch, 224 in the softmax warps; the compiler keeps 36 to 44 bytes a thread in local memory (a row's 128
+// scores and 32 words of P are live together).
 // TMEM: O0, O1, S 128 columns each, P0, P1 64 (two bf16 per column).  Shared memory (head_dim 128): Q 2 x 32 KiB,
 // K ring 2 x 32 KiB, V ring 2 x 32 KiB.  Every mbarrier wait is bounded; a wait that runs out records
 // kErrDevWaitTimeout and the thread stops waiting but keeps the loop structure, so the kernel ends.
@@ -424,7 +426,8 @@ paged_attn_prefill_pairs_kernel(const __grid_constant__ CUtensorMap q_map, const
 
 // When the last CTA is done, in thirds of a single tile's key tile, if the first `pairs` CTAs of a kv head take two tiles of rows: every SM
 // takes the next CTA in the order of the grid.  A key tile of two tiles of rows counts 4/3 of one of a single tile, and what a CTA
-// does before and after its walk four key tiles.
+// does before and after its walk four key tiles.  Single tiles are priced as this file's; in the other form, which takes them in a call
+// that sees few keys, a key tile costs a twentieth to an eighth more.
 static int last_walk_end(int row_tiles, int pairs, int hkv, int qt, int first_pos, int num_tokens, int chunk, int sms) {
   using Free = std::pair<int, int>;  // a time, and how many SMs are free at it
   constexpr int kMost = 256;
@@ -449,10 +452,12 @@ static int last_walk_end(int row_tiles, int pairs, int hkv, int qt, int first_po
   }
   return end;
 }
-// Single tiles that see at most this many keys go to the other form (paged_prefill_tc.cu).  Its loop is the slower one by 0.14 us per key
-// tile of 128, but two threads share a row and its straight-line code is half as long, which a kernel that runs once per layer fetches anew
-// each time: back to back both take 7.2 us for 91 tokens from nothing, and a whole pass over such a prompt (12 layers) 2211 us with
-// the other form, 2255 with this one; 17 tokens behind 14000 150 and 133 us.
+// A call of single tiles that sees at most this many keys goes to the other form (paged_prefill_tc.cu).  Its loop is the slower one by
+// 0.12 to 0.14 us per key tile of 128, but two threads share a row and its straight-line code is half as long, which a kernel that runs once per layer
+// fetches anew each time: back to back both take 7.2 us for 91 tokens from nothing, and this form takes 33.7 -> 29.9 us for 91 tokens behind
+// 2500 and 43.5 -> 39.3 behind 3500; in a whole pass (12 layers, us with the other form and with this one) 91 tokens from
+// nothing take 2072, 2122, behind 2000 2393, 2414, behind 2900 2505, 2512, behind 3500 2578, 2576, behind 5000 2791, 2767; 300 tokens behind
+// 2900 2740, 2745, behind 3500 2826, 2818; 17 tokens behind 3500 2138, 2146, behind 5000 2344, 2324.
 constexpr int kSingleKeys = 3072;
 // How many CTAs of a kv head take two tiles of rows.  None while every tile has an SM of its own (us, single tiles and pairs,
 // 32 / 4 heads, 500 tokens behind 333, 128 tiles: 16.3, 18.6; 8 / 8 heads, 2048 behind 8192, 128 tiles: 121, 138).  With up to three
@@ -472,6 +477,21 @@ static int prefill_pairs(int row_tiles, int hkv, int qt, int first_pos, int num_
   if (row_tiles * hkv > 3 * sms) return all;
   const int two = last_walk_end(row_tiles, all, hkv, qt, first_pos, num_tokens, chunk, sms);
   return two < last_walk_end(row_tiles, 0, hkv, qt, first_pos, num_tokens, chunk, sms) ? all : 0;
+}
+
+// How a call is laid out: tiles of 128 score rows per kv head, how many CTAs of a head take two of them, and whether its single tiles go to
+// the other form.
+struct PrefillPlan {
+  int row_tiles, pairs;
+  bool other_form;
+};
+static PrefillPlan prefill_plan(int num_tokens, int first_pos, int hq, int hkv, int chunk, int sms) {
+  PrefillPlan p;
+  const int qt = kTcRows / (hq / hkv), keys = first_pos + num_tokens;
+  p.row_tiles = (num_tokens + qt - 1) / qt;
+  p.pairs = prefill_pairs(p.row_tiles, hkv, qt, first_pos, num_tokens, chunk, sms);
+  p.other_form = p.pairs == 0 && (chunk > 0 ? std::min(chunk, keys) : keys) <= kSingleKeys;
+  return p;
 }
 
 template <int D, int G>
@@ -513,13 +533,12 @@ int launch_prefill_tc(const void* q, const void* k_pool, const void* v_pool, con
   } else {
     qmap = kmap;  // not read
   }
-  const int qt = kTcRows / group, row_tiles = (num_tokens + qt - 1) / qt;
   int sms = 0;
   rc = device_sm_count(&sms);
   if (rc) return rc;
-  const int pairs = prefill_pairs(row_tiles, hkv, qt, first_pos, num_tokens, chunk, sms);
-  const int seen = chunk > 0 ? std::min(chunk, first_pos + num_tokens) : first_pos + num_tokens;
-  if (pairs == 0 && seen <= kSingleKeys)
+  const PrefillPlan plan = prefill_plan(num_tokens, first_pos, hq, hkv, chunk, sms);
+  const int row_tiles = plan.row_tiles, pairs = plan.pairs;
+  if (plan.other_form)
     return launch_prefill_single(qmap, kmap, vmap, q_tma, head_dim, q, table_row, out, err, num_tokens, first_pos, hq, hkv, num_blocks,
                                  scale, chunk, gate, st);
 #define B200_TC_ARGS qmap, kmap, vmap, q, table_row, out, err, num_tokens, first_pos, hq, hkv, num_blocks, scale, chunk, \
@@ -532,3 +551,16 @@ int launch_prefill_tc(const void* q, const void* k_pool, const void* v_pool, con
 }
 
 }  // namespace b200
+
+using namespace b200;
+
+extern "C" int b200_paged_attn_prefill_pairs(int num_tokens, int first_position, int num_q_heads, int num_kv_heads, int chunk, int num_sms,
+                                             int* short_form) {
+  B200_REQUIRE(num_tokens > 0 && first_position >= 0 && num_kv_heads > 0 && num_q_heads % num_kv_heads == 0 && num_q_heads > 0 &&
+                   num_q_heads / num_kv_heads <= kTcRows && chunk >= 0 && num_sms > 0,
+               "paged_attn_prefill_pairs: %d tokens from %d, %d query heads over %d, chunk %d, %d SMs", num_tokens, first_position, num_q_heads,
+               num_kv_heads, chunk, num_sms);
+  const PrefillPlan plan = prefill_plan(num_tokens, first_position, num_q_heads, num_kv_heads, chunk, num_sms);
+  if (short_form != nullptr) *short_form = plan.other_form;
+  return plan.pairs;
+}

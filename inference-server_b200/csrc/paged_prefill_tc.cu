@@ -4,8 +4,9 @@
 // reference is described there (src/inference_server/kv_cache/hf_format.py:21-45 gather +
 // src/inference_server/backends/torch_backend.py:107-147 chunk forward).
 //
-// This form has one tile of rows per CTA and short chains; it serves calls whose tiles all have an SM of their own and whose
-// walks are short (paged_prefill_pairs.cu has the rule and the other form).
+// This form has one tile of rows per CTA and short chains; it serves calls for which no CTAs with two tiles are chosen (every tile has an
+// SM of its own, or up to three share one and end sooner that way) and that see at most 3072 keys (paged_prefill_pairs.cu has
+// the rule and the other form).
 //
 //   grid     query tiles x kv heads.  A CTA owns 128 rows of the score matrix: 128 / G consecutive prompt
 //            positions x the G query heads of its kv head, and walks the key tiles (128 keys = 8 pages) of
@@ -414,7 +415,7 @@ static int launch_prefill_tc_g(const CUtensorMap& qmap, const CUtensorMap& kmap,
   return 0;
 }
 
-// Arguments as launch_prefill_pairs, which calls this form where it is the better one.
+// Arguments as launch_prefill_tc (paged_prefill_pairs.cu), which calls this form where it is the better one.
 int launch_prefill_single(const CUtensorMap& qmap, const CUtensorMap& kmap, const CUtensorMap& vmap, bool q_tma, int head_dim, const void* q,
                           const int* table_row, void* out, int* err, int num_tokens, int first_pos, int hq, int hkv, int num_blocks,
                           float scale, int chunk, const float* gate, cudaStream_t st) {

@@ -408,6 +408,16 @@ def paged_attn_prefill_chunked_supported(num_q_heads: int, num_kv_heads: int, he
     return dtype == torch.bfloat16 and head_dim in (64, 128) and num_q_heads // num_kv_heads <= 128
 
 
+def paged_attn_prefill_pairs(num_tokens: int, first_pos: int, num_q_heads: int, num_kv_heads: int, chunk: int = 0,
+                             num_sms: int = 148) -> tuple[int, bool]:
+    """How the prompt attention lays out a call: CTAs per kv head that take two tiles of rows each, and whether it goes to the kernel
+    for single tiles that see few keys."""
+    import ctypes
+    short = ctypes.c_int(0)
+    pairs = _form("b200_paged_attn_prefill_pairs", num_tokens, first_pos, num_q_heads, num_kv_heads, chunk, num_sms, ctypes.addressof(short))
+    return pairs, bool(short.value)
+
+
 def paged_attn_prefill_chunked(q, k_pool, v_pool, table_row, first_pos: int, scale: float, status=None, chunk: int = 0, gate=None,
                                out=None):
     """`paged_attn_prefill` with the options of `paged_attn_decode_chunked`; head_dim 64 or 128, any head grouping."""

@@ -109,3 +109,49 @@ def test_two_tiles_per_cta_give_the_bits_of_one(ops, hq, hkv, d, first, rows, ch
         lens = torch.tensor([first + p + 1], dtype=torch.int32, device=DEV)
         dec = ops.paged_attn_decode_chunked(q[p:p + 1], kp, vp, row[None], lens, d ** -0.5, 1024, ws, chunk, gate[p:p + 1])
         assert rel_err(whole[p:p + 1], dec) < TOL
+
+
+@pytest.mark.parametrize("hq,hkv,d,first,rows,chunk,pairs,short", [
+    (32, 4, 128, 4000, 1500, 0, 37, False),  # a wave of CTAs with two tiles, then one of single tiles
+    (32, 4, 128, 5000, 1208, 0, 37, False),  # the same with two single tiles per head
+    (32, 4, 128, 1800, 1200, 0, 37, True),   # pieces by the other kernel, over up to 3000 keys
+    (40, 8, 64, 1900, 1100, 0, 18, True),
+])
+def test_mixed_grids_and_both_kernels_give_the_same_bits(ops, hq, hkv, d, first, rows, chunk, pairs, short):
+    sms, tile = torch.cuda.get_device_properties(0).multi_processor_count, 128 // (hq // hkv)
+    step = sms // hkv // 2 * tile
+    if sms == 148:
+        assert ops.paged_attn_prefill_pairs(rows, first, hq, hkv, chunk) == (pairs, False)
+        assert ops.paged_attn_prefill_pairs(step, first, hq, hkv, chunk) == (0, short)
+    q, kp, vp, row = (t.to(DEV) for t in case(hq, hkv, d, first, rows, seed=rows))
+    status = torch.zeros(64, dtype=torch.int32, device=DEV)
+
+    def run(lo, hi):
+        return ops.paged_attn_prefill_chunked(q[lo:hi], kp, vp, row, first + lo, d ** -0.5, status, chunk)
+
+    whole = run(0, rows)
+    assert torch.equal(whole, torch.cat([run(lo, min(rows, lo + step)) for lo in range(0, rows, step)]))
+    ops.read_status(status, "paged_attn_prefill_chunked")
+    # and tiles of both kinds against decode attention: the same bound as above
+    for p in (0, tile, rows // 2, rows - 1):
+        ws = ops.paged_attn_workspace(1, hq, d, row.numel(), 16, 1024, DEV)
+        lens = torch.tensor([first + p + 1], dtype=torch.int32, device=DEV)
+        dec = ops.paged_attn_decode_chunked(q[p:p + 1], kp, vp, row[None], lens, d ** -0.5, 1024, ws, chunk)
+        assert rel_err(whole[p:p + 1], dec) < TOL
+
+
+@pytest.mark.parametrize("hq,hkv,d,first,rows", [
+    (32, 4, 128, 3056, 17),  # queries by TMA, 8 and 16 heads per kv head
+    (64, 4, 128, 3100, 21),
+    (24, 8, 128, 3500, 50),  # copied queries, 42 positions per tile
+    (40, 8, 64, 3300, 60),   # head_dim 64, 25 positions per tile
+])
+def test_single_tiles_that_see_many_keys(ops, hq, hkv, d, first, rows):
+    assert ops.paged_attn_prefill_pairs(rows, first, hq, hkv) == (0, False)
+    q, kp, vp, row = case(hq, hkv, d, first, rows, seed=first)
+    status = torch.zeros(64, dtype=torch.int32, device=DEV)
+    out = ops.paged_attn_prefill_chunked(q.to(DEV), kp.to(DEV), vp.to(DEV), row.to(DEV), first, d ** -0.5, status)
+    ops.read_status(status, "paged_attn_prefill_chunked")
+    ref = oracle.paged_prefill_ref(q, kp, vp, row.tolist(), first, d ** -0.5)
+    per_row = (out.float().cpu() - ref).abs().amax(dim=(1, 2)) / ref.abs().amax()
+    assert float(per_row.max()) < TOL
