@@ -371,12 +371,12 @@ static int resident_route_clusters(int H, int E, int* out) {
   return 0;
 }
 
-// Rows per cluster: 16, or 32 where that leaves at most three waves of clusters in place of four.  A wave of 32-row clusters takes
-// 1.0-1.15 times one of 16-row clusters (128 experts: width 512 10.2 and 9.2 us, 2048 9.5 and 8.8), and how many of either
-// the GPU holds depends on their shared memory, so on width and experts.  us with 16 and with 32, 128 experts:
-//   width 2048   513 rows 8.8, 9.8   576: 12.9, 10.1   1024: 16.8, 11.3   2048: 32.1, 21.7
-//   width  512  1024 rows 9.2, 10.2  1500: 14.9, 10.9   2048: 17.1, 17.7   4096: 31.5, 28.3
-//   width 4096   256 rows 14.7, 9.5   512: 22.8, 18.6   1024: 39.6, 29.0
+// Rows per cluster: 16, or 32 where their waves take less.  A wave of 32-row clusters takes at most 1.15 times one of 16-row clusters, and how many
+// of either the GPU holds depends on their shared memory, so on width and experts.  us with 16 and with 32, and the waves of each:
+//   128 experts, width  512  1024 rows 9.2, 10.2   2048: 16.9, 17.4 (2, 2)   4096: 31.3, 28.2 (4, 3)   5000: 38.0, 34.4 (5, 4)
+//   128 experts, width 2048   513 rows 8.8, 9.8    1024: 16.8, 11.3 (2, 1)   2048: 32.1, 21.6 (4, 2)
+//   128 experts, width 4096   256 rows 14.7, 9.5    512: 22.8, 18.6         1024: 39.6, 29.1 (5, 3)
+//    64 experts, width 2048  5000 rows 42.0, 37.3 (5, 4)   6000: 49.8, 41.8 (6, 4)
 static int route_rows(int T, int H, int E, int* out) {
   *out = 16;
   const int c16 = (T + 15) / 16, c32 = (T + 31) / 32;
@@ -387,7 +387,7 @@ static int route_rows(int T, int H, int E, int* out) {
   if (c16 <= n16) return 0;
   rc = resident_route_clusters<32>(H, E, &n32);
   if (rc) return rc;
-  if (4 * ((c32 + n32 - 1) / n32) <= 3 * ((c16 + n16 - 1) / n16)) *out = 32;
+  if (23 * ((c32 + n32 - 1) / n32) <= 20 * ((c16 + n16 - 1) / n16)) *out = 32;
   return 0;
 }
 

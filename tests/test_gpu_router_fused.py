@@ -101,3 +101,21 @@ def test_unsupported_shapes_are_refused(ops):
     x, delta, nw, rw = make(4, 768, 16, seed=3)
     with pytest.raises(Exception, match="multiple of 512"):
         ops.add_rmsnorm_route(x.to(DEV), None, nw.to(DEV), 1e-6, rw.to(DEV), 4)
+
+
+@pytest.mark.parametrize("T,H,E", [(5000, 512, 128), (5000, 2048, 64)])
+def test_four_waves_of_long_clusters_in_place_of_five(ops, T, H, E):
+    """On 148 SMs; the same rows in calls of one wave of short clusters: the same bits."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("wave counts of a GPU with 148 SMs")
+    assert ops.add_rmsnorm_route_rows(T, H, E) == 32 and ops.add_rmsnorm_route_rows(400, H, E) == 16
+    g = torch.Generator().manual_seed(T + H)
+    x, delta = (torch.randn(T, H, generator=g).bfloat16().to(DEV) for _ in range(2))
+    nw, rw = (1 + 0.1 * torch.randn(H, generator=g)).bfloat16().to(DEV), (torch.randn(E, H, generator=g) * 0.05).bfloat16().to(DEV)
+
+    def run(lo, hi):
+        xs = x[lo:hi].clone()
+        return xs, *ops.add_rmsnorm_route(xs, delta[lo:hi], nw, 1e-6, rw, 8, want_logits=True)
+    parts = [run(lo, min(T, lo + 400)) for lo in range(0, T, 400)]
+    for i, whole in enumerate(run(0, T)):
+        assert torch.equal(whole, torch.cat([p[i] for p in parts]))
