@@ -130,3 +130,45 @@ def test_ranks_on_both_sides_of_the_line(ops, T, E, K):
     want[order] = torch.arange(len(order), dtype=torch.int32)
     assert torch.equal(p.row_of_pair.cpu().flatten(), want)
     assert torch.equal(p.expert_offsets.cpu().diff(), torch.bincount(flat[flat >= 0], minlength=E).to(torch.int32))
+
+
+FIRST_CALL_IN_A_CAPTURE = """
+import importlib, sys, torch
+from types import SimpleNamespace
+sys.path.insert(0, {root!r})
+ops = importlib.import_module("inference-server_b200.ops")
+torch.manual_seed(0)
+M, W = 400, 2048
+r = lambda *s, dtype=torch.bfloat16: torch.randn(*s, device="cuda", dtype=dtype)
+x, w, d = r(M, W, dtype=torch.float32), r(W, dtype=torch.float32), r(M, W)
+y, xb, rows, pw = r(M * 2, W), r(M, W), torch.randperm(M * 2, device="cuda").to(torch.int32).view(M, 2), torch.rand(M, 2, device="cuda")
+ids = torch.rand(M, 16, device="cuda").topk(2, dim=1).indices.to(torch.int32)
+H, D = 4, 128
+act, state, decay = r(M, 3 * H * D), r(M, 2, H, D, D, dtype=torch.float32), torch.rand(H, device="cuda")
+slots, pos = torch.arange(M, device="cuda", dtype=torch.int32), torch.full((M,), 3, device="cuda", dtype=torch.int32)
+sw = SimpleNamespace(heads=H, qk_heads=H, d=D, dv=D, decay=decay)
+q, kp, table = r(600, 32, 128), r(40, 4, 16, 128), torch.arange(40, device="cuda", dtype=torch.int32)
+def all_of_them():
+    xs, xg, xc, S, o = x.clone(), x.clone(), xb.clone(), state.clone(), torch.empty(M, H, D, device="cuda")
+    ops.state_step(act, sw, S, slots, pos, o)
+    return [ops.residual_norm(xs, None, w, 1e-5, W), ops.group_rmsnorm(xg, d, w.bfloat16(), 1e-5, W, 4),
+            ops.moe_combine_add_rmsnorm(y, rows, pw, xc, w.bfloat16(), 1e-5), ops.moe_permute(ids, 16).row_of_pair, o, S,
+            ops.paged_attn_prefill(q, kp, kp, table, 0, 0.1)]
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    captured = all_of_them()
+g.replay()
+torch.cuda.synchronize()
+assert all(torch.equal(a, b) for a, b in zip(captured, all_of_them()))
+print("same")
+"""
+
+
+def test_the_first_call_of_a_process_may_be_captured(ops):
+    """What the rules ask of the runtime they may ask while a graph is being captured."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+    run = subprocess.run([sys.executable, "-c", FIRST_CALL_IN_A_CAPTURE.format(root=ROOT)], capture_output=True, text=True, timeout=240)
+    assert run.returncode == 0 and run.stdout.strip().endswith("same"), run.stderr[-2000:]
